@@ -244,7 +244,7 @@ int psc_step_windows_ex(int store, const psc_window* d_windows, int nwin, int64_
         // (TRT windows are rejected by the hosts that build tables; the exact kernel runs BGK)
         if (c.cells_per_thread != 1)
             return fail(PSC_E_UNSUPPORTED, "psc_step_windows: PSC_STORE_F64_EXACT runs one cell per thread");
-        e = launch_step(store, d_windows, nwin, total_tiles, flags, moving, c.grid_ctas, as_stream(stream));
+        e = launch_step_exact(d_windows, nwin, total_tiles, flags, moving, c.grid_ctas, as_stream(stream));
     } else if (c.kernel == PSC_KERNEL_AUTO || c.kernel == PSC_KERNEL_DIRECT) {
         e = launch_step_fast(store, d_windows, nwin, total_tiles, flags, moving, c.cells_per_thread, c.grid_ctas,
                              as_stream(stream));

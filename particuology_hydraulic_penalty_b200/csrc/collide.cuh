@@ -155,6 +155,284 @@ PSC_HD void collide_exact(double* f, const ExactMoments& mo, double solid, bool 
     imb[2] = iz;
 }
 
+// ---------------------------------------------------------------------------
+// The same arithmetic without branches (the step kernels' path)
+// ---------------------------------------------------------------------------
+// moments_exact and collide_exact rounding for rounding, with the divisions of
+// d3q19.cuh's branch-free forms and the window's constants made once.  Each
+// function returns whether an operand left the range of those forms; the
+// caller then takes the cell through moments_exact / collide_exact.
+//
+// The range is tested on the roots of a cell's arithmetic, in integer instructions (the FP64 pipe is
+// what bounds the exact kernels): every population in [2^-15, 2), rho in [2^-8, 2^8), tau in
+// [2^-8, 2^8], the components of F and of the solid velocity and the solid fraction zero or in
+// [2^-200, 2^200).  All other
+// operands follow.  A sum or difference of doubles is a multiple of the smaller one's ulp, so
+// m + F/2 is zero or >= 2^-253, u + F/(2 rho) zero or >= 2^-313, c.u zero or >= 2^-365 and its
+// square >= 2^-730, u.F and c.F - u.F zero or >= 2^-565, (c.u)(c.F) >= 2^-617, feq zero or >= 2^-796
+// and f - feq zero or >= 2^-848; nothing exceeds 2^500.  Each form needs zero or 2^-900 .. 2^900.
+//
+// FP64 operations of a static cell with IMB momentum and F along an axis: about 575 (1360 with
+// xdiv_r's five operations and two comparisons per division, and a branch each).
+constexpr int kExactRootRange = 200;
+
+struct ExactWin {
+    double tau, rtau, rtau_lo;       // 1/tau = rtau + rtau_lo
+    double fx, fy, fz, hfx, hfy, hfz;
+    double pw[3];                    // (1 - 0.5 / tau) w for the rest, axis and diagonal weights
+    double cf[9];                    // c_k . F of the nine direction pairs
+    int axis;                        // the axis of a body force along one axis, else -1
+    int out;                         // tau or F outside the branch-free forms' range
+};
+
+// The parts of ExactWin, independent of one another (a CTA's warps make one each).
+PSC_HD void exact_win_force(ExactWin& w, double tau, double fx, double fy, double fz) {
+    w.tau = tau;
+    w.fx = fx;
+    w.fy = fy;
+    w.fz = fz;
+    w.hfx = xmul(0.5, fx);
+    w.hfy = xmul(0.5, fy);
+    w.hfz = xmul(0.5, fz);
+    w.out = !div_r_divisor_ok(tau) || out_of_range<kExactRootRange>(fx) || out_of_range<kExactRootRange>(fy) ||
+            out_of_range<kExactRootRange>(fz);
+    w.axis = fx == 0.0 && fy == 0.0 ? 2 : (fx == 0.0 && fz == 0.0 ? 1 : (fy == 0.0 && fz == 0.0 ? 0 : -1));
+}
+PSC_HD void exact_win_tau(ExactWin& w, double tau) {
+    w.rtau = xdiv(1.0, tau);
+    w.rtau_lo = xmul(xfma(-w.rtau, tau, 1.0), w.rtau);
+}
+PSC_HD void exact_win_guo(ExactWin& w, double tau) {
+    const double pref = xsub(1.0, xdiv(0.5, tau));
+    w.pw[0] = xmul(pref, W0);
+    w.pw[1] = xmul(pref, W1);
+    w.pw[2] = xmul(pref, W2);
+}
+PSC_HD void exact_win_pairs(ExactWin& w, double fx, double fy, double fz) {
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        const int i = 2 * k + 1;
+        w.cf[k] = xadd(xadd(cm(cxv(i), fx), cm(cyv(i), fy)), cm(czv(i), fz));
+    }
+}
+PSC_HD void make_exact_win(ExactWin& w, double tau, double fx, double fy, double fz) {
+    exact_win_force(w, tau, fx, fy, fz);
+    exact_win_tau(w, tau);
+    exact_win_guo(w, tau);
+    exact_win_pairs(w, fx, fy, fz);
+}
+
+// What a cell's Guo terms share.  (c_k . F - u . F) / c_s^2 depends on c_k . F alone, which takes three
+// values where F lies along one axis: they are divided once per cell (d0, dp, dm) and selected per pair.
+struct ExactGuo {
+    double uf, d0, dp, dm;
+};
+
+// u + F / (2 rho), u . F and the shared Guo terms; AXIS: F lies along the axis w.axis.
+template <bool AXIS>
+PSC_HD ExactGuo exact_guo_s(const ExactWin& w, double rho, double rrho, double half, double& ux, double& uy, double& uz) {
+    ExactGuo g;
+    if (AXIS) {
+        const int a = w.axis;
+        const double F = a == 0 ? w.fx : (a == 1 ? w.fy : w.fz);
+        if (half != 0.0) {
+            const double h = xdiv_r_s(xmul(half, F), rho, rrho);
+            ux = xadd(ux, a == 0 ? h : 0.0);
+            uy = xadd(uy, a == 1 ? h : 0.0);
+            uz = xadd(uz, a == 2 ? h : 0.0);
+        }
+        g.uf = xmul(a == 0 ? ux : (a == 1 ? uy : uz), F);
+        g.d0 = div_cs2_s(-g.uf);
+        g.dp = div_cs2_s(xsub(F, g.uf));
+        g.dm = div_cs2_s(xsub(-F, g.uf));
+    } else {
+        if (half != 0.0) {
+            ux = xadd(ux, xdiv_r_s(w.hfx, rho, rrho));
+            uy = xadd(uy, xdiv_r_s(w.hfy, rho, rrho));
+            uz = xadd(uz, xdiv_r_s(w.hfz, rho, rrho));
+        }
+        g.uf = xadd(xadd(xmul(ux, w.fx), xmul(uy, w.fy)), xmul(uz, w.fz));
+        g.d0 = div_cs2_s(-g.uf);
+        g.dp = g.dm = 0.0;
+    }
+    return g;
+}
+
+// (c . F - u . F) / c_s^2 for the direction c = (CX, CY, CZ) and F along `axis`.
+template <int C>
+PSC_HD double exact_by_sign(const ExactGuo& g) {
+    return C == 0 ? g.d0 : (C > 0 ? g.dp : g.dm);
+}
+template <int CX, int CY, int CZ>
+PSC_HD double exact_by_axis(int axis, const ExactGuo& g) {
+    if constexpr (CX == CY) return axis == 2 ? exact_by_sign<CZ>(g) : exact_by_sign<CX>(g);
+    else if constexpr (CX == CZ) return axis == 1 ? exact_by_sign<CY>(g) : exact_by_sign<CX>(g);
+    else if constexpr (CY == CZ) return axis == 0 ? exact_by_sign<CX>(g) : exact_by_sign<CY>(g);
+    else return axis == 0 ? exact_by_sign<CX>(g) : (axis == 1 ? exact_by_sign<CY>(g) : exact_by_sign<CZ>(g));
+}
+
+// The Guo terms of a pair, pref w ((c . F - u . F) / c_s^2 + (c . u)(c . F) / c_s^4).
+template <bool AXIS, int K>
+PSC_HD void exact_guo_pair_s(const ExactWin& w, const ExactGuo& g, double pw, double cu, double& g_i, double& g_j) {
+    const double cf = w.cf[K];
+    const double t2 = div_cs2sq_s(xmul(cu, cf));
+    if (AXIS) {
+        g_i = xmul(pw, xadd(exact_by_axis<cxv(2 * K + 1), cyv(2 * K + 1), czv(2 * K + 1)>(w.axis, g), t2));
+        g_j = xmul(pw, xadd(exact_by_axis<cxv(2 * K + 2), cyv(2 * K + 2), czv(2 * K + 2)>(w.axis, g), t2));
+    } else {
+        g_i = xmul(pw, xadd(div_cs2_s(xsub(cf, g.uf)), t2));
+        g_j = xmul(pw, xadd(div_cs2_s(xsub(-cf, g.uf)), t2));
+    }
+}
+
+// c_i . v without the additions of a zero component (they change no value).
+template <int I>
+PSC_HD double cdot_s(double x, double y, double z) {
+    constexpr int a = cxv(I), b = cyv(I), c = czv(I);
+    if constexpr (a != 0 && b != 0) return xadd(a > 0 ? x : -x, b > 0 ? y : -y);
+    else if constexpr (a != 0 && c != 0) return xadd(a > 0 ? x : -x, c > 0 ? z : -z);
+    else if constexpr (b != 0 && c != 0) return xadd(b > 0 ? y : -y, c > 0 ? z : -z);
+    else if constexpr (a != 0) return a > 0 ? x : -x;
+    else if constexpr (b != 0) return b > 0 ? y : -y;
+    else return c > 0 ? z : -z;
+}
+
+// acc + c v for the component c of direction I along AXIS (the first term starts the sum).
+template <int AXIS, int I>
+PSC_HD void moment_add_s(double& acc, bool& first, double v) {
+    constexpr int c = cv(AXIS, I);
+    if constexpr (c != 0) {
+        acc = first ? (c > 0 ? v : -v) : (c > 0 ? xadd(acc, v) : xsub(acc, v));
+        first = false;
+    }
+}
+template <int AXIS, int I = 0>
+PSC_HD void seq_moment_s(const double* f, double& acc, bool& first) {
+    if constexpr (I < Q) {
+        moment_add_s<AXIS, I>(acc, first, f[I]);
+        seq_moment_s<AXIS, I + 1>(f, acc, first);
+    }
+}
+
+struct ExactMomentsS {
+    double rho, ux, uy, uz, rrho;
+    bool out;
+};
+
+PSC_HD ExactMomentsS moments_exact_s(const double* f, double hfx, double hfy, double hfz) {
+    ExactMomentsS m;
+    double rho = f[0];
+#pragma unroll
+    for (int i = 1; i < Q; ++i) rho = xadd(rho, f[i]);
+    double mx = 0.0, my = 0.0, mz = 0.0;
+    bool a = true, b = true, c = true;
+    seq_moment_s<0>(f, mx, a);
+    seq_moment_s<1>(f, my, b);
+    seq_moment_s<2>(f, mz, c);
+    mx = xadd(mx, hfx);
+    my = xadd(my, hfy);
+    mz = xadd(mz, hfz);
+    uint32_t h = hi_word(f[0]) ^ 0x3f000000u;  // 2^-15 <= f < 2: the sign and seven exponent bits are 0x3f
+#pragma unroll
+    for (int i = 1; i < Q; ++i) h |= hi_word(f[i]) ^ 0x3f000000u;
+    m.out = (h >= 0x01000000u) | (hi_word(rho) - (1015u << 20) >= (16u << 20));  // 2^-8 <= rho < 2^8
+    m.rho = rho;
+    m.rrho = xrcp(rho);
+    m.ux = xdiv_r_s(mx, rho, m.rrho);
+    m.uy = xdiv_r_s(my, rho, m.rrho);
+    m.uz = xdiv_r_s(mz, rho, m.rrho);
+    return m;
+}
+
+template <int K, bool MOVING, bool IMB, bool AXIS>
+PSC_HD void exact_pair_s(double* f, const ExactWin& w, double wr, double pw, double ct, const ExactGuo& guo, double B,
+                         double omB, double uex, double uey, double uez, double usx, double usy, double usz,
+                         double cts, double& ix, double& iy, double& iz) {
+    constexpr int i = 2 * K + 1, j = i + 1;
+    const double cu = cdot_s<i>(uex, uey, uez);
+    const double q = div_cs2_s(cu);
+    const double b = half_div_cs2sq_s(xmul(cu, cu));
+    const double feqf_i = xmul(wr, xsub(xadd(xadd(1.0, q), b), ct));
+    const double feqf_j = xmul(wr, xsub(xadd(xsub(1.0, q), b), ct));
+    double feqs_i = wr, feqs_j = wr;
+    if (MOVING) {
+        const double cus = cdot_s<i>(usx, usy, usz);
+        const double qs = div_cs2_s(cus);
+        const double bs = half_div_cs2sq_s(xmul(cus, cus));
+        feqs_i = xmul(wr, xsub(xadd(xadd(1.0, qs), bs), cts));
+        feqs_j = xmul(wr, xsub(xadd(xsub(1.0, qs), bs), cts));
+    }
+    const double fi = f[i], fj = f[j];
+    const double dji = xsub(fj, fi);
+    const double os_i = xsub(xadd(dji, feqs_i), feqf_j);
+    const double os_j = xsub(xadd(-dji, feqs_j), feqf_i);
+    const double di = xsub(fi, feqf_i), dj = xsub(fj, feqf_j);
+    const double bo_i = xmul(B, os_i), bo_j = xmul(B, os_j);
+    const double coll_i = xsub(bo_i, xmul(omB, xdiv_s(di, w.tau, w.rtau, w.rtau_lo)));
+    const double coll_j = xsub(bo_j, xmul(omB, xdiv_s(dj, w.tau, w.rtau, w.rtau_lo)));
+    double g_i, g_j;
+    exact_guo_pair_s<AXIS, K>(w, guo, pw, cu, g_i, g_j);
+    f[i] = xadd(fi, xadd(coll_i, g_i));
+    f[j] = xadd(fj, xadd(coll_j, g_j));
+    if (IMB) {
+        if constexpr (cxv(i) != 0) ix = cxv(i) > 0 ? xsub(xadd(ix, bo_i), bo_j) : xadd(xsub(ix, bo_i), bo_j);
+        if constexpr (cyv(i) != 0) iy = cyv(i) > 0 ? xsub(xadd(iy, bo_i), bo_j) : xadd(xsub(iy, bo_i), bo_j);
+        if constexpr (czv(i) != 0) iz = czv(i) > 0 ? xsub(xadd(iz, bo_i), bo_j) : xadd(xsub(iz, bo_i), bo_j);
+    }
+}
+
+// collide_exact in the branch-free forms; true where an operand left their range (f is then undefined).
+template <bool MOVING, bool IMB, bool AXIS>
+PSC_HD bool collide_exact_s(double* f, const ExactMomentsS& mo, double solid, double usx, double usy, double usz,
+                            const ExactWin& w, double* imb) {
+    const double rho = mo.rho;
+    double uex = mo.ux, uey = mo.uy, uez = mo.uz;
+    const ExactGuo guo = exact_guo_s<AXIS>(w, rho, mo.rrho, 0.5, uex, uey, uez);
+    bool out = mo.out | (w.out != 0);
+    const double ct = half_div_cs2_s(xadd(xadd(xmul(uex, uex), xmul(uey, uey)), xmul(uez, uez)));
+    double cts = 0.0;
+    if (MOVING) {
+        out |= out_of_range<kExactRootRange>(usx) | out_of_range<kExactRootRange>(usy) |
+               out_of_range<kExactRootRange>(usz);
+        cts = half_div_cs2_s(xadd(xadd(xmul(usx, usx), xmul(usy, usy)), xmul(usz, usz)));
+    }
+    const double al = solid < 0.0 ? 0.0 : (solid > 1.0 ? 1.0 : solid);
+    out |= out_of_range<kExactRootRange>(al);
+    const double den = xadd(xadd(al, xmul(w.tau, xsub(1.0, al))), 1.0e-14);  // between 1 and tau
+    const double B = xdiv_r_s(al, den, xrcp(den));
+    const double omB = xsub(1.0, B);
+    double ix = 0.0, iy = 0.0, iz = 0.0;
+    {  // rest population
+        const double wr = xmul(W0, rho);
+        const double feqf = xmul(wr, xsub(1.0, ct));
+        const double feqs = MOVING ? xmul(wr, xsub(1.0, cts)) : wr;
+        const double d = xsub(f[0], feqf);
+        const double coll = xsub(xmul(B, xsub(feqs, feqf)), xmul(omB, xdiv_s(d, w.tau, w.rtau, w.rtau_lo)));
+        f[0] = xadd(f[0], xadd(coll, xmul(w.pw[0], guo.d0)));
+    }
+    const double wr1 = xmul(W1, rho), wr2 = xmul(W2, rho);
+    const double pw1 = w.pw[1], pw2 = w.pw[2];
+#define PSC_EXACT_PAIR(K)                                                                                          \
+    exact_pair_s<K, MOVING, IMB, AXIS>(f, w, K < 3 ? wr1 : wr2, K < 3 ? pw1 : pw2, ct, guo, B, omB, uex, uey, uez,  \
+                                       usx, usy, usz, cts, ix, iy, iz)
+    PSC_EXACT_PAIR(0);
+    PSC_EXACT_PAIR(1);
+    PSC_EXACT_PAIR(2);
+    PSC_EXACT_PAIR(3);
+    PSC_EXACT_PAIR(4);
+    PSC_EXACT_PAIR(5);
+    PSC_EXACT_PAIR(6);
+    PSC_EXACT_PAIR(7);
+    PSC_EXACT_PAIR(8);
+#undef PSC_EXACT_PAIR
+    if (IMB) {
+        imb[0] = ix;
+        imb[1] = iy;
+        imb[2] = iz;
+    }
+    return out;
+}
+
 // ===========================================================================
 // fast deviation form, arithmetic type R
 // ===========================================================================
@@ -449,6 +727,45 @@ PSC_HD void collide_bb_exact(double* f, bool solid, double tau, double fx, doubl
         f[i] = xadd(xsub(f[i], xdiv_d(xsub(f[i], feq_i), by_tau)), g_i);
         f[j] = xadd(xsub(f[j], xdiv_d(xsub(f[j], feq_j), by_tau)), g_j);
     }
+}
+
+// collide_bb_exact in the branch-free forms (moments_exact_s, ExactWin); true where an operand left
+// their range (f is then undefined).
+template <int K, bool AXIS>
+PSC_HD void bb_pair_s(double* f, const ExactWin& w, double wr, double pw, double ct, const ExactGuo& guo, double ux, double uy,
+                      double uz) {
+    constexpr int i = 2 * K + 1, j = i + 1;
+    const double cu = cdot_s<i>(ux, uy, uz);
+    const double q = div_cs2_s(cu);
+    const double b = half_div_cs2sq_s(xmul(cu, cu));
+    const double di = xsub(f[i], xmul(wr, xsub(xadd(xadd(1.0, q), b), ct)));
+    const double dj = xsub(f[j], xmul(wr, xsub(xadd(xsub(1.0, q), b), ct)));
+    double g_i, g_j;
+    exact_guo_pair_s<AXIS, K>(w, guo, pw, cu, g_i, g_j);
+    f[i] = xadd(xsub(f[i], xdiv_s(di, w.tau, w.rtau, w.rtau_lo)), g_i);
+    f[j] = xadd(xsub(f[j], xdiv_s(dj, w.tau, w.rtau, w.rtau_lo)), g_j);
+}
+
+template <bool AXIS>
+PSC_HD bool collide_bb_exact_s(double* f, const ExactMomentsS& mo, bool solid, const ExactWin& w) {
+    double ux = solid ? 0.0 : mo.ux, uy = solid ? 0.0 : mo.uy, uz = solid ? 0.0 : mo.uz;
+    const ExactGuo guo = exact_guo_s<AXIS>(w, mo.rho, mo.rrho, 0.0, ux, uy, uz);
+    const double ct = half_div_cs2_s(xadd(xadd(xmul(ux, ux), xmul(uy, uy)), xmul(uz, uz)));
+    {
+        const double d = xsub(f[0], xmul(xmul(W0, mo.rho), xsub(1.0, ct)));
+        f[0] = xadd(xsub(f[0], xdiv_s(d, w.tau, w.rtau, w.rtau_lo)), xmul(w.pw[0], guo.d0));
+    }
+    const double wr1 = xmul(W1, mo.rho), wr2 = xmul(W2, mo.rho);
+    bb_pair_s<0, AXIS>(f, w, wr1, w.pw[1], ct, guo, ux, uy, uz);
+    bb_pair_s<1, AXIS>(f, w, wr1, w.pw[1], ct, guo, ux, uy, uz);
+    bb_pair_s<2, AXIS>(f, w, wr1, w.pw[1], ct, guo, ux, uy, uz);
+    bb_pair_s<3, AXIS>(f, w, wr2, w.pw[2], ct, guo, ux, uy, uz);
+    bb_pair_s<4, AXIS>(f, w, wr2, w.pw[2], ct, guo, ux, uy, uz);
+    bb_pair_s<5, AXIS>(f, w, wr2, w.pw[2], ct, guo, ux, uy, uz);
+    bb_pair_s<6, AXIS>(f, w, wr2, w.pw[2], ct, guo, ux, uy, uz);
+    bb_pair_s<7, AXIS>(f, w, wr2, w.pw[2], ct, guo, ux, uy, uz);
+    bb_pair_s<8, AXIS>(f, w, wr2, w.pw[2], ct, guo, ux, uy, uz);
+    return mo.out | (w.out != 0);
 }
 
 }  // namespace psc

@@ -9,6 +9,7 @@
 #include <stdint.h>
 
 #include <cmath>
+#include <cstring>
 
 #if defined(__CUDACC__)
 #define PSC_HD __host__ __device__ __forceinline__
@@ -71,12 +72,14 @@ PSC_HD double xadd(double a, double b) { return __dadd_rn(a, b); }
 PSC_HD double xsub(double a, double b) { return __dsub_rn(a, b); }
 PSC_HD double xmul(double a, double b) { return __dmul_rn(a, b); }
 PSC_HD double xdiv(double a, double b) { return __ddiv_rn(a, b); }
+PSC_HD double xrcp(double a) { return __drcp_rn(a); }
 #else
 // Host builds compile with -ffp-contract=off; SSE2 double is IEEE binary64.
 PSC_HD double xadd(double a, double b) { return a + b; }
 PSC_HD double xsub(double a, double b) { return a - b; }
 PSC_HD double xmul(double a, double b) { return a * b; }
 PSC_HD double xdiv(double a, double b) { return a / b; }
+PSC_HD double xrcp(double a) { return 1.0 / a; }
 #endif
 
 #if defined(__CUDA_ARCH__)
@@ -130,6 +133,68 @@ PSC_HD Divisor make_divisor(double y) {
     return d;
 }
 PSC_HD double xdiv_d(double x, const Divisor& d) { return d.ok ? xdiv_r(x, d.y, d.r) : xdiv(x, d.y); }
+
+// ---------------------------------------------------------------------------
+// x / c_s^2, x / c_s^4 and x / tau without branches, for the exact kernels.
+//
+// c_s^2 = RN(1/3) = (1 - 2^-54) / 3 and RN(c_s^2 c_s^2) = (1 - 2^-54) / 9, so
+// x / c_s^2 = 3 x (1 + 2^-54 + ...) and x / c_s^4 = 9 x (1 + 2^-54 + ...).  With
+// k = 3 or 9, s = RN(k 2^-54 x) and one rounded FMA k x + s this is a multiplication
+// by a constant held as an unevaluated sum (N. Brisebarre, J.-M. Muller,
+// "Correctly rounded multiplication by arbitrary precision constants", IEEE
+// Trans. Comput. 57(2), 2008).  Its result differs from RN(x / c) only where x / c
+// lies within the rounding of s of a midpoint; for k = 3 and 9 no significand
+// does (the few candidates are enumerated in tests/test_exact_straight_host.py).
+// Two operations instead of the five of xdiv_r.
+// Valid for x = +-0 (which keeps its sign) and 2^-960 <= |x| <= 2^1000.
+// ---------------------------------------------------------------------------
+PSC_HD double div_cs2_s(double x) { return xfma(3.0, x, xmul(x, 0x1.8p-53)); }
+PSC_HD double div_cs2sq_s(double x) { return xfma(9.0, x, xmul(x, 0x1.2p-51)); }
+// (0.5 p) / c_s^2 and (0.5 p) / c_s^4: halving is exact, so it goes into the constants
+PSC_HD double half_div_cs2_s(double p) { return xfma(1.5, p, xmul(p, 0x1.8p-54)); }
+PSC_HD double half_div_cs2sq_s(double p) { return xfma(4.5, p, xmul(p, 0x1.2p-52)); }
+
+// x / y from r = RN(1/y) and rl, 1/y = r + rl to twice the precision: the first
+// quotient RN(x r + RN(x rl)) is within half an ulp and a rounding of rl of x / y,
+// so it is faithful and one correction rounds it correctly (Markstein's theorem,
+// above).  Four operations.  Valid for y in range (div_r_divisor_ok) and
+// x = 0 or 2^-900 <= |x| <= 2^900.
+PSC_HD double xdiv_s(double x, double y, double r, double rl) {
+    const double q = xfma(x, r, xmul(x, rl));
+    return xfma(xfma(-q, y, x), r, q);
+}
+// The same from r alone: xdiv_r without its range test.
+PSC_HD double xdiv_r_s(double x, double y, double r) {
+    const double q0 = xmul(x, r);
+    const double q1 = xfma(xfma(-q0, y, x), r, q0);
+    return xfma(xfma(-q1, y, x), r, q1);
+}
+
+PSC_HD uint32_t hi_word(double x) {
+#if defined(__CUDA_ARCH__)
+    return (uint32_t)__double2hiint(x);
+#else
+    uint64_t b;
+    std::memcpy(&b, &x, sizeof(b));
+    return (uint32_t)(b >> 32);
+#endif
+}
+PSC_HD uint32_t lo_word(double x) {
+#if defined(__CUDA_ARCH__)
+    return (uint32_t)__double2loint(x);
+#else
+    uint64_t b;
+    std::memcpy(&b, &x, sizeof(b));
+    return (uint32_t)b;
+#endif
+}
+// Whether x is neither zero nor in 2^-E <= |x| < 2^E (NaN and infinities included), in integer
+// instructions (the FP64 pipe is what bounds the exact kernels).
+template <int E>
+PSC_HD bool out_of_range(double x) {
+    const uint32_t h = hi_word(x) & 0x7fffffffu;
+    return (h - ((uint32_t)(1023 - E) << 20) >= ((uint32_t)(2 * E) << 20)) & ((h | lo_word(x)) != 0u);
+}
 
 // c * x for a lattice component c in {-1, 0, 1}.  A zero product is returned
 // as +0; it only ever feeds an addition with a non-zero partner or an exact

@@ -25,11 +25,10 @@ inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s
 int sm_count();
 
 constexpr int STEP_THREADS = 256;
-constexpr int MAX_SMEM_WINDOWS = 256;
 
 // launchers (return cudaError_t of the launch)
-cudaError_t launch_step(int store, const psc_window* d_windows, int nwin, int64_t total_tiles, unsigned flags,
-                        bool moving, int grid_ctas, cudaStream_t stream);
+cudaError_t launch_step_exact(const psc_window* d_windows, int nwin, int64_t total_tiles, unsigned flags, bool moving,
+                              int grid_ctas, cudaStream_t stream);
 cudaError_t launch_step_fast(int store, const psc_window* d_windows, int nwin, int64_t total_tiles, unsigned flags,
                              bool moving, int cpt, int grid_ctas, cudaStream_t stream);
 cudaError_t launch_step_tma(int store, const psc_window* d_windows, int nwin, int64_t total_tiles, unsigned flags,

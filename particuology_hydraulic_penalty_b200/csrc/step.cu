@@ -1,190 +1,10 @@
-// Fused pull-stream + PSC-IMB collide kernel over a list of lattice windows.
-//
-// One launch = one lattice step of every window (src/lbm_dem/psc3d.py:208-246):
-//   pull      f_i(x) = f*_i(x - c_i)   (periodic; equivalent to the
-//             reference's push np.roll(f*_i, c_i) at :239-242)
-//   moments   rho, u of the pulled (post-stream) state           (:211-214)
-//   collide   Noble-Torczynski PSC + Guo forcing                  (:215-232)
-//   write     f*_i(x) to the other buffer, optional IMB momentum   (:234-236)
-//   reduce    per-tile FP64 partial sums (flux, porosity, IMB, NaN count)
-//
-// Work decomposition: each window is cut into tiles of STEP_THREADS
-// consecutive cells (flat index (ix*ny + iy)*nz + iz), and a persistent grid
-// (a multiple of the SM count) walks the global tile list.  One thread owns
-// one cell of a tile: every population plane is read and written with
-// consecutive addresses (the +-z pulls are off by one element and hit L1),
-// so each population crosses HBM exactly once per step.
+// Sums of the step kernels' partial rows, and the conversions between stored
+// populations and the reference's post-stream f (src/lbm_dem/psc3d.py:239-242).
 #include "collide.cuh"
 #include "internal.cuh"
 #include "step_common.cuh"
 
 namespace psc {
-
-// The exact FP64 variant is bound by its FP64 dependency chains: two CTAs per SM
-// (at most 128 registers) hide their latency better than one.
-template <int STORE, bool MOVING>
-__global__ void __launch_bounds__(STEP_THREADS, STORE == PSC_STORE_F64_EXACT ? 2 : 1)
-    k_step(const psc_window* __restrict__ wins, int nwin,
-                                                        int64_t total_tiles, unsigned flags) {
-    using TR = StoreTraits<STORE>;
-    using T = typename TR::T;
-    using R = typename TR::R;
-    using O = typename TR::O;
-    __shared__ int64_t s_begin[MAX_SMEM_WINDOWS];
-    static_assert(STEP_THREADS / 32 == PSC_PARTIAL_ROWS, "one partial row per warp");
-    const bool in_smem = nwin <= MAX_SMEM_WINDOWS;
-    if (in_smem) {
-        for (int i = threadIdx.x; i < nwin; i += blockDim.x) s_begin[i] = wins[i].tile_begin;
-    }
-    __syncthreads();
-    const bool do_collide = flags & PSC_STEP_COLLIDE;
-    const bool do_imb = do_collide && (flags & PSC_STEP_IMB);
-    const bool do_mom = flags & PSC_STEP_MOMENTS;
-    const bool do_red = flags & PSC_STEP_REDUCE;
-
-    for (int64_t t = blockIdx.x; t < total_tiles; t += gridDim.x) {
-        const int wi = find_window(wins, in_smem ? s_begin : nullptr, nwin, t);
-        const psc_window& W = wins[wi];
-        if (W.flags & PSC_WIN_INACTIVE) continue;  // block-uniform
-        const int nx = W.nx, ny = W.ny, nz = W.nz;
-        const uint32_t N = (uint32_t)nx * (uint32_t)ny * (uint32_t)nz;
-        const int64_t local_tile = t - W.tile_begin;
-        const uint32_t cell = (uint32_t)(local_tile * W.tile_cells) + threadIdx.x;
-        const bool valid = cell < N;
-        double red[PSC_NRED];
-#pragma unroll
-        for (int k = 0; k < PSC_NRED; ++k) red[k] = 0.0;
-
-        if (valid) {
-            const uint32_t iz = cell % (uint32_t)nz;
-            const uint32_t rr = cell / (uint32_t)nz;
-            const uint32_t iy = rr % (uint32_t)ny;
-            const uint32_t ix = rr / (uint32_t)ny;
-            const bool open_x = (W.flags & PSC_WIN_OPEN_X) != 0;
-            const NbrOffsets nb = nbr_offsets(ix, iy, iz, nx, ny, nz, open_x);
-            const bool moving = MOVING && (W.flags & PSC_WIN_MOVING) && W.us != nullptr;
-            R f[Q];
-            const R scale = TR::scaled ? (R)W.store_scale : R(1);
-            PullLoop<T, R, Q>::run(f, reinterpret_cast<const T*>(W.f_src), N, cell, nb, R(1) / scale, TR::scaled);
-            if (open_x && ix == 0) {  // velocity inlet: bounce-back of the node's own opp(i) + momentum term
-                const T* srcT = reinterpret_cast<const T*>(W.f_src);
-#pragma unroll
-                for (int i = 0; i < Q; ++i) {
-                    if (!enters_x0(i)) continue;
-                    const R back = ld_pop(srcT + (size_t)opp(i) * N + cell);
-                    const double corr =
-                        inlet_correction_exact(i, W.inlet_rho, W.inlet_u[0], W.inlet_u[1], W.inlet_u[2]);
-                    if constexpr (TR::exact) f[i] = xadd((double)back, corr);
-                    else f[i] = (TR::scaled ? back / scale : back) + (R)corr;
-                }
-            }
-            O* mom = reinterpret_cast<O*>(W.moments);
-            O* imbp = reinterpret_cast<O*>(W.imb);
-            const O* usp = reinterpret_cast<const O*>(W.us);
-            double rho_d, ux_d, uy_d, uz_d, solid_d;
-            double imb_d[3] = {0.0, 0.0, 0.0};
-            if constexpr (TR::exact) {
-                const double hfx = xmul(0.5, W.force[0]), hfy = xmul(0.5, W.force[1]), hfz = xmul(0.5, W.force[2]);
-                const ExactMoments mo = moments_exact(f, hfx, hfy, hfz);
-                rho_d = mo.rho;
-                ux_d = mo.ux;
-                uy_d = mo.uy;
-                uz_d = mo.uz;
-                solid_d = W.solid[cell];
-                if (do_collide) {
-                    double usx = 0.0, usy = 0.0, usz = 0.0;
-                    if (moving) {
-                        usx = usp[cell];
-                        usy = usp[(size_t)N + cell];
-                        usz = usp[2 * (size_t)N + cell];
-                    }
-                    collide_exact(f, mo, solid_d, moving, usx, usy, usz, W.tau, W.force[0], W.force[1], W.force[2],
-                                  hfx, hfy, hfz, imb_d);
-                }
-            } else {
-                const FastMoments<R> mo = moments_fast(f);
-                const R irho = R(1) / mo.rho;
-                const R fx = (R)W.force[0], fy = (R)W.force[1], fz = (R)W.force[2];
-                const R ux = (mo.mx + R(0.5) * fx) * irho;
-                const R uy = (mo.my + R(0.5) * fy) * irho;
-                const R uz = (mo.mz + R(0.5) * fz) * irho;
-                rho_d = (double)mo.rho;
-                ux_d = (double)ux;
-                uy_d = (double)uy;
-                uz_d = (double)uz;
-                const int s = W.subsamples;
-                const int s3 = s * s * s;
-                // uint8 clipped sample level; without one (smooth geometry) the FP64 solid field
-                const R al = W.level ? (R)W.level[cell] / (R)s3 : (R)W.solid[cell];
-                solid_d = (double)al;
-                if (do_collide) {
-                    const R tau = (R)W.tau;
-                    const R B = al / (al + tau * (R(1) - al) + R(1.0e-14));
-                    FastParams<R> p;
-                    p.inv_tau = R(1) / tau;
-                    p.pref = R(1) - R(0.5) / tau;
-                    p.fx = fx;
-                    p.fy = fy;
-                    p.fz = fz;
-                    R usx = R(0), usy = R(0), usz = R(0);
-                    if (moving) {
-                        usx = (R)usp[cell];
-                        usy = (R)usp[(size_t)N + cell];
-                        usz = (R)usp[2 * (size_t)N + cell];
-                    }
-                    R im[3];
-                    if (do_imb || do_red) {
-                        if (moving) collide_fast<R, MOVING, true>(f, mo, irho, B, usx, usy, usz, p, im);
-                        else collide_fast<R, false, true>(f, mo, irho, B, usx, usy, usz, p, im);
-                        imb_d[0] = (double)im[0];
-                        imb_d[1] = (double)im[1];
-                        imb_d[2] = (double)im[2];
-                    } else {
-                        if (moving) collide_fast<R, MOVING, false>(f, mo, irho, B, usx, usy, usz, p, im);
-                        else collide_fast<R, false, false>(f, mo, irho, B, usx, usy, usz, p, im);
-                    }
-                }
-            }
-            if (do_mom) {
-                mom[cell] = (O)rho_d;
-                mom[(size_t)N + cell] = (O)ux_d;
-                mom[2 * (size_t)N + cell] = (O)uy_d;
-                mom[3 * (size_t)N + cell] = (O)uz_d;
-            }
-            if (do_collide) {
-                T* dst = reinterpret_cast<T*>(W.f_dst);
-#pragma unroll
-                for (int i = 0; i < Q; ++i) st_pop(dst + (size_t)i * N + cell, TR::scaled ? f[i] * scale : f[i]);
-                if (do_imb) {
-                    imbp[cell] = (O)imb_d[0];
-                    imbp[(size_t)N + cell] = (O)imb_d[1];
-                    imbp[2 * (size_t)N + cell] = (O)imb_d[2];
-                }
-            }
-            if (do_red) {
-                const double fl = 1.0 - solid_d;
-                red[PSC_RED_RHO] = rho_d;
-                red[PSC_RED_UX] = ux_d;
-                red[PSC_RED_UY] = uy_d;
-                red[PSC_RED_UZ] = uz_d;
-                red[PSC_RED_FLUID_UX] = fl * ux_d;
-                red[PSC_RED_FLUID_UY] = fl * uy_d;
-                red[PSC_RED_FLUID_UZ] = fl * uz_d;
-                red[PSC_RED_FLUID] = fl;
-                red[PSC_RED_IMBX] = imb_d[0];
-                red[PSC_RED_IMBY] = imb_d[1];
-                red[PSC_RED_IMBZ] = imb_d[2];
-                red[PSC_RED_NONFINITE] =
-                    (isfinite(rho_d) && isfinite(ux_d) && isfinite(uy_d) && isfinite(uz_d)) ? 0.0 : 1.0;
-                red[PSC_RED_SOLID] = solid_d;
-            }
-        }
-        if (do_red) {  // one row per warp and tile; the block of local tile 0 writes the header
-            warp_reduce_store<PSC_NRED>(red, W.partials + (1 + local_tile * PSC_PARTIAL_ROWS) * PSC_NRED);
-            if (local_tile == 0 && threadIdx.x == 0) W.partials[0] = (double)(W.tile_count * PSC_PARTIAL_ROWS);
-        }
-    }
-}
 
 // Window sums of the partial rows (header row: element 0 = row count; the
 // rows follow it), deterministic, in two launches:
@@ -340,46 +160,6 @@ __global__ void k_stream_pull_store(const double* src, void* dst, int nx, int ny
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-template <int STORE, bool MOVING>
-static cudaError_t launch_step_t(const psc_window* d_windows, int nwin, int64_t total_tiles, unsigned flags,
-                                 int grid_ctas, cudaStream_t stream) {
-    if (grid_ctas <= 0) {
-        static int per_sm[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        int dev = 0;
-        cudaGetDevice(&dev);
-        int& occ = per_sm[dev & 7];
-        if (occ == 0) {
-            cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_step<STORE, MOVING>, STEP_THREADS, 0);
-            if (e != cudaSuccess) return e;
-            if (occ <= 0) occ = 1;
-        }
-        const int64_t g = (int64_t)sm_count() * occ;
-        grid_ctas = (int)(total_tiles < g ? total_tiles : g);
-    }
-    if ((int64_t)grid_ctas > total_tiles) grid_ctas = (int)total_tiles;
-    if (grid_ctas <= 0) return cudaSuccess;
-    k_step<STORE, MOVING><<<grid_ctas, STEP_THREADS, 0, stream>>>(d_windows, nwin, total_tiles, flags);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_step(int store, const psc_window* d_windows, int nwin, int64_t total_tiles, unsigned flags,
-                        bool moving, int grid_ctas, cudaStream_t stream) {
-#define PSC_STEP_CASE(S)                                                                                          \
-    case S:                                                                                                       \
-        return moving ? launch_step_t<S, true>(d_windows, nwin, total_tiles, flags, grid_ctas, stream)           \
-                      : launch_step_t<S, false>(d_windows, nwin, total_tiles, flags, grid_ctas, stream);
-    switch (store) {
-        PSC_STEP_CASE(PSC_STORE_F64_EXACT)
-        PSC_STEP_CASE(PSC_STORE_F64)
-        PSC_STEP_CASE(PSC_STORE_F32)
-        PSC_STEP_CASE(PSC_STORE_F16)
-        PSC_STEP_CASE(PSC_STORE_BF16)
-        default:
-            return cudaErrorInvalidValue;
-    }
-#undef PSC_STEP_CASE
-}
-
 cudaError_t launch_reduce_windows(const psc_window* d_windows, int nwin, double* out, cudaStream_t stream) {
     k_reduce_segments<<<dim3(REDUCE_SEG_BLOCKS, (unsigned)nwin), STEP_THREADS, 0, stream>>>(d_windows);
     cudaError_t e = cudaGetLastError();

@@ -113,19 +113,14 @@ __device__ __forceinline__ int32_t pull_offset(const NbrOffsets& o) {
            (czv(I) == 1 ? o.zm : (czv(I) == -1 ? o.zp : 0));
 }
 
-template <typename T, typename R, int I>
-struct PullLoop {
-    __device__ __forceinline__ static void run(R* f, const T* src, size_t N, uint32_t cell, const NbrOffsets& o,
-                                               R inv_scale, bool scaled) {
-        PullLoop<T, R, I - 1>::run(f, src, N, cell, o, inv_scale, scaled);
-        const R v = ld_pop(src + (size_t)(I - 1) * N + (size_t)((int64_t)cell + pull_offset<I - 1>(o)));
-        f[I - 1] = scaled ? v * inv_scale : v;
-    }
-};
-template <typename T, typename R>
-struct PullLoop<T, R, 0> {
-    __device__ __forceinline__ static void run(R*, const T*, size_t, uint32_t, const NbrOffsets&, R, bool) {}
-};
+// The constants of the exact arithmetic, by the block: each warp makes a part.
+__device__ __forceinline__ void make_exact_win_block(ExactWin& w, double tau, double fx, double fy, double fz) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp == 1 && lane == 0) exact_win_force(w, tau, fx, fy, fz);
+    if (warp == 2 && lane == 0) exact_win_tau(w, tau);
+    if (warp == 3 && lane == 0) exact_win_guo(w, tau);
+    if (warp == 4 && lane == 0) exact_win_pairs(w, fx, fy, fz);
+}
 
 __device__ __forceinline__ int find_window(const psc_window* wins, const int64_t* s_begin, int nwin, int64_t t) {
     int lo = 0, hi = nwin - 1;

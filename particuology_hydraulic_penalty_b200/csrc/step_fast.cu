@@ -1,6 +1,6 @@
 // Throughput kernel for the deviation storage modes (F64 / F32 / F16 / BF16).
 //
-// Same step as k_step (pull-stream + PSC-IMB collide, src/lbm_dem/psc3d.py:
+// The step of psc_step_windows (pull-stream + PSC-IMB collide, src/lbm_dem/psc3d.py:
 // 208-246), organised to keep the SM's issue slots for the collision:
 //  * each persistent CTA owns a CONTIGUOUS run of tiles, so it meets a new
 //    window only a few times; per-window constants (Guo terms, 1/tau, the

@@ -10,6 +10,7 @@
 // Exact FP64 arithmetic in the reference's operation order.
 #include "collide.cuh"
 #include "internal.cuh"
+#include "step_common.cuh"
 
 namespace psc {
 
@@ -42,45 +43,104 @@ __global__ void k_vox_spheres(const double* __restrict__ pts, int M, double lox,
     }
 }
 
-__global__ void __launch_bounds__(256) k_bb_step(const double* __restrict__ src, double* __restrict__ dst,
-                                                  const uint8_t* __restrict__ solid, int nx, int ny, int nz,
-                                                  double tau, double fx, double fy, double fz, unsigned flags,
-                                                  double* __restrict__ mom) {
-    const uint32_t N = (uint32_t)nx * ny * nz;
-    const bool do_collide = flags & PSC_STEP_COLLIDE;
-    const bool do_mom = flags & PSC_STEP_MOMENTS;
-    for (uint32_t cell = blockIdx.x * blockDim.x + threadIdx.x; cell < N; cell += gridDim.x * blockDim.x) {
-        const uint32_t iz = cell % nz, r = cell / nz, iy = r % ny, ix = r / ny;
-        const int32_t nyz = ny * nz;
-        const int32_t xm = ix == 0 ? (nx - 1) * nyz : -nyz, xp = ix == (uint32_t)(nx - 1) ? -(nx - 1) * nyz : nyz;
-        const int32_t ym = iy == 0 ? (ny - 1) * nz : -nz, yp = iy == (uint32_t)(ny - 1) ? -(ny - 1) * nz : nz;
-        const int32_t zm = iz == 0 ? nz - 1 : -1, zp = iz == (uint32_t)(nz - 1) ? -(nz - 1) : 1;
+struct BbArgs {
+    const double* src;
+    double* dst;
+    const uint8_t* solid;
+    double* mom;
+    int32_t nx, ny, nz;
+    double tau, fx, fy, fz;
+    unsigned flags;
+};
+
+__device__ __forceinline__ void bb_pull(const BbArgs& a, uint32_t N, uint32_t cell, const NbrOffsets& o,
+                                        double (&f)[Q]) {
+    const double* p = a.src + cell;  // 64-bit: a window may hold up to 2^31 cells per plane
+#pragma unroll
+    for (int i = 0; i < Q; ++i) {
+        const int32_t off = (cxv(i) == 1 ? o.xm : (cxv(i) == -1 ? o.xp : 0)) +
+                            (cyv(i) == 1 ? o.ym : (cyv(i) == -1 ? o.yp : 0)) +
+                            (czv(i) == 1 ? o.zm : (czv(i) == -1 ? o.zp : 0));
+        f[i] = ld_pop(p + (int64_t)off);
+        p += N;
+    }
+}
+
+// A cell whose operands left the range of the branch-free forms: pulled again, general forms.
+struct BbCell {
+    double f[Q], mom[4];
+};
+
+__device__ __noinline__ void bb_cell_general(const BbArgs& a, uint32_t N, uint32_t cell, NbrOffsets o, bool solid,
+                                             BbCell& r) {
+    double f[Q], m[4];
+    bb_pull(a, N, cell, o, f);
+    if (solid) bounce_solid_as_reference(f);
+    if (a.flags & PSC_STEP_COLLIDE) {
+        collide_bb_exact(f, solid, a.tau, a.fx, a.fy, a.fz, m);
+    } else {
+        const ExactMoments mo = moments_exact(f, xmul(0.5, a.fx), xmul(0.5, a.fy), xmul(0.5, a.fz));
+        m[0] = mo.rho;
+        m[1] = solid ? 0.0 : mo.ux;
+        m[2] = solid ? 0.0 : mo.uy;
+        m[3] = solid ? 0.0 : mo.uz;
+    }
+    for (int i = 0; i < Q; ++i) r.f[i] = f[i];
+    for (int k = 0; k < 4; ++k) r.mom[k] = m[k];
+}
+
+// One cell per thread of a grid-stride loop, two CTAs per SM (128 registers): bound by the FP64 pipe
+// like k_step_exact, whose branch-free forms it shares (64^3: 15 us a step, 32.5 with a branch per division).
+__global__ void __launch_bounds__(256, 2) k_bb_step(const __grid_constant__ BbArgs a) {
+    __shared__ ExactWin w;
+    make_exact_win_block(w, a.tau, a.fx, a.fy, a.fz);
+    __syncthreads();
+    const uint32_t N = (uint32_t)a.nx * a.ny * a.nz;
+    const bool do_collide = a.flags & PSC_STEP_COLLIDE;
+    const bool do_mom = a.flags & PSC_STEP_MOMENTS;
+    const uint32_t ny = (uint32_t)a.ny, nz = (uint32_t)a.nz;
+    const uint32_t stride = gridDim.x * blockDim.x;
+    uint32_t cell = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t iz = cell % nz, r = cell / nz, iy = r % ny, ix = r / ny;
+    const uint32_t step_z = stride % nz, q = stride / nz, step_y = q % ny, step_x = q / ny;
+    for (; cell < N; cell += stride) {
+        const NbrOffsets o = nbr_offsets(ix, iy, iz, a.nx, a.ny, a.nz);
         double f[Q];
-#pragma unroll
-        for (int i = 0; i < Q; ++i) {
-            const int32_t o = (cxv(i) == 1 ? xm : (cxv(i) == -1 ? xp : 0)) +
-                              (cyv(i) == 1 ? ym : (cyv(i) == -1 ? yp : 0)) +
-                              (czv(i) == 1 ? zm : (czv(i) == -1 ? zp : 0));
-            f[i] = src[(size_t)i * N + (size_t)((int64_t)cell + o)];
-        }
-        const bool s = solid[cell] != 0;
+        bb_pull(a, N, cell, o, f);
+        const bool s = a.solid[cell] != 0;
         if (s) bounce_solid_as_reference(f);
-        double m[4];
-        if (do_collide) {
-            collide_bb_exact(f, s, tau, fx, fy, fz, m);
+        const ExactMomentsS mo = moments_exact_s(f, w.hfx, w.hfy, w.hfz);
+        double m[4] = {mo.rho, s ? 0.0 : mo.ux, s ? 0.0 : mo.uy, s ? 0.0 : mo.uz};
+        bool out = mo.out;
+        if (do_collide) out = w.axis >= 0 ? collide_bb_exact_s<true>(f, mo, s, w) : collide_bb_exact_s<false>(f, mo, s, w);
+        if (out) {
+            BbCell g;
+            bb_cell_general(a, N, cell, o, s, g);
 #pragma unroll
-            for (int i = 0; i < Q; ++i) dst[(size_t)i * N + cell] = f[i];
-        } else {
-            ExactMoments mo = moments_exact(f, xmul(0.5, fx), xmul(0.5, fy), xmul(0.5, fz));
-            m[0] = mo.rho;
-            m[1] = s ? 0.0 : mo.ux;
-            m[2] = s ? 0.0 : mo.uy;
-            m[3] = s ? 0.0 : mo.uz;
+            for (int i = 0; i < Q; ++i) f[i] = g.f[i];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) m[k] = g.mom[k];
+        }
+        if (do_collide) {
+            double* p = a.dst + cell;
+#pragma unroll
+            for (int i = 0; i < Q; ++i) {
+                *p = f[i];
+                p += N;
+            }
         }
         if (do_mom) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) mom[(size_t)k * N + cell] = m[k];
+            for (int k = 0; k < 4; ++k) a.mom[(size_t)k * N + cell] = m[k];
         }
+        // the stride's own (x, y, z) digits with carries
+        iz += step_z;
+        const uint32_t cz = iz >= nz;
+        iz -= cz ? nz : 0u;
+        iy += step_y + cz;
+        const uint32_t cy = iy >= ny;
+        iy -= cy ? ny : 0u;
+        ix += step_x + cy;
     }
 }
 
@@ -95,9 +155,10 @@ cudaError_t launch_bb_step(const double* src, double* dst, const uint8_t* solid,
                            double fx, double fy, double fz, unsigned flags, double* mom, cudaStream_t s) {
     const int64_t N = (int64_t)nx * ny * nz;
     int64_t g = (N + 255) / 256;
-    const int64_t cap = (int64_t)sm_count() * 8;
+    const int64_t cap = (int64_t)sm_count() * 2;  // resident CTAs
     if (g > cap) g = cap;
-    k_bb_step<<<(unsigned)g, 256, 0, s>>>(src, dst, solid, nx, ny, nz, tau, fx, fy, fz, flags, mom);
+    const BbArgs a = {src, dst, solid, mom, nx, ny, nz, tau, fx, fy, fz, flags};
+    k_bb_step<<<(unsigned)g, 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 
