@@ -118,8 +118,8 @@ typedef struct psc_launch {
  * tile_count * PSC_PARTIAL_ROWS rows of PSC_NRED doubles.  The persistent
  * kernels accumulate each thread's cells over the CTA's whole run of tiles
  * inside the window and write one row per warp and CTA (no per-tile
- * reduction, no block barrier); the exact kernel writes one row per warp and
- * tile.  Sums are deterministic for a given launch configuration. */
+ * reduction, no block barrier).  Sums are deterministic for a given launch
+ * configuration. */
 #define PSC_PARTIAL_ROWS 8
 
 /* Diagnostics written by psc_particle_loads() (psc3d.py:247-253). */
@@ -295,9 +295,7 @@ int psc_step_windows(int store, const struct psc_window* d_windows, int nwin, in
 int psc_step_windows_ex(int store, const struct psc_window* d_windows, int nwin, int64_t total_tiles, unsigned flags,
                 const psc_launch* cfg, void* stream);
 /* Sum the per-tile partials of each window in a fixed order (deterministic)
- * into out[nwin][PSC_NRED] (device).  The partials are consumed: segment sums
- * are written over them, so reduce once per PSC_STEP_REDUCE pass.  nwin must
- * not exceed 65535. */
+ * into out[nwin][PSC_NRED] (device).  nwin must not exceed 65535. */
 int psc_reduce_windows(const struct psc_window* d_windows, int nwin, double* out, void* stream);
 
 /* ---- particle loads (psc3d.py:255-281 / 375-407) ------------------------ */

@@ -21,6 +21,8 @@
 //            clip to the solid fraction, clipped integer level
 //   loads    chunks of bbox entries per particle, deterministic block sums,
 //            then a fixed-order per-particle sum of the chunk partials
+#include <cooperative_groups.h>
+
 #include "collide.cuh"
 #include "internal.cuh"
 
@@ -178,9 +180,10 @@ __device__ __forceinline__ double smooth_alpha(int32_t ix, int32_t iy, int32_t i
 }
 
 // Descriptor of one load-reduction chunk, computed by k_chunk_desc (one
-// thread per chunk, so the lookups of many chunks overlap) into the chunk's
-// own partial row (6 doubles); every thread of the chunk's block reads it
-// before the chunk's last warp overwrites the row with the sums.
+// thread per chunk, so the lookups of many chunks overlap) into an array that
+// is kept with the geometry, or into the chunk's own partial row (6 doubles):
+// every thread of the chunk's block reads it before the chunk's last warp
+// overwrites the row with the sums.
 struct ChunkDesc {
     int64_t e0, e1;       // entry range
     int32_t p;            // particle
@@ -656,7 +659,7 @@ __device__ __forceinline__ void chunk_thread_sums(const ChunkDesc& dsc, const do
 // One block per chunk of one particle's bbox entries.
 template <typename I>
 __global__ void __launch_bounds__(LOAD_THREADS, PSC_LOADS_MIN_BLOCKS) k_loads_chunks(psc_geometry g, const I* imb,
-                                                                                 double* part) {
+                                                                                 const double* desc, double* part) {
     __shared__ ChunkRing rows;
     __shared__ LoadRing<I> ring;
     extern __shared__ double s_al[];  // S^3 + 1 entries (dynamic)
@@ -669,7 +672,7 @@ __global__ void __launch_bounds__(LOAD_THREADS, PSC_LOADS_MIN_BLOCKS) k_loads_ch
     long long j = 0;
     for (int64_t chunk = blockIdx.x; chunk < C; chunk += gridDim.x, ++j) {  // every warp, in this order
         // every thread reads the chunk's descriptor before the chunk's last warp overwrites the row
-        const ChunkDesc dsc = *reinterpret_cast<const ChunkDesc*>(part + chunk * 6);
+        const ChunkDesc dsc = *reinterpret_cast<const ChunkDesc*>(desc + chunk * 6);
         double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
         chunk_thread_sums<I>(dsc, g.particles, g.ent_cnt, g.capacity_entries, g.alpha_sum, imb, N, (uint32_t)g.ny,
                              (uint32_t)g.nz, s_al, ring, acc);
@@ -776,7 +779,8 @@ __device__ __forceinline__ void list_chunk_sums(const ListCursor& cur, int64_t s
 // the next chunk's first list copy as soon as its own sums are done (its stage
 // slots are free then), before its warp's sum.
 template <typename I>
-__global__ void __launch_bounds__(LOAD_THREADS, 3) k_loads_chunks_list(psc_geometry g, const I* imb, double* part) {
+__global__ void __launch_bounds__(LOAD_THREADS, 3) k_loads_chunks_list(psc_geometry g, const I* imb,
+                                                                         const double* desc, double* part) {
     __shared__ ChunkRing rows;
     extern __shared__ __align__(16) unsigned char list_stage[];
     chunk_ring_init(rows);
@@ -785,7 +789,7 @@ __global__ void __launch_bounds__(LOAD_THREADS, 3) k_loads_chunks_list(psc_geome
     ListCursor cur{};
     int64_t chunk = blockIdx.x;
     if (chunk < C) {
-        cur.dsc = *reinterpret_cast<const ChunkDesc*>(part + chunk * 6);
+        cur.dsc = *reinterpret_cast<const ChunkDesc*>(desc + chunk * 6);
         cur.n_t = g.load_n[chunk * LOAD_THREADS + threadIdx.x];
         list_issue(chunk * g.chunk_entries + threadIdx.x, g.load_w, g.load_abk, 0, list_pass_size(cur.n_t, 0),
                    list_stage);
@@ -795,7 +799,7 @@ __global__ void __launch_bounds__(LOAD_THREADS, 3) k_loads_chunks_list(psc_geome
         const int64_t nxt = chunk + gridDim.x;
         ListCursor nc{};
         if (nxt < C) {
-            nc.dsc = *reinterpret_cast<const ChunkDesc*>(part + nxt * 6);
+            nc.dsc = *reinterpret_cast<const ChunkDesc*>(desc + nxt * 6);
             nc.n_t = g.load_n[nxt * LOAD_THREADS + threadIdx.x];
         }
         double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
@@ -855,7 +859,7 @@ __device__ __forceinline__ void chunk_list_build(const ChunkDesc& dsc, const uin
 
 // The loads list of every chunk of one geometry (descriptors in the partial rows).
 __global__ void __launch_bounds__(LOAD_THREADS) k_loads_list_build(const __grid_constant__ psc_geometry g,
-                                                                   const double* part) {
+                                                                   const double* desc) {
     extern __shared__ double s_al[];  // S^3 + 1 entries (dynamic)
     const int S3 = g.subsamples * g.subsamples * g.subsamples;
     const double S3d = (double)S3;
@@ -864,7 +868,7 @@ __global__ void __launch_bounds__(LOAD_THREADS) k_loads_list_build(const __grid_
     const int64_t C = g.totals[1];
     const int64_t E = min(g.totals[0], g.capacity_entries);
     for (int64_t chunk = blockIdx.x; chunk < C; chunk += gridDim.x) {
-        const ChunkDesc dsc = *reinterpret_cast<const ChunkDesc*>(part + chunk * 6);
+        const ChunkDesc dsc = *reinterpret_cast<const ChunkDesc*>(desc + chunk * 6);
         chunk_list_build(dsc, g.ent_cnt, E, g.alpha_sum, (uint32_t)g.ny, (uint32_t)g.nz, s_al, g.chunk_entries,
                          g.load_w, g.load_abk, chunk * g.chunk_entries, g.load_n + chunk * LOAD_THREADS);
     }
@@ -873,12 +877,12 @@ __global__ void __launch_bounds__(LOAD_THREADS) k_loads_list_build(const __grid_
 // The loads lists of the jobs whose list is not current, in one launch.
 __global__ void __launch_bounds__(LOAD_THREADS) k_loads_list_build_multi(const LoadsJob* jobs,
                                                                          const int64_t* chunk_base, int njobs,
-                                                                         const double* part) {
+                                                                         const double* desc) {
     extern __shared__ double s_al[];  // S^3 + 1 entries for the largest S of the jobs (dynamic)
     const int64_t C = chunk_base[njobs];
     int cur_S = 0;  // S of the table in s_al (block-uniform: every thread visits the same chunks)
     for (int64_t chunk = blockIdx.x; chunk < C; chunk += gridDim.x) {
-        const ChunkDesc dsc = *reinterpret_cast<const ChunkDesc*>(part + chunk * 6);
+        const ChunkDesc dsc = *reinterpret_cast<const ChunkDesc*>(desc + chunk * 6);
         const psc_geometry& g = jobs[dsc.pad].g;
         if (g.list_ready) continue;  // block-uniform
         const int S = g.subsamples;
@@ -900,9 +904,10 @@ __global__ void __launch_bounds__(LOAD_THREADS) k_loads_list_build_multi(const L
 // Per-particle sums of the chunk partials c0 .. c1-1: one warp per particle,
 // lane l sums chunks c0 + l, c0 + l + 32, ... in order, then a fixed shuffle tree.
 __device__ __forceinline__ void particle_sums(const double* part, int64_t c0, int64_t c1, double* force,
-                                              double* torque) {
+                                              double* torque, double (&F)[6]) {
     const int lane = threadIdx.x & 31;
-    double F[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < 6; ++k) F[k] = 0.0;
     for (int64_t c = c0 + lane; c < c1; c += 32) {
 #pragma unroll
         for (int k = 0; k < 6; ++k) F[k] += part[c * 6 + k];
@@ -912,9 +917,9 @@ __device__ __forceinline__ void particle_sums(const double* part, int64_t c0, in
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) F[k] += __shfl_xor_sync(0xffffffffu, F[k], o);
     }
-    if (lane < 3) {
-        force[lane] = F[lane];
-        torque[lane] = F[3 + lane];
+    if (lane < 3) {  // (every lane holds the sums)
+        force[lane] = lane == 0 ? F[0] : (lane == 1 ? F[1] : F[2]);
+        torque[lane] = lane == 0 ? F[3] : (lane == 1 ? F[4] : F[5]);
     }
 }
 
@@ -922,13 +927,32 @@ __global__ void __launch_bounds__(256) k_loads_particles(psc_geometry g, const d
                                                          double* torques) {
     const int p = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
     if (p >= g.nparticles) return;  // warp-uniform
-    particle_sums(part, g.chunk_off[p], g.chunk_off[p + 1], forces + (size_t)p * 3, torques + (size_t)p * 3);
+    double F[6];
+    particle_sums(part, g.chunk_off[p], g.chunk_off[p + 1], forces + (size_t)p * 3, torques + (size_t)p * 3, F);
+}
+
+__device__ __forceinline__ void write_loads_diag(const double (&r)[5], const double* imb_sums, double* diag,
+                                                 double* host_diag) {
+    const double cx = r[0] + imb_sums[0], cy = r[1] + imb_sums[1], cz = r[2] + imb_sums[2];
+    double d[PSC_NDIAG];
+    d[PSC_DIAG_MOMENTUM_RESIDUAL] = sqrt(cx * cx + cy * cy + cz * cz);
+    d[PSC_DIAG_MAX_FORCE] = sqrt(r[3]);
+    d[PSC_DIAG_MAX_TORQUE] = sqrt(r[4]);
+    d[PSC_DIAG_FORCE_SUM_X] = r[0];
+    d[PSC_DIAG_FORCE_SUM_Y] = r[1];
+    d[PSC_DIAG_FORCE_SUM_Z] = r[2];
+#pragma unroll
+    for (int k = 0; k < PSC_NDIAG; ++k) diag[k] = d[k];
+    if (host_diag) {
+#pragma unroll
+        for (int k = 0; k < PSC_NDIAG; ++k) host_diag[k] = d[k];
+    }
 }
 
 // One block: the closure residual |sum_p F_p + sum_x imb| and the max force /
 // torque norms (psc3d.py:247-253, :280-281) from the per-particle loads.
 __device__ __forceinline__ void loads_diag_block(int P, const double* imb_sums, const double* forces,
-                                                 const double* torques, double* diag) {
+                                                 const double* torques, double* diag, double* host_diag) {
     __shared__ double s[32][5];
     double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // sum Fx, Fy, Fz, max |F|^2, max |T|^2
     for (int p = threadIdx.x; p < P; p += blockDim.x) {
@@ -958,19 +982,73 @@ __device__ __forceinline__ void loads_diag_block(int P, const double* imb_sums, 
             r[3] = fmax(r[3], s[w][3]);
             r[4] = fmax(r[4], s[w][4]);
         }
-        const double cx = r[0] + imb_sums[0], cy = r[1] + imb_sums[1], cz = r[2] + imb_sums[2];
-        diag[PSC_DIAG_MOMENTUM_RESIDUAL] = sqrt(cx * cx + cy * cy + cz * cz);
-        diag[PSC_DIAG_MAX_FORCE] = sqrt(r[3]);
-        diag[PSC_DIAG_MAX_TORQUE] = sqrt(r[4]);
-        diag[PSC_DIAG_FORCE_SUM_X] = r[0];
-        diag[PSC_DIAG_FORCE_SUM_Y] = r[1];
-        diag[PSC_DIAG_FORCE_SUM_Z] = r[2];
+        write_loads_diag(r, imb_sums, diag, host_diag);
     }
 }
 
+// Per-particle sums and the diagnostics of one window by one cluster, a warp per particle in turn: one
+// launch where a kernel over the particles and a one-block kernel over the forces were two (2.1 + 3.4 us
+// with 128 particles, 3.2 + 5.4 us with 1136).  For windows of up to FINAL_PARTICLES particles: beyond, a
+// cluster's 256 warps take more turns than the whole GPU's.
+constexpr int FINAL_CTAS = 8;
+constexpr int FINAL_THREADS = 1024;
+constexpr int FINAL_PARTICLES = 4096;
+
+__device__ __forceinline__ void loads_final_cluster(int P, const int64_t* chunk_off, const double* part,
+                                                    const double* imb_sums, double* forces, double* torques,
+                                                    double* diag, double* host_diag) {
+    namespace cg = cooperative_groups;
+    __shared__ double s_w[FINAL_THREADS / 32][5];
+    __shared__ double s_cta[5];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // sum Fx, Fy, Fz, max |F|^2, max |T|^2
+    for (int p = (int)cluster.block_rank() * (FINAL_THREADS / 32) + warp; p < P; p += FINAL_CTAS * (FINAL_THREADS / 32)) {
+        double F[6];
+        particle_sums(part, chunk_off[p], chunk_off[p + 1], forces + (size_t)p * 3, torques + (size_t)p * 3, F);
+        v[0] += F[0];
+        v[1] += F[1];
+        v[2] += F[2];
+        v[3] = fmax(v[3], F[0] * F[0] + F[1] * F[1] + F[2] * F[2]);
+        v[4] = fmax(v[4], F[3] * F[3] + F[4] * F[4] + F[5] * F[5]);
+    }
+    if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) s_w[warp][k] = v[k];
+    }
+    __syncthreads();
+    if (warp < 5) {  // a warp per value: the CTA's warps by a shuffle tree
+        double x = s_w[lane][warp];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double y = __shfl_xor_sync(0xffffffffu, x, o);
+            x = warp < 3 ? x + y : fmax(x, y);
+        }
+        if (lane == 0) s_cta[warp] = x;
+    }
+    cluster.sync();
+    if (cluster.block_rank() == 0 && threadIdx.x == 0) {
+        double r[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        for (int j = 0; j < FINAL_CTAS; ++j) {
+            const double* s = cluster.map_shared_rank(s_cta, j);
+            for (int k = 0; k < 3; ++k) r[k] += s[k];
+            r[3] = fmax(r[3], s[3]);
+            r[4] = fmax(r[4], s[4]);
+        }
+        write_loads_diag(r, imb_sums, diag, host_diag);
+    }
+    cluster.sync();  // the CTAs' values stay in place until they are read
+}
+
+__global__ void __cluster_dims__(FINAL_CTAS, 1, 1) __launch_bounds__(FINAL_THREADS)
+    k_loads_final(const __grid_constant__ psc_geometry g, const double* part, const double* imb_sums, double* forces,
+                  double* torques, double* diag, double* host_diag) {
+    loads_final_cluster(g.nparticles, g.chunk_off, part, imb_sums, forces, torques, diag, host_diag);
+}
+
 __global__ void __launch_bounds__(1024) k_loads_diag(psc_geometry g, const double* imb_sums, const double* forces,
-                                                     const double* torques, double* diag) {
-    loads_diag_block(g.nparticles, imb_sums, forces, torques, diag);
+                                                     const double* torques, double* diag, double* host_diag) {
+    loads_diag_block(g.nparticles, imb_sums, forces, torques, diag, host_diag);
 }
 
 // ---------------------------------------------------------------------------
@@ -996,7 +1074,7 @@ __global__ void __launch_bounds__(256) k_chunk_desc_multi(const LoadsJob* jobs, 
 
 template <typename I>
 __global__ void __launch_bounds__(LOAD_THREADS, PSC_LOADS_MIN_BLOCKS)
-    k_loads_chunks_multi(const LoadsJob* jobs, const int64_t* chunk_base, int njobs, double* part) {
+    k_loads_chunks_multi(const LoadsJob* jobs, const int64_t* chunk_base, int njobs, const double* desc, double* part) {
     __shared__ ChunkRing rows;
     __shared__ LoadRing<I> ring;
     extern __shared__ double s_al[];  // S^3 + 1 entries for the largest S of the jobs (dynamic)
@@ -1005,7 +1083,7 @@ __global__ void __launch_bounds__(LOAD_THREADS, PSC_LOADS_MIN_BLOCKS)
     int cur_S = 0;  // S of the table in s_al (the same in every warp: all visit the same chunks)
     long long j = 0;
     for (int64_t chunk = blockIdx.x; chunk < C; chunk += gridDim.x, ++j) {  // every warp, in this order
-        const ChunkDesc dsc = *reinterpret_cast<const ChunkDesc*>(part + chunk * 6);
+        const ChunkDesc dsc = *reinterpret_cast<const ChunkDesc*>(desc + chunk * 6);
         const psc_geometry& g = jobs[dsc.pad].g;
         const int S = g.subsamples;
         if (S != cur_S) {  // every warp at the same chunk: the barriers are block-uniform
@@ -1028,7 +1106,7 @@ __global__ void __launch_bounds__(LOAD_THREADS, PSC_LOADS_MIN_BLOCKS)
 template <typename I>
 __global__ void __launch_bounds__(LOAD_THREADS, 3) k_loads_chunks_list_multi(const LoadsJob* jobs,
                                                                            const int64_t* chunk_base, int njobs,
-                                                                           double* part) {
+                                                                           const double* desc, double* part) {
     __shared__ ChunkRing rows;
     extern __shared__ __align__(16) unsigned char list_stage[];
     chunk_ring_init(rows);
@@ -1036,7 +1114,7 @@ __global__ void __launch_bounds__(LOAD_THREADS, 3) k_loads_chunks_list_multi(con
     ListCursor cur{};
     int64_t chunk = blockIdx.x;
     if (chunk < C) {
-        cur.dsc = *reinterpret_cast<const ChunkDesc*>(part + chunk * 6);
+        cur.dsc = *reinterpret_cast<const ChunkDesc*>(desc + chunk * 6);
         const psc_geometry& g0 = jobs[cur.dsc.pad].g;
         const int64_t local0 = chunk - chunk_base[cur.dsc.pad];
         cur.n_t = g0.load_n[local0 * LOAD_THREADS + threadIdx.x];
@@ -1047,7 +1125,7 @@ __global__ void __launch_bounds__(LOAD_THREADS, 3) k_loads_chunks_list_multi(con
         const int64_t nxt = chunk + gridDim.x;
         ListCursor nc{};
         if (nxt < C) {
-            nc.dsc = *reinterpret_cast<const ChunkDesc*>(part + nxt * 6);
+            nc.dsc = *reinterpret_cast<const ChunkDesc*>(desc + nxt * 6);
             nc.n_t = jobs[nc.dsc.pad].g.load_n[(nxt - chunk_base[nc.dsc.pad]) * LOAD_THREADS + threadIdx.x];
         }
         const LoadsJob& J = jobs[cur.dsc.pad];
@@ -1074,13 +1152,22 @@ __global__ void __launch_bounds__(256) k_loads_particles_multi(const LoadsJob* j
     const int k = owner_of(particle_base, njobs, gp);
     const LoadsJob& J = jobs[k];
     const int p = (int)(gp - particle_base[k]);
+    double F[6];
     particle_sums(part + chunk_base[k] * 6, J.g.chunk_off[p], J.g.chunk_off[p + 1], J.forces + (size_t)p * 3,
-                  J.torques + (size_t)p * 3);
+                  J.torques + (size_t)p * 3, F);
 }
 
 __global__ void __launch_bounds__(1024) k_loads_diag_multi(const LoadsJob* jobs) {
     const LoadsJob& J = jobs[blockIdx.x];
-    loads_diag_block(J.g.nparticles, J.imb_sums, J.forces, J.torques, J.diag);
+    loads_diag_block(J.g.nparticles, J.imb_sums, J.forces, J.torques, J.diag, J.host_diag);
+}
+
+__global__ void __cluster_dims__(FINAL_CTAS, 1, 1) __launch_bounds__(FINAL_THREADS)
+    k_loads_final_multi(const LoadsJob* jobs, const int64_t* chunk_base, const double* part) {
+    const int k = blockIdx.x / FINAL_CTAS;
+    const LoadsJob& J = jobs[k];
+    loads_final_cluster(J.g.nparticles, J.g.chunk_off, part + chunk_base[k] * 6, J.imb_sums, J.forces, J.torques, J.diag,
+                        J.host_diag);
 }
 
 // ---------------------------------------------------------------------------
@@ -1243,78 +1330,93 @@ static cudaError_t loads_smem_optin() {
     return cudaSuccess;
 }
 
+cudaError_t launch_chunk_desc(const psc_geometry& g, double* desc, cudaStream_t stream) {
+    const int64_t cap = (int64_t)sm_count() * 16, cg = (g.capacity_chunks + 255) / 256;
+    k_chunk_desc<<<(unsigned)(cg < 1 ? 1 : (cg < cap ? cg : cap)), 256, 0, stream>>>(g, desc);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_particle_loads(const psc_geometry& g, int imb_type, const void* imb, double* chunk_partials,
                                   const double* imb_sums, double* forces, double* torques, double* diag,
-                                  cudaStream_t stream) {
+                                  cudaStream_t stream, const double* desc, double* host_diag) {
+    cudaError_t e = cudaSuccess;
     if (g.capacity_chunks > 0 && g.nparticles > 0) {
         const int64_t cap = (int64_t)sm_count() * 16;
         const unsigned grid = (unsigned)(g.capacity_chunks < cap ? g.capacity_chunks : cap);
         const size_t lut = (size_t)(g.subsamples * g.subsamples * g.subsamples + 1) * sizeof(double);
-        const int64_t cg = (g.capacity_chunks + 255) / 256;
-        cudaError_t e0 = loads_smem_optin();
-        if (e0 != cudaSuccess) return e0;
-        k_chunk_desc<<<(unsigned)(cg < cap ? cg : cap), 256, 0, stream>>>(g, chunk_partials);
+        if ((e = loads_smem_optin()) != cudaSuccess) return e;
+        if (!desc) {
+            if ((e = launch_chunk_desc(g, chunk_partials, stream)) != cudaSuccess) return e;
+            desc = chunk_partials;
+        }
         if (g.load_w && g.load_abk && g.load_n) {  // the list path: the list first, unless it is current
-            if (!g.list_ready) k_loads_list_build<<<grid, LOAD_THREADS, lut, stream>>>(g, chunk_partials);
+            if (!g.list_ready) k_loads_list_build<<<grid, LOAD_THREADS, lut, stream>>>(g, desc);
             if (imb_type == 0)
                 k_loads_chunks_list<double><<<grid, LOAD_THREADS, list_stage_bytes<double>(), stream>>>(
-                    g, reinterpret_cast<const double*>(imb), chunk_partials);
+                    g, reinterpret_cast<const double*>(imb), desc, chunk_partials);
             else
                 k_loads_chunks_list<float><<<grid, LOAD_THREADS, list_stage_bytes<float>(), stream>>>(
-                    g, reinterpret_cast<const float*>(imb), chunk_partials);
+                    g, reinterpret_cast<const float*>(imb), desc, chunk_partials);
         } else if (imb_type == 0) {  // no loads list: the whole boxes
-            k_loads_chunks<double><<<grid, LOAD_THREADS, lut, stream>>>(g, reinterpret_cast<const double*>(imb),
+            k_loads_chunks<double><<<grid, LOAD_THREADS, lut, stream>>>(g, reinterpret_cast<const double*>(imb), desc,
                                                                         chunk_partials);
         } else {
-            k_loads_chunks<float><<<grid, LOAD_THREADS, lut, stream>>>(g, reinterpret_cast<const float*>(imb),
+            k_loads_chunks<float><<<grid, LOAD_THREADS, lut, stream>>>(g, reinterpret_cast<const float*>(imb), desc,
                                                                        chunk_partials);
         }
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    if (g.nparticles > 0 && g.nparticles <= FINAL_PARTICLES) {
+        k_loads_final<<<FINAL_CTAS, FINAL_THREADS, 0, stream>>>(g, chunk_partials, imb_sums, forces, torques, diag,
+                                                               host_diag);
+        return cudaGetLastError();
     }
     if (g.nparticles > 0) {
         k_loads_particles<<<(g.nparticles + 7) / 8, 256, 0, stream>>>(g, chunk_partials, forces, torques);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    k_loads_diag<<<1, 1024, 0, stream>>>(g, imb_sums, forces, torques, diag);
+    k_loads_diag<<<1, 1024, 0, stream>>>(g, imb_sums, forces, torques, diag, host_diag);
     return cudaGetLastError();
 }
 
 cudaError_t launch_particle_loads_multi(const LoadsJob* d_jobs, const int64_t* d_chunk_base,
                                         const int64_t* d_particle_base, int njobs, int64_t total_chunks,
                                         int64_t total_particles, int imb_type, int max_subsamples,
-                                        bool all_lists, bool list_ready, double* part, cudaStream_t stream) {
+                                        bool all_lists, bool list_ready, double* part, double* desc, bool desc_ready,
+                                        int max_particles, cudaStream_t stream) {
     if (njobs <= 0) return cudaSuccess;
     const int64_t cap = (int64_t)sm_count() * 16;
+    cudaError_t e = cudaSuccess;
     if (total_chunks > 0) {
         const int64_t cg = (total_chunks + 255) / 256;
-        cudaError_t e0 = loads_smem_optin();
-        if (e0 != cudaSuccess) return e0;
-        k_chunk_desc_multi<<<(unsigned)(cg < cap ? cg : cap), 256, 0, stream>>>(d_jobs, d_chunk_base, njobs, part);
+        if ((e = loads_smem_optin()) != cudaSuccess) return e;
+        if (!desc_ready)
+            k_chunk_desc_multi<<<(unsigned)(cg < cap ? cg : cap), 256, 0, stream>>>(d_jobs, d_chunk_base, njobs, desc);
         const unsigned grid = (unsigned)(total_chunks < cap ? total_chunks : cap);
         const size_t lut = (size_t)(max_subsamples * max_subsamples * max_subsamples + 1) * sizeof(double);
         // every job has a loads list: the lists that are not current first, then the list path
         if (all_lists && !list_ready)
-            k_loads_list_build_multi<<<grid, LOAD_THREADS, lut, stream>>>(d_jobs, d_chunk_base, njobs, part);
+            k_loads_list_build_multi<<<grid, LOAD_THREADS, lut, stream>>>(d_jobs, d_chunk_base, njobs, desc);
         if (all_lists && imb_type == 0)
             k_loads_chunks_list_multi<double><<<grid, LOAD_THREADS, list_stage_bytes<double>(), stream>>>(
-                d_jobs, d_chunk_base, njobs, part);
+                d_jobs, d_chunk_base, njobs, desc, part);
         else if (all_lists)
             k_loads_chunks_list_multi<float><<<grid, LOAD_THREADS, list_stage_bytes<float>(), stream>>>(
-                d_jobs, d_chunk_base, njobs, part);
+                d_jobs, d_chunk_base, njobs, desc, part);
         else if (imb_type == 0)
-            k_loads_chunks_multi<double><<<grid, LOAD_THREADS, lut, stream>>>(d_jobs, d_chunk_base, njobs, part);
+            k_loads_chunks_multi<double><<<grid, LOAD_THREADS, lut, stream>>>(d_jobs, d_chunk_base, njobs, desc, part);
         else
-            k_loads_chunks_multi<float><<<grid, LOAD_THREADS, lut, stream>>>(d_jobs, d_chunk_base, njobs, part);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
+            k_loads_chunks_multi<float><<<grid, LOAD_THREADS, lut, stream>>>(d_jobs, d_chunk_base, njobs, desc, part);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    if (max_particles <= FINAL_PARTICLES) {
+        k_loads_final_multi<<<(unsigned)(njobs * FINAL_CTAS), FINAL_THREADS, 0, stream>>>(d_jobs, d_chunk_base, part);
+        return cudaGetLastError();
     }
     if (total_particles > 0) {
         k_loads_particles_multi<<<(unsigned)((total_particles + 7) / 8), 256, 0, stream>>>(
             d_jobs, d_chunk_base, d_particle_base, njobs, part);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     k_loads_diag_multi<<<(unsigned)njobs, 1024, 0, stream>>>(d_jobs);
     return cudaGetLastError();

@@ -38,7 +38,24 @@ cudaError_t launch_step_pair(int store, const psc_window* d_windows, int nwin, i
 cudaError_t read_device_status(int* out, bool clear);
 cudaError_t read_pair_status(int* out, bool clear);
 cudaError_t read_loads_status(int* out, bool clear);
-cudaError_t launch_reduce_windows(const psc_window* d_windows, int nwin, double* out, cudaStream_t stream);
+// Window sums of the step partials into out[nwin][PSC_NRED] and, where given, out2 (device or
+// page-locked host memory).
+cudaError_t launch_reduce_windows(const psc_window* d_windows, int nwin, double* out, cudaStream_t stream,
+                                  double* out2 = nullptr);
+// One check of the lbm_converge criterion (couple_psc_liggghts.py:284-296) on a window's mean u_z
+// after step `step`, made with the sums of the state after it.
+struct ConvergeCheck {
+    const double* pre;   // the sums taken by step `step` (the state before it and its IMB momentum)
+    double* state;       // [0] mean u_z of the last check, [1] its step, [2] converged, [3] stopping step,
+                         // [4] residual; [kConvState ..) the two rows of sums of the stopping step
+    psc_window* tab[2];  // the window's descriptors: marked inactive on convergence
+    int step, min_steps, last;  // last: keep the rows whether or not the step converges
+    double tol, cells;
+};
+constexpr int kConvState = 8;
+// The sums of one window into out, then the check.
+cudaError_t launch_reduce_converge(const psc_window* d_window, double* out, const ConvergeCheck& cc,
+                                   cudaStream_t stream);
 cudaError_t launch_init_equilibrium(int store, double scale, void* f, int64_t ncells, cudaStream_t stream);
 // inlet = {rho, ux, uy, uz} when open_x (PSC_WIN_OPEN_X faces), else unused
 cudaError_t launch_stream_push(int store, double scale, const void* src, double* dst, int nx, int ny, int nz,
@@ -49,9 +66,13 @@ cudaError_t launch_stream_pull_store(int store, double scale, const double* src,
 cudaError_t launch_geometry_plan(const psc_geometry& g, cudaStream_t stream);
 cudaError_t launch_geometry_build(const psc_geometry& g, cudaStream_t stream);
 cudaError_t launch_solid_velocity(const psc_geometry& g, int us_type, void* us, cudaStream_t stream);
+// desc: the chunk descriptors of this geometry (launch_chunk_desc), or null: made on every call in the
+// chunks' partial rows.  host_diag: page-locked copy of diag, or null.
 cudaError_t launch_particle_loads(const psc_geometry& g, int imb_type, const void* imb, double* chunk_partials,
                                   const double* imb_sums, double* forces, double* torques, double* diag,
-                                  cudaStream_t stream);
+                                  cudaStream_t stream, const double* desc = nullptr, double* host_diag = nullptr);
+// The load-chunk descriptors of one geometry, 6 doubles per chunk.
+cudaError_t launch_chunk_desc(const psc_geometry& g, double* desc, cudaStream_t stream);
 
 // One window of a many-window particle-loads launch (a device table).
 struct LoadsJob {
@@ -61,6 +82,7 @@ struct LoadsJob {
     double* forces;           // [P][3]
     double* torques;          // [P][3]
     double* diag;             // [PSC_NDIAG]
+    double* host_diag;        // page-locked copy of diag, or null
 };
 // Particle loads and load diagnostics of njobs windows in four launches.
 // d_chunk_base / d_particle_base: [njobs + 1] exclusive prefix sums of the
@@ -68,11 +90,14 @@ struct LoadsJob {
 // passed by value); part: total_chunks rows of 6 doubles.  all_lists: every
 // job gives loads-list arrays (the list path: the lists of the jobs whose list
 // is not current are built first); list_ready: every job's list is current.
-// Without all_lists the loads are reduced over the whole boxes.
+// Without all_lists the loads are reduced over the whole boxes.  desc: room for the chunk descriptors
+// (6 doubles per chunk), which hold what an earlier call with the same jobs wrote when desc_ready.
+// max_particles: the largest particle count of a job.
 cudaError_t launch_particle_loads_multi(const LoadsJob* d_jobs, const int64_t* d_chunk_base,
                                         const int64_t* d_particle_base, int njobs, int64_t total_chunks,
                                         int64_t total_particles, int imb_type, int max_subsamples,
-                                        bool all_lists, bool list_ready, double* part, cudaStream_t stream);
+                                        bool all_lists, bool list_ready, double* part, double* desc, bool desc_ready,
+                                        int max_particles, cudaStream_t stream);
 
 cudaError_t launch_adjoint_seed(const psc_adjoint_args& a, cudaStream_t stream);
 cudaError_t launch_adjoint_step(const psc_adjoint_args& a, cudaStream_t stream);

@@ -251,6 +251,8 @@ struct Window {
     DArray<uint8_t> level;
     DArray<unsigned char> scan_tmp;
     DArray<double> chunk_partials;
+    DArray<double> chunk_desc;  // load-chunk descriptors of the geometry of desc_built (window_chunk_desc)
+    uint64_t desc_built = 0;
     double smooth_eps = 0.0;  // > 0: smooth solid fraction (the adjoint's differentiable surrogate)
     DArray<double> ent_alpha;
     DArray<int32_t> cl_ent;
@@ -264,11 +266,13 @@ struct Window {
     int64_t cap_entries = 0, cap_chunks = 0, n_entries = 0, n_chunks = 0;
     DArray<double> forces, torques;
     uint64_t pversion = 1, built_version = 0, us_version = 0;
+    uint64_t builds = 0;  // geometry builds so far
     bool built = false;
     bool moving = false;
     // state of the last step's results
     bool stepped = false, moments_ready = false, loads_ready = false, diag_ready = false;
     DArray<double> out;  // [red_pre][red_post][diag]
+    const double* pre = nullptr;  // the last step's own sums where they are not in out (a step run ahead)
     psc_diag last{};
 
     ~Window() {
@@ -537,6 +541,7 @@ int window_rebuild_finish(Window& w, cudaStream_t s, const int64_t* tot4, const 
     if (w.n_chunks > w.cap_chunks) {
         const int64_t cap = w.n_chunks + w.n_chunks / 4 + 16;
         PSC_CUDA(w.chunk_partials.ensure(cap * 6, false, s), who);
+        PSC_CUDA(w.chunk_desc.ensure(cap * 6, false, s), who);
         if (w.list_allowed()) {
             PSC_CUDA(w.load_w.ensure(cap * kChunkEntries, false, s), who);
             PSC_CUDA(w.load_abk.ensure(cap * kChunkEntries, false, s), who);
@@ -547,8 +552,10 @@ int window_rebuild_finish(Window& w, cudaStream_t s, const int64_t* tot4, const 
     psc_geometry g = w.geometry();
     PSC_TRY(psc_geometry_build(&g, s));
     w.built = true;
+    ++w.builds;
     w.built_version = w.pversion;
     w.list_version = 0;
+    w.desc_built = 0;
     w.us_version = 0;
     w.loads_ready = false;
     w.diag_ready = false;
@@ -627,11 +634,23 @@ double* red_pre(Window& w) { return w.out.p; }
 double* red_post(Window& w) { return w.out.p + PSC_NRED; }
 double* diag_dev(Window& w) { return w.out.p + 2 * PSC_NRED; }
 
-int window_loads(Window& w, cudaStream_t s) {
-    psc_geometry g = w.geometry();
-    PSC_TRY(psc_particle_loads(&g, w.field_type(), w.imb_for(w.imb_par), w.chunk_partials.p,
-                               red_pre(w) + PSC_RED_IMBX, w.forces.p, w.torques.p, diag_dev(w), s));
+// The loads of the geometry's particles from one IMB field, its sums at imb_sums; the chunk
+// descriptors are made once per geometry.
+int window_loads_from(Window& w, const void* imb, const double* imb_sums, cudaStream_t s, double* host_diag = nullptr) {
+    const psc_geometry g = w.geometry();
+    if (w.P > 0 && w.cap_chunks > 0 && (!w.built || w.desc_built != w.built_version)) {
+        PSC_CUDA(launch_chunk_desc(g, w.chunk_desc.p, s), "particle loads");
+        w.desc_built = w.built ? w.built_version : 0;
+    }
+    PSC_CUDA(launch_particle_loads(g, w.field_type(), imb, w.chunk_partials.p, imb_sums, w.forces.p, w.torques.p,
+                                   diag_dev(w), s, w.chunk_desc.p, host_diag),
+             "particle loads");
     w.loads_enqueued();
+    return PSC_OK;
+}
+
+int window_loads(Window& w, cudaStream_t s) {
+    PSC_TRY(window_loads_from(w, w.imb_for(w.imb_par), (w.pre ? w.pre : red_pre(w)) + PSC_RED_IMBX, s));
     w.loads_ready = true;
     return PSC_OK;
 }
@@ -855,12 +874,13 @@ struct psc_solver {
     // buffer and IMB field instead of a reduction-only pass; the next reporting call takes it as
     // its step when its inputs are still the same.  Every other call that steps or sets the state
     // drops it (the current state is untouched by it).
-    DArray<double> ahead_red;             // reductions of the step run ahead
+    DArray<double> ahead_red;             // its sums: a row per buffer parity it ran into
+    double ahead_host[PSC_NRED] = {};     // the same on the host
     bool ahead_ready = false;
     std::vector<uint64_t> ahead_inputs;   // step inputs it ran with
     std::vector<uint64_t> report_inputs;  // step inputs of the last reporting call
-    // device-side convergence (psc_converge): criterion state [kConvState] + reductions snapshot,
-    // and two pinned status slots the host polls
+    // device-side convergence (psc_converge): criterion state [kConvState], the stopping step's two rows of
+    // sums, the rows of the last two steps; and two pinned status slots the host polls
     DArray<double> conv;
     HArray<double> conv_host;
     cudaEvent_t conv_ev[2] = {nullptr, nullptr};
@@ -896,49 +916,13 @@ int solver_report(psc_solver& h, bool loads, bool fields, bool post = true) {
     if (loads) PSC_CUDA(h.lanes.end(s), "psc_step");
     PSC_CUDA(h.host_out.ensure(kOutLen), "psc_step");
     PSC_CUDA(cudaMemcpyAsync(h.host_out.p, w.out.p, kOutLen * sizeof(double), cudaMemcpyDeviceToHost, s), "psc_step");
+    if (w.pre)
+        PSC_CUDA(cudaMemcpyAsync(h.host_out.p, w.pre, PSC_NRED * sizeof(double), cudaMemcpyDeviceToHost, s), "psc_step");
     PSC_CUDA(cudaStreamSynchronize(s), "psc_step");
     if (fields) w.moments_ready = true;
     fill_diag(w, h.host_out.p, w.last);
     w.diag_ready = loads;
     return PSC_OK;
-}
-
-// ---------------------------------------------------------------------------
-// lbm_converge on the device (couple_psc_liggghts.py:284-296)
-// ---------------------------------------------------------------------------
-// Criterion state, doubles: [0] mean_uz of the last check, [1] its step,
-// [2] converged flag, [3] stopping step, [4] residual of the last check;
-// [kConvState ..) the out row (red_pre, red_post) of the stopping step.
-constexpr int kConvState = 8;
-
-// One check after step `step` of the call: out holds red_pre (the reductions
-// of the state before the step, i.e. the previous step's post-stream state)
-// and red_post (the post-stream state of the step).  mean_uz of the previous
-// step is the value this kernel kept when it checked that step (every step
-// checked: the reference's sequence of values), else red_pre's.  Step 1 has
-// no previous value (residual inf, as the reference's first iteration).  On
-// convergence the out row is kept and the window is marked inactive in both
-// descriptor tables, so the launches already enqueued after it do nothing.
-__global__ void k_converge_check(const double* out, double* cs, psc_window* tab0, psc_window* tab1, int step,
-                                 int min_steps, double tol, double N) {
-    if (threadIdx.x != 0 || blockIdx.x != 0 || cs[2] != 0.0) return;
-    const double now = out[PSC_NRED + PSC_RED_UZ] / N;
-    double resid = __longlong_as_double(0x7ff0000000000000ll);  // +inf
-    if (step > 1) {
-        const double prev = cs[1] == (double)(step - 1) ? cs[0] : out[PSC_RED_UZ] / N;
-        const double a = fabs(now);
-        resid = fabs(now - prev) / (a < 1.0e-30 ? 1.0e-30 : a);
-    }
-    cs[0] = now;
-    cs[1] = (double)step;
-    cs[4] = resid;
-    if (step >= min_steps && resid < tol) {
-        cs[2] = 1.0;
-        cs[3] = (double)step;
-        for (int k = 0; k < 2 * PSC_NRED; ++k) cs[kConvState + k] = out[k];
-        tab0->flags |= PSC_WIN_INACTIVE;
-        tab1->flags |= PSC_WIN_INACTIVE;
-    }
 }
 
 // One collide_stream_psc step; `imb` writes the IMB field and reduces the
@@ -958,7 +942,10 @@ int solver_collide(psc_solver& h, bool imb) {
     w.moments_ready = false;
     w.loads_ready = false;
     w.diag_ready = false;
-    if (imb) PSC_TRY(psc_reduce_windows(w.solo[w.cur].p, 1, red_pre(w), s));
+    if (imb) {
+        PSC_TRY(psc_reduce_windows(w.solo[w.cur].p, 1, red_pre(w), s));
+        w.pre = nullptr;
+    }
     return PSC_OK;
 }
 
@@ -977,11 +964,12 @@ std::vector<unsigned char> report_key(const psc_solver& h, int par, int kind) {
         const void* ahead;
         const void* host;
         const void* chunks;
+        const void* descs;
         const void* forces;
         const void* torques;
         uint64_t desc_version;
         int64_t tiles;
-        int32_t kernel, store, moving, par, field_type, kind;
+        int32_t kernel, store, moving, par, field_type, kind, desc_ready;
     } k;
     std::memset(&k, 0, sizeof(k));  // padding too: keys compare bytewise
     k.g = w.geometry();
@@ -993,6 +981,8 @@ std::vector<unsigned char> report_key(const psc_solver& h, int par, int kind) {
     k.ahead = h.ahead_red.p;
     k.host = h.host_out.p;
     k.chunks = w.chunk_partials.p;
+    k.descs = w.chunk_desc.p;
+    k.desc_ready = w.built && w.desc_built == w.built_version ? 1 : 0;
     k.forces = w.forces.p;
     k.torques = w.torques.p;
     k.desc_version = w.desc_version;
@@ -1016,39 +1006,35 @@ std::vector<uint64_t> solver_step_inputs(const psc_solver& h) {
 
 // The GPU work of one reporting step from buffer parity `par` (the launches of
 // solver_collide(imb) + solver_report(loads, post) without their host-side
-// bookkeeping), ending with the read-back into host_out.  kReportCommit: the
-// step from `par` is in place already (buffer par ^ 1, its IMB field and its
-// reductions in ahead_red).  kReportAhead: the post-stream sums come from the
-// next step, run from par ^ 1 into buffer par and IMB field par.
+// bookkeeping).  The kernels write what the caller reads into the page-locked
+// host_out themselves.  kReportCommit: the step from `par` is in place already
+// (buffer par ^ 1, its IMB field, its sums in ahead_red's row par ^ 1 and
+// ahead_host).  kReportAhead: the post-stream sums come from the next step,
+// run from par ^ 1 into buffer par and IMB field par, its sums into row par.
 int report_step_work(psc_solver& h, int par, int kind) {
     Window& w = h.w;
     cudaStream_t s = h.stream;
     const unsigned mv = w.moving ? PSC_STEP_MOVING : 0u;
     const psc_launch c = {0, 1, w.solo_kernel, 0, 0};
     const unsigned full = PSC_STEP_COLLIDE | PSC_STEP_IMB | PSC_STEP_REDUCE | mv;
-    if (kind & kReportCommit) {
-        PSC_CUDA(cudaMemcpyAsync(red_pre(w), h.ahead_red.p, PSC_NRED * sizeof(double), cudaMemcpyDeviceToDevice, s),
-                 "psc_step");
-    } else {
+    const double* pre = h.ahead_red.p + (par ^ 1) * PSC_NRED;
+    if (!(kind & kReportCommit)) {
+        pre = red_pre(w);
         PSC_TRY(psc_step_windows_ex(w.cfg.store, w.solo[par].p, 1, w.solo_tiles, full, &c, s));
-        PSC_TRY(psc_reduce_windows(w.solo[par ^ 1].p, 1, red_pre(w), s));
+        PSC_CUDA(launch_reduce_windows(w.solo[par ^ 1].p, 1, red_pre(w), s, h.host_out.p), "psc_step");
     }
     PSC_CUDA(h.lanes.begin(s), "psc_step");  // the loads on a lane; the main stream's kernel first
+    double* host_post = h.host_out.p + PSC_NRED;
     if (kind & kReportAhead) {
         PSC_TRY(psc_step_windows_ex(w.cfg.store, w.solo[par ^ 1].p, 1, w.solo_tiles, full, &c, s));
-        PSC_TRY(psc_reduce_windows(w.solo[par].p, 1, h.ahead_red.p, s));
-        PSC_CUDA(cudaMemcpyAsync(red_post(w), h.ahead_red.p, PSC_NRED * sizeof(double), cudaMemcpyDeviceToDevice, s),
-                 "psc_step");
+        PSC_CUDA(launch_reduce_windows(w.solo[par].p, 1, h.ahead_red.p + par * PSC_NRED, s, host_post), "psc_step");
     } else {
         PSC_TRY(psc_step_windows_ex(w.cfg.store, w.solo[par ^ 1].p, 1, w.solo_tiles, PSC_STEP_REDUCE | mv, &c, s));
-        PSC_TRY(psc_reduce_windows(w.solo[par ^ 1].p, 1, red_post(w), s));
+        PSC_CUDA(launch_reduce_windows(w.solo[par ^ 1].p, 1, red_post(w), s, host_post), "psc_step");
     }
-    psc_geometry g = w.geometry();
-    PSC_TRY(psc_particle_loads(&g, w.field_type(), w.imb_for(par ^ 1), w.chunk_partials.p, red_pre(w) + PSC_RED_IMBX,
-                               w.forces.p, w.torques.p, diag_dev(w), h.lanes.lane(0)));
-    w.loads_enqueued();
+    PSC_TRY(window_loads_from(w, w.imb_for(par ^ 1), pre + PSC_RED_IMBX, h.lanes.lane(0),
+                              h.host_out.p + 2 * PSC_NRED));
     PSC_CUDA(h.lanes.end(s), "psc_step");
-    PSC_CUDA(cudaMemcpyAsync(h.host_out.p, w.out.p, kOutLen * sizeof(double), cudaMemcpyDeviceToHost, s), "psc_step");
     return PSC_OK;
 }
 
@@ -1062,7 +1048,7 @@ int solver_report_step(psc_solver& h) {
     PSC_TRY(window_ensure_imb(w, s));
     PSC_TRY(window_upload_solo(w, s));
     PSC_CUDA(h.host_out.ensure(kOutLen), "psc_step");
-    PSC_CUDA(h.ahead_red.ensure(PSC_NRED, true, s), "psc_step");
+    PSC_CUDA(h.ahead_red.ensure(2 * PSC_NRED, true, s), "psc_step");
     const std::vector<uint64_t> inputs = solver_step_inputs(h);
     int kind = 0;
     if (h.ahead_ready && inputs == h.ahead_inputs) kind |= kReportCommit;
@@ -1110,8 +1096,11 @@ int solver_report_step(psc_solver& h) {
     w.stepped = true;
     w.moments_ready = false;
     w.loads_ready = true;
+    w.pre = (kind & kReportCommit) ? h.ahead_red.p + (par ^ 1) * PSC_NRED : nullptr;
     PSC_CUDA(cudaStreamSynchronize(s), "psc_step");
+    if (kind & kReportCommit) std::memcpy(h.host_out.p, h.ahead_host, sizeof(h.ahead_host));
     if (kind & kReportAhead) {  // the step run ahead added its own IMB; a reduction pass adds none
+        std::memcpy(h.ahead_host, h.host_out.p + PSC_NRED, sizeof(h.ahead_host));
         for (int q = PSC_RED_IMBX; q <= PSC_RED_IMBZ; ++q) h.host_out.p[PSC_NRED + q] = 0.0;
         h.ahead_ready = true;
         h.ahead_inputs = inputs;
@@ -1126,9 +1115,14 @@ int solver_report_step(psc_solver& h) {
 // enqueued in blocks with the criterion evaluated on the device at every
 // check step (a multiple of check_every, and the last step); the host reads
 // the criterion state once per block, one block behind, and stops enqueuing
-// once it reports convergence.  Steps enqueued after the stopping step find
-// the window inactive and do nothing, so the populations stay those of the
-// stopping step: buffer parity start ^ (steps & 1).
+// once it reports convergence.
+//
+// The mean velocity after step k is a sum that step k + 1 takes anyway (of the
+// state it pulls), so step k is checked when step k + 1 has run: one step and
+// one sum-and-check launch per checked step.  Step k + 1 writes the other
+// buffer and IMB field, so the state of step k is untouched; steps enqueued
+// after a stopping step find the window inactive and do nothing.  The last
+// step is followed by a pass that only takes the sums.
 int solver_converge(psc_solver& h, int nsteps, double tol, int min_steps, int check_every, bool fields,
                     psc_status& st) {
     Window& w = h.w;
@@ -1139,7 +1133,7 @@ int solver_converge(psc_solver& h, int nsteps, double tol, int min_steps, int ch
     // from here on the device may mark the window inactive in its descriptor tables: whatever
     // path leaves this function, the next launch uploads them afresh
     w.solo_dirty = true;
-    PSC_CUDA(h.conv.ensure(kConvState + 2 * PSC_NRED, false, s), who);
+    PSC_CUDA(h.conv.ensure(kConvState + 4 * PSC_NRED, false, s), who);
     PSC_CUDA(h.conv_host.ensure(2 * kConvState), who);
     for (auto& e : h.conv_ev)
         if (!e) PSC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), who);
@@ -1147,6 +1141,19 @@ int solver_converge(psc_solver& h, int nsteps, double tol, int min_steps, int ch
     const unsigned mv = w.moving ? PSC_STEP_MOVING : 0u;
     const psc_launch c = {0, 1, w.solo_kernel, 0, 0};
     const int start = w.cur;
+    const auto row = [&](int u) { return h.conv.p + kConvState + (2 + (u & 1)) * PSC_NRED; };
+    const auto checked = [&](int u) { return u >= 1 && (u % check_every == 0 || u == nsteps); };
+    // the sums of window table `tab` into step u's row, and the check of step u - 1 with them
+    const auto sums = [&](const psc_window* tab, int u) -> int {
+        if (!checked(u - 1)) {
+            PSC_CUDA(launch_reduce_windows(tab, 1, row(u), s), who);
+            return PSC_OK;
+        }
+        const ConvergeCheck cc = {row(u - 1), h.conv.p, {w.solo[0].p, w.solo[1].p}, u - 1, min_steps,
+                                  u - 1 == nsteps ? 1 : 0, tol, (double)w.N};
+        PSC_CUDA(launch_reduce_converge(tab, row(u), cc, s), who);
+        return PSC_OK;
+    };
     // steps per poll: ~3e7 lattice updates (about a millisecond of the step kernel), 4 .. 256 steps
     const int64_t per = std::max<int64_t>(4, std::min<int64_t>(256, 30000000 / std::max<int64_t>(w.N, 1)));
     const int block = (int)std::max<int64_t>(check_every, per);
@@ -1156,18 +1163,15 @@ int solver_converge(psc_solver& h, int nsteps, double tol, int min_steps, int ch
         const int end = (int)std::min<int64_t>(nsteps, (int64_t)t + block);
         for (int u = t + 1; u <= end; ++u) {
             const int par = start ^ ((u - 1) & 1);
-            if (u % check_every != 0 && u != nsteps) {
-                PSC_TRY(psc_step_windows_ex(w.cfg.store, w.solo[par].p, 1, w.solo_tiles, PSC_STEP_COLLIDE | mv, &c, s));
-                continue;
-            }
-            PSC_TRY(psc_step_windows_ex(w.cfg.store, w.solo[par].p, 1, w.solo_tiles,
-                                        PSC_STEP_COLLIDE | PSC_STEP_IMB | PSC_STEP_REDUCE | mv, &c, s));
-            PSC_TRY(psc_reduce_windows(w.solo[par ^ 1].p, 1, red_pre(w), s));
-            PSC_TRY(psc_step_windows_ex(w.cfg.store, w.solo[par ^ 1].p, 1, w.solo_tiles, PSC_STEP_REDUCE | mv, &c, s));
-            PSC_TRY(psc_reduce_windows(w.solo[par ^ 1].p, 1, red_post(w), s));
-            k_converge_check<<<1, 32, 0, s>>>(w.out.p, h.conv.p, w.solo[0].p, w.solo[1].p, u, min_steps, tol,
-                                              (double)w.N);
-            PSC_CUDA(cudaGetLastError(), who);
+            const bool here = checked(u), before = checked(u - 1);
+            const unsigned flags = PSC_STEP_COLLIDE | (here ? PSC_STEP_IMB : 0u) | (here || before ? PSC_STEP_REDUCE : 0u);
+            PSC_TRY(psc_step_windows_ex(w.cfg.store, w.solo[par].p, 1, w.solo_tiles, flags | mv, &c, s));
+            if (here || before) PSC_TRY(sums(w.solo[par].p, u));
+        }
+        if (end == nsteps) {
+            const int par = start ^ (nsteps & 1);
+            PSC_TRY(psc_step_windows_ex(w.cfg.store, w.solo[par].p, 1, w.solo_tiles, PSC_STEP_REDUCE | mv, &c, s));
+            PSC_TRY(sums(w.solo[par].p, nsteps + 1));
         }
         t = end;
         const int slot = polls & 1;
@@ -1195,10 +1199,10 @@ int solver_converge(psc_solver& h, int nsteps, double tol, int min_steps, int ch
     w.moments_ready = false;
     w.loads_ready = false;
     w.diag_ready = false;
-    if (converged)  // the reductions of the stopping step (later enqueued reductions read no new partials)
-        PSC_CUDA(cudaMemcpyAsync(w.out.p, h.conv.p + kConvState, 2 * PSC_NRED * sizeof(double),
-                                 cudaMemcpyDeviceToDevice, s),
-                 who);
+    w.pre = nullptr;
+    // the sums of the stopping step
+    PSC_CUDA(cudaMemcpyAsync(w.out.p, h.conv.p + kConvState, 2 * PSC_NRED * sizeof(double), cudaMemcpyDeviceToDevice, s),
+             who);
     PSC_TRY(window_upload_solo(w, s));  // the descriptor tables without the inactive flag
     // loads and diagnostics of the stopping step (its IMB field; the post-stream reductions are
     // taken already unless the fields are wanted)
@@ -1451,6 +1455,7 @@ struct psc_batch {
     // and IMB field; the current state stays as it is) instead of a reduction-only pass, and the
     // next call takes it as its first step when its inputs are still the same.
     DArray<double> red_next;            // reductions of the step run ahead
+    std::vector<double> ahead_host;     // the same on the host
     bool ahead_ready = false;           // a step run ahead is waiting in the other buffer
     std::vector<uint64_t> ahead_inputs;  // the step inputs it ran with
     std::vector<uint64_t> report_inputs;  // the step inputs of the last reporting call
@@ -1481,7 +1486,9 @@ struct psc_batch {
     DArray<unsigned char> jobs_dev[2];
     int jobs_par = 0;  // the table of the last batch_loads_table
     DArray<double> loads_part;  // chunk partials of all jobs
-    int jobs_n = 0, jobs_max_s = 1;
+    DArray<double> loads_desc;  // chunk descriptors of all jobs, of the geometries in desc_built
+    std::vector<uint64_t> desc_built;
+    int jobs_n = 0, jobs_max_s = 1, jobs_max_p = 0;
     int64_t jobs_chunks = 0, jobs_particles = 0;
     bool jobs_list_ready = false;  // every job's loads list is current
     bool jobs_all_lists = false;   // every job has loads-list arrays (the list path of the loads)
@@ -1506,6 +1513,7 @@ int batch_loads_table(psc_batch& b, const char* who) {
     std::vector<LoadsJob> jobs;
     std::vector<int64_t> cb(1, 0), pb(1, 0);
     int max_s = 1;
+    int max_p = 0;
     bool ready = true, lists = true;
     for (int k = 0; k < nwin; ++k) {
         if (b.frozen[(size_t)k] >= 0) continue;
@@ -1520,10 +1528,12 @@ int batch_loads_table(psc_batch& b, const char* who) {
         j.forces = w.forces.p;
         j.torques = w.torques.p;
         j.diag = b.diag.p + (size_t)k * PSC_NDIAG;
+        j.host_diag = b.host.p + 2 * (size_t)nwin * PSC_NRED + (size_t)k * PSC_NDIAG;
         jobs.push_back(j);
         cb.push_back(cb.back() + (w.P > 0 ? w.n_chunks : 0));
         pb.push_back(pb.back() + w.P);
         max_s = std::max(max_s, w.cfg.subsamples);
+        max_p = std::max(max_p, w.P);
     }
     const size_t n = jobs.size();
     const size_t jb = n * sizeof(LoadsJob), bb = (n + 1) * sizeof(int64_t);
@@ -1533,6 +1543,7 @@ int batch_loads_table(psc_batch& b, const char* who) {
     std::memcpy(bytes.data() + jb + bb, pb.data(), bb);
     b.jobs_n = (int)n;
     b.jobs_max_s = max_s;
+    b.jobs_max_p = max_p;
     b.jobs_chunks = cb.back();
     b.jobs_particles = pb.back();
     b.jobs_list_ready = ready;
@@ -1544,6 +1555,8 @@ int batch_loads_table(psc_batch& b, const char* who) {
     // the partials, and every reporting call ends with a stream synchronisation, so nothing of an
     // earlier call still reads them (a buffer that grows is freed by cudaFree, which waits anyway).
     PSC_CUDA(b.loads_part.ensure(std::max<int64_t>(b.jobs_chunks, 1) * 6, false, b.stream), who);
+    if (b.loads_desc.n < b.jobs_chunks * 6) b.desc_built.clear();
+    PSC_CUDA(b.loads_desc.ensure(std::max<int64_t>(b.jobs_chunks, 1) * 6, false, b.stream), who);
     PSC_CUDA(b.jobs_dev[t].ensure((int64_t)bytes.size(), false, b.stream), who);
     PSC_CUDA(b.jobs_host[t].ensure((int64_t)bytes.size()), who);
     std::memcpy(b.jobs_host[t].p, bytes.data(), bytes.size());
@@ -1551,6 +1564,18 @@ int batch_loads_table(psc_batch& b, const char* who) {
              who);
     b.jobs_last[t].swap(bytes);
     return PSC_OK;
+}
+
+// What the chunk descriptors of the job table depend on: the active windows and their geometries.
+std::vector<uint64_t> batch_geometries(const psc_batch& b) {
+    std::vector<uint64_t> v;
+    for (size_t k = 0; k < b.w.size(); ++k) {
+        if (b.frozen[k] >= 0) continue;
+        v.push_back(k);
+        v.push_back(b.w[k]->builds);
+        v.push_back((uint64_t)b.w[k]->P);
+    }
+    return v;
 }
 
 const LoadsJob* batch_jobs(const psc_batch& b) { return reinterpret_cast<const LoadsJob*>(b.jobs_dev[b.jobs_par].p); }
@@ -1992,7 +2017,8 @@ int psc_batch_step(psc_batch* b, int nsteps, unsigned flags, psc_status* h_statu
             PSC_TRY(batch_launch(*b, PSC_STEP_COLLIDE | PSC_STEP_IMB | PSC_STEP_REDUCE));
             b->parity ^= 1;
             batch_sync_cur(*b);
-            PSC_TRY(psc_reduce_windows(b->table[b->parity].p, nwin, b->red_pre.p, b->stream));
+            PSC_CUDA(launch_reduce_windows(b->table[b->parity].p, nwin, b->red_pre.p, b->stream, b->host.p),
+                     "psc_batch_step");
             for (int k = 0; k < nwin; ++k)
                 if (b->frozen[(size_t)k] < 0) b->w[(size_t)k]->imb_par = b->w[(size_t)k]->cur;
         }
@@ -2003,37 +2029,39 @@ int psc_batch_step(psc_batch* b, int nsteps, unsigned flags, psc_status* h_statu
         PSC_TRY(batch_loads_table(*b, "psc_batch_step"));
         PSC_CUDA(b->lanes.begin(b->stream), "psc_batch_step");
         const bool ahead = batch_may_run_ahead(*b, fields, inputs);
-        const double* post_rows = ahead ? b->red_next.p : b->red_post.p;
+        // (the kernels write the sums and diagnostics into the page-locked host rows themselves)
+        double* host = b->host.p;
         if (ahead) {
             PSC_TRY(batch_launch(*b, PSC_STEP_COLLIDE | PSC_STEP_IMB | PSC_STEP_REDUCE));
-            PSC_TRY(psc_reduce_windows(b->table[b->parity ^ 1].p, nwin, b->red_next.p, b->stream));
+            PSC_CUDA(launch_reduce_windows(b->table[b->parity ^ 1].p, nwin, b->red_next.p, b->stream, host + rows),
+                     "psc_batch_step");
         } else {
             PSC_TRY(batch_launch(*b, PSC_STEP_REDUCE | (fields ? PSC_STEP_MOMENTS : 0u)));
-            PSC_TRY(psc_reduce_windows(b->table[b->parity].p, nwin, b->red_post.p, b->stream));
+            PSC_CUDA(launch_reduce_windows(b->table[b->parity].p, nwin, b->red_post.p, b->stream, host + rows),
+                     "psc_batch_step");
         }
         if (b->up_pending)  // the loads read the particles: after their upload
             PSC_CUDA(cudaStreamWaitEvent(b->lanes.lane(0), b->up_done, 0), "psc_batch_step");
+        // the chunk descriptors are made when a geometry or the set of active windows changed
+        std::vector<uint64_t> geos = batch_geometries(*b);
+        const bool desc_ready = geos == b->desc_built;
         PSC_CUDA(launch_particle_loads_multi(batch_jobs(*b), batch_chunk_base(*b),
                                              batch_particle_base(*b), b->jobs_n, b->jobs_chunks, b->jobs_particles,
                                              b->w[0]->field_type(), b->jobs_max_s, b->jobs_all_lists,
-                                             b->jobs_list_ready,
-                                             b->loads_part.p, b->lanes.lane(0)),
+                                             b->jobs_list_ready, b->loads_part.p, b->loads_desc.p, desc_ready,
+                                             b->jobs_max_p, b->lanes.lane(0)),
                  "psc_batch_step: particle loads");
+        if (!desc_ready) b->desc_built.swap(geos);
         for (int k = 0; k < nwin; ++k)
             if (b->frozen[(size_t)k] < 0) {
                 b->w[(size_t)k]->loads_enqueued();
                 b->w[(size_t)k]->loads_ready = true;
             }
         PSC_CUDA(b->lanes.end(b->stream), "psc_batch_step");
-        double* host = b->host.p;
-        PSC_CUDA(cudaMemcpyAsync(host, b->red_pre.p, rows * 8, cudaMemcpyDeviceToHost, b->stream), "psc_batch_step");
-        PSC_CUDA(cudaMemcpyAsync(host + rows, post_rows, rows * 8, cudaMemcpyDeviceToHost, b->stream),
-                 "psc_batch_step");
-        PSC_CUDA(cudaMemcpyAsync(host + 2 * rows, b->diag.p, (size_t)nwin * PSC_NDIAG * 8, cudaMemcpyDeviceToHost,
-                                 b->stream),
-                 "psc_batch_step");
         PSC_CUDA(cudaStreamSynchronize(b->stream), "psc_batch_step");
+        if (final_done) std::memcpy(host, b->ahead_host.data(), rows * 8);
         if (ahead) {
+            b->ahead_host.assign(host + rows, host + 2 * rows);
             b->ahead_ready = true;
             b->ahead_inputs = inputs;
         }

@@ -1,5 +1,7 @@
 // Sums of the step kernels' partial rows, and the conversions between stored
 // populations and the reference's post-stream f (src/lbm_dem/psc3d.py:239-242).
+#include <cooperative_groups.h>
+
 #include "collide.cuh"
 #include "internal.cuh"
 #include "step_common.cuh"
@@ -7,12 +9,16 @@
 namespace psc {
 
 // Window sums of the partial rows (header row: element 0 = row count; the
-// rows follow it), deterministic, in two launches:
-//  1. k_reduce_segments: blockIdx.y = window; blocks stride over segments of
-//     REDUCE_SEG consecutive rows; each segment is summed by a fixed tree and
-//     its sum written over the segment's first row (the partials are consumed);
-//  2. k_reduce_windows: one block per window sums the segment rows in order.
-constexpr int REDUCE_SEG = STEP_THREADS;
+// rows follow it) by one cluster of REDUCE_CTAS CTAs per window, in a fixed
+// order: thread (c, g, k) of CTA c adds column k of the rows c * 32 + g,
+// + 32 * REDUCE_CTAS, ...; a warp per column adds the CTA's 32 groups by a
+// shuffle tree; the cluster's first CTA adds the CTAs' sums in order through
+// distributed shared memory.  A reporting call waits for these sums, so what
+// counts is latency: a window of 296 CTAs leaves 2368 rows, nine independent
+// loads per thread.  One launch of 3 us instead of two of 3.5 us.
+constexpr int REDUCE_CTAS = 8;
+constexpr int REDUCE_GROUPS = 32;
+constexpr int REDUCE_THREADS = REDUCE_GROUPS * PSC_NRED;  // a warp per column
 
 // Row count from the header, clamped to the window's capacity.
 __device__ __forceinline__ int64_t partial_rows(const psc_window& W) {
@@ -22,46 +28,91 @@ __device__ __forceinline__ int64_t partial_rows(const psc_window& W) {
     const int64_t r = (int64_t)h;
     return r < cap ? r : cap;
 }
-constexpr int REDUCE_SEG_BLOCKS = 64;  // blocks per window in launch 1
 
-__global__ void __launch_bounds__(STEP_THREADS) k_reduce_segments(const psc_window* __restrict__ wins) {
-    __shared__ double s_red[STEP_THREADS / 32][PSC_NRED];
-    __shared__ double s_out[PSC_NRED];
-    const psc_window& W = wins[blockIdx.y];
-    const int64_t rows = partial_rows(W);
-    const int64_t nseg = (rows + REDUCE_SEG - 1) / REDUCE_SEG;
-    double* body = W.partials + PSC_NRED;
-    for (int64_t sg = blockIdx.x; sg < nseg; sg += gridDim.x) {  // block-uniform
-        const int64_t r = sg * REDUCE_SEG + threadIdx.x;
-        double v[PSC_NRED];
-        if (r < rows) {
-            const double* p = body + r * PSC_NRED;
-#pragma unroll
-            for (int k = 0; k < PSC_NRED; ++k) v[k] = p[k];
-        } else {
-#pragma unroll
-            for (int k = 0; k < PSC_NRED; ++k) v[k] = 0.0;
+// The residual |mean_k - mean_{k-1}| / |mean_k| of step k = cc.step; step 1 has no previous value
+// (residual inf, as the reference's first iteration).  On convergence the step's rows are kept and the
+// window is marked inactive in both descriptor tables, so the launches already enqueued do nothing.
+__device__ void converge_check(const ConvergeCheck& cc, const double* post) {
+    double* cs = cc.state;
+    if (cs[2] != 0.0) return;
+    const double now = post[PSC_RED_UZ] / cc.cells;
+    double resid = __longlong_as_double(0x7ff0000000000000ll);  // +inf
+    if (cc.step > 1) {
+        const double a = fabs(now);
+        resid = fabs(now - cc.pre[PSC_RED_UZ] / cc.cells) / (a < 1.0e-30 ? 1.0e-30 : a);
+    }
+    cs[0] = now;
+    cs[1] = (double)cc.step;
+    cs[4] = resid;
+    const bool done = cc.step >= cc.min_steps && resid < cc.tol;
+    if (done || cc.last) {
+        for (int k = 0; k < PSC_NRED; ++k) {
+            cs[kConvState + k] = cc.pre[k];
+            // the sums of the state after the step: an IMB momentum among them is the next step's
+            cs[kConvState + PSC_NRED + k] = k >= PSC_RED_IMBX && k <= PSC_RED_IMBZ ? 0.0 : post[k];
         }
-        block_reduce_store<PSC_NRED>(v, s_red, s_out);  // every read of the segment precedes its barrier
-        if (threadIdx.x < PSC_NRED) body[sg * REDUCE_SEG * PSC_NRED + threadIdx.x] = s_out[threadIdx.x];
+    }
+    if (done) {
+        cs[2] = 1.0;
+        cs[3] = (double)cc.step;
+        cc.tab[0]->flags |= PSC_WIN_INACTIVE;
+        cc.tab[1]->flags |= PSC_WIN_INACTIVE;
     }
 }
 
-__global__ void __launch_bounds__(STEP_THREADS) k_reduce_windows(const psc_window* __restrict__ wins,
-                                                                 double* __restrict__ out) {
-    __shared__ double s_red[STEP_THREADS / 32][PSC_NRED];
-    const psc_window& W = wins[blockIdx.x];
+template <bool CONV>
+__global__ void __cluster_dims__(REDUCE_CTAS, 1, 1) __launch_bounds__(REDUCE_THREADS)
+    k_reduce_windows(const psc_window* __restrict__ wins, double* __restrict__ out, double* __restrict__ out2,
+                     const __grid_constant__ ConvergeCheck cc) {
+    namespace cg = cooperative_groups;
+    __shared__ double s_g[REDUCE_GROUPS * PSC_NRED];
+    __shared__ double s_cta[PSC_NRED];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int c = (int)cluster.block_rank(), t = threadIdx.x;
+    const int w = blockIdx.x / REDUCE_CTAS;
+    const psc_window& W = wins[w];
     const int64_t rows = partial_rows(W);
-    const int64_t nseg = (rows + REDUCE_SEG - 1) / REDUCE_SEG;
-    double acc[PSC_NRED];
+    const double* body = W.partials + PSC_NRED;
+    double acc = 0.0;
+    const int g = t / PSC_NRED, k = t - g * PSC_NRED;
+    int64_t r = c * REDUCE_GROUPS + g;
+    constexpr int kStride = REDUCE_GROUPS * REDUCE_CTAS, kAhead = 8;
+    for (; r + (kAhead - 1) * kStride < rows; r += kAhead * kStride) {
+        double v[kAhead];
 #pragma unroll
-    for (int k = 0; k < PSC_NRED; ++k) acc[k] = 0.0;
-    for (int64_t sg = threadIdx.x; sg < nseg; sg += blockDim.x) {
-        const double* p = W.partials + PSC_NRED + sg * REDUCE_SEG * PSC_NRED;
+        for (int j = 0; j < kAhead; ++j) v[j] = body[(r + j * kStride) * PSC_NRED + k];
 #pragma unroll
-        for (int k = 0; k < PSC_NRED; ++k) acc[k] += p[k];
+        for (int j = 0; j < kAhead; ++j) acc += v[j];
     }
-    block_reduce_store<PSC_NRED>(acc, s_red, out + (size_t)blockIdx.x * PSC_NRED);
+    double v[kAhead];
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+        const int64_t q = r + j * kStride;
+        v[j] = q < rows ? body[q * PSC_NRED + k] : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) acc += v[j];
+    s_g[t] = acc;
+    __syncthreads();
+    const int lane = t & 31, col = t >> 5;
+    double x = s_g[lane * PSC_NRED + col];
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) x += __shfl_xor_sync(0xffffffffu, x, s);
+    if (lane == 0) s_cta[col] = x;
+    cluster.sync();
+    if (c == 0 && t < PSC_NRED) {
+        double sum = 0.0;
+#pragma unroll
+        for (int j = 0; j < REDUCE_CTAS; ++j) sum += cluster.map_shared_rank(s_cta, j)[t];
+        out[(size_t)w * PSC_NRED + t] = sum;
+        if (out2) out2[(size_t)w * PSC_NRED + t] = sum;
+        if (CONV) s_g[t] = sum;
+    }
+    cluster.sync();  // the CTAs' sums stay in place until they are read
+    if (CONV && c == 0 && t < 32) {
+        __syncwarp();
+        if (t == 0) converge_check(cc, s_g);
+    }
 }
 
 template <int STORE>
@@ -160,11 +211,16 @@ __global__ void k_stream_pull_store(const double* src, void* dst, int nx, int ny
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-cudaError_t launch_reduce_windows(const psc_window* d_windows, int nwin, double* out, cudaStream_t stream) {
-    k_reduce_segments<<<dim3(REDUCE_SEG_BLOCKS, (unsigned)nwin), STEP_THREADS, 0, stream>>>(d_windows);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    k_reduce_windows<<<nwin, STEP_THREADS, 0, stream>>>(d_windows, out);
+cudaError_t launch_reduce_windows(const psc_window* d_windows, int nwin, double* out, cudaStream_t stream,
+                                  double* out2) {
+    k_reduce_windows<false>
+        <<<nwin * REDUCE_CTAS, REDUCE_THREADS, 0, stream>>>(d_windows, out, out2, ConvergeCheck{});
+    return cudaGetLastError();
+}
+
+cudaError_t launch_reduce_converge(const psc_window* d_window, double* out, const ConvergeCheck& cc,
+                                   cudaStream_t stream) {
+    k_reduce_windows<true><<<REDUCE_CTAS, REDUCE_THREADS, 0, stream>>>(d_window, out, nullptr, cc);
     return cudaGetLastError();
 }
 
