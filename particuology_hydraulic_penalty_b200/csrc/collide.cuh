@@ -541,131 +541,287 @@ namespace psc {
 // window: (1 - B)/tau comes from a per-level table, the Guo terms are split
 // into per-direction constants A_k = 3 pref w_k (c_k . F) and
 // K_k = 9 pref w_k (c_k . F) so that G_i = K_k cu - 3 pref w uF +- A_k.
-template <typename R>
+//
+// V is what one evaluation works on: one cell in float or double, or two cells
+// at once in packed FP32 (F2).  Every product that feeds a sum is an explicit
+// fused multiply-add, so a packed cell and a scalar cell round alike.
+PSC_HD float vadd(float a, float b) { return a + b; }
+PSC_HD double vadd(double a, double b) { return a + b; }
+PSC_HD float vsub(float a, float b) { return a - b; }
+PSC_HD double vsub(double a, double b) { return a - b; }
+#if defined(__CUDA_ARCH__)
+PSC_HD float vmul(float a, float b) { return __fmul_rn(a, b); }
+PSC_HD double vmul(double a, double b) { return __dmul_rn(a, b); }
+PSC_HD float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+PSC_HD double vfma(double a, double b, double c) { return __fma_rn(a, b, c); }
+#else
+PSC_HD float vmul(float a, float b) { return a * b; }
+PSC_HD double vmul(double a, double b) { return a * b; }
+PSC_HD float vfma(float a, float b, float c) { return std::fma(a, b, c); }
+PSC_HD double vfma(double a, double b, double c) { return std::fma(a, b, c); }
+#endif
+
+// Two floats in one 64-bit register pair: the sm_100 instructions on both halves at once (a host
+// build computes the halves one after the other).
+struct F2 {
+    unsigned long long v;
+};
+PSC_HD F2 f2(float a, float b) {
+    F2 r;
+#if defined(__CUDA_ARCH__)
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+#else
+    const float h[2] = {a, b};
+    std::memcpy(&r.v, h, sizeof(r.v));
+#endif
+    return r;
+}
+PSC_HD void f2_get(F2 x, float& a, float& b) {
+#if defined(__CUDA_ARCH__)
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v));
+#else
+    float h[2];
+    std::memcpy(h, &x.v, sizeof(x.v));
+    a = h[0];
+    b = h[1];
+#endif
+}
+#if defined(__CUDA_ARCH__)
+#define PSC_F2_OP2(NAME)                                                                        \
+    PSC_HD F2 v##NAME(F2 a, F2 b) {                                                             \
+        F2 r;                                                                                   \
+        asm(#NAME ".rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));                    \
+        return r;                                                                               \
+    }
+#else
+#define PSC_F2_OP2(NAME)                                                                        \
+    PSC_HD F2 v##NAME(F2 a, F2 b) {                                                             \
+        float a0, a1, b0, b1;                                                                   \
+        f2_get(a, a0, a1);                                                                      \
+        f2_get(b, b0, b1);                                                                      \
+        return f2(v##NAME(a0, b0), v##NAME(a1, b1));                                            \
+    }
+#endif
+PSC_F2_OP2(add)
+PSC_F2_OP2(sub)
+PSC_F2_OP2(mul)
+#undef PSC_F2_OP2
+PSC_HD F2 vfma(F2 a, F2 b, F2 c) {
+    F2 r;
+#if defined(__CUDA_ARCH__)
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+#else
+    float a0, a1, b0, b1, c0, c1;
+    f2_get(a, a0, a1);
+    f2_get(b, b0, b1);
+    f2_get(c, c0, c1);
+    r = f2(vfma(a0, b0, c0), vfma(a1, b1, c1));
+#endif
+    return r;
+}
+
+template <typename V>
+struct Lift {
+    PSC_HD static V of(double x) { return (V)x; }
+};
+template <>
+struct Lift<F2> {
+    PSC_HD static F2 of(double x) { return f2((float)x, (float)x); }
+};
+template <typename V>
+PSC_HD V lift(double x) {
+    return Lift<V>::of(x);
+}
+
+template <typename V>
 struct WinConst {
-    R inv_tau;
-    R trt_ratio;  // omega- / omega+ (1 for BGK)
-    R fx, fy, fz;
-    R pw3[3];  // 3 pref w for the rest, axis and diagonal weights
-    R A[9];    // 3 pref w_k (c_k . F) for the nine direction pairs
-    R K[9];    // 9 pref w_k (c_k . F)
+    V inv_tau;
+    V trt_ratio;  // omega- / omega+ (1 for BGK)
+    V fx, fy, fz;
+    V hfx, hfy, hfz;  // F / 2
+    V npw3[3];        // -3 pref w for the rest, axis and diagonal weights
+    V A[9];           // 3 pref w_k (c_k . F) for the nine direction pairs
+    V K[9];           // 9 pref w_k (c_k . F)
 };
 
 // tau_minus > 0 selects two-relaxation-time collision (symmetric parts relax
 // with 1/tau, antisymmetric with 1/tau_minus; Guo's antisymmetric term takes
 // the prefactor 1 - 1/(2 tau_minus)).  tau_minus = tau is BGK.
-template <typename R>
-PSC_HD void make_win_const(WinConst<R>& c, double tau, double fx, double fy, double fz, double tau_minus = 0.0) {
+template <typename V>
+PSC_HD void make_win_const(WinConst<V>& c, double tau, double fx, double fy, double fz, double tau_minus = 0.0) {
     const double pref = 1.0 - 0.5 / tau;
     const double tm = tau_minus > 0.0 ? tau_minus : tau;
     const double pref_m = 1.0 - 0.5 / tm;
-    c.inv_tau = (R)(1.0 / tau);
-    c.trt_ratio = (R)(tau / tm);
-    c.fx = (R)fx;
-    c.fy = (R)fy;
-    c.fz = (R)fz;
-    c.pw3[0] = (R)(3.0 * pref * W0);
-    c.pw3[1] = (R)(3.0 * pref * W1);
-    c.pw3[2] = (R)(3.0 * pref * W2);
+    c.inv_tau = lift<V>(1.0 / tau);
+    c.trt_ratio = lift<V>(tau / tm);
+    c.fx = lift<V>(fx);
+    c.fy = lift<V>(fy);
+    c.fz = lift<V>(fz);
+    c.hfx = lift<V>(0.5 * fx);
+    c.hfy = lift<V>(0.5 * fy);
+    c.hfz = lift<V>(0.5 * fz);
+    c.npw3[0] = lift<V>(-3.0 * pref * W0);
+    c.npw3[1] = lift<V>(-3.0 * pref * W1);
+    c.npw3[2] = lift<V>(-3.0 * pref * W2);
+#pragma unroll
     for (int k = 0; k < 9; ++k) {
         const int i = 2 * k + 1;
         const double w = wgt(i);
         const double cf = cxv(i) * fx + cyv(i) * fy + czv(i) * fz;
-        c.A[k] = (R)(3.0 * pref_m * w * cf);
-        c.K[k] = (R)(9.0 * pref * w * cf);
+        c.A[k] = lift<V>(3.0 * pref_m * w * cf);
+        c.K[k] = lift<V>(9.0 * pref * w * cf);
     }
 }
 
-// Collide deviations g in place.  B solid weight, kb = (1 - B) / tau.
-// mom receives rho - 1 and the moment velocity u = (m + F/2)/rho of the
-// incoming state; imb the node IMB momentum when IMB.
+// c_i . v for the first direction i of pair K (its first non-zero component is +1).
+template <int K, typename V>
+PSC_HD V cdot_v(V x, V y, V z) {
+    constexpr int i = 2 * K + 1, a = cxv(i), b = cyv(i), c = czv(i);
+    if constexpr (a != 0 && b != 0) return b > 0 ? vadd(x, y) : vsub(x, y);
+    else if constexpr (a != 0 && c != 0) return c > 0 ? vadd(x, z) : vsub(x, z);
+    else if constexpr (b != 0 && c != 0) return c > 0 ? vadd(y, z) : vsub(y, z);
+    else return a != 0 ? x : (b != 0 ? y : z);
+}
+
+template <typename V>
+PSC_HD V sum_populations(const V* g) {
+    return vadd(vadd(vadd(vadd(vadd(g[0], g[1]), vadd(g[2], g[3])), vadd(vadd(g[4], g[5]), vadd(g[6], g[7]))),
+                     vadd(vadd(vadd(g[8], g[9]), vadd(g[10], g[11])), vadd(vadd(g[12], g[13]), vadd(g[14], g[15])))),
+                vadd(vadd(g[16], g[17]), g[18]));
+}
+template <typename V>
+PSC_HD void momentum(const V* g, V& mx, V& my, V& mz) {
+    mx = vadd(vadd(vadd(vsub(g[1], g[2]), vsub(g[7], g[8])), vadd(vsub(g[9], g[10]), vsub(g[11], g[12]))),
+              vsub(g[13], g[14]));
+    my = vadd(vadd(vadd(vsub(g[3], g[4]), vsub(g[7], g[8])), vadd(vsub(g[10], g[9]), vsub(g[15], g[16]))),
+              vsub(g[17], g[18]));
+    mz = vadd(vadd(vadd(vsub(g[5], g[6]), vsub(g[11], g[12])), vadd(vsub(g[14], g[13]), vsub(g[15], g[16]))),
+              vsub(g[18], g[17]));
+}
+// The moments handed on: rho - 1 and u = (m + F/2) / rho of the incoming state.
+template <typename V>
+PSC_HD void moments_v(const WinConst<V>& c, V drho, V irho, V mx, V my, V mz, V* mom) {
+    mom[0] = drho;
+    mom[1] = vmul(vadd(mx, c.hfx), irho);
+    mom[2] = vmul(vadd(my, c.hfy), irho);
+    mom[3] = vmul(vadd(mz, c.hfz), irho);
+}
+
+// What the nine pairs of a cell share (see collide_v).
+template <typename V>
+struct PairTerms {
+    V uex, uey, uez, usx, usy, usz, uus15;
+    V omB, bB, B, B2;
+    V wr[2], q[2], b[2], t[2], a[2];  // axis and diagonal weights
+};
+
+template <int K, bool MOVING, bool IMB, typename V>
+PSC_HD void collide_pair_v(V* g, const WinConst<V>& c, const PairTerms<V>& p, V* imb) {
+    constexpr int i = 2 * K + 1, j = i + 1, d = i < 7 ? 0 : 1;
+    const V cu = cdot_v<K>(p.uex, p.uey, p.uez);
+    V S = vfma(cu, vfma(p.q[d], cu, c.K[K]), p.b[d]);
+    V T = vfma(p.t[d], cu, c.A[K]);
+    const V gi = g[i], gj = g[j];
+    V h = vsub(gj, gi);  // + h: (os_i - os_j) / 2
+    if (IMB) h = vfma(p.a[d], cu, h);
+    if (MOVING) {
+        const V cus = cdot_v<K>(p.usx, p.usy, p.usz);
+        S = vfma(p.B, vmul(p.wr[d], vsub(vmul(lift<V>(4.5), vmul(cus, cus)), p.uus15)), S);
+        const V hs = vmul(p.a[d], cus);
+        T = vfma(p.B, hs, T);
+        if (IMB) h = vadd(h, hs);
+    }
+    g[i] = vfma(p.omB, gi, vfma(p.bB, gj, vadd(S, T)));
+    g[j] = vfma(p.omB, gj, vfma(p.bB, gi, vsub(S, T)));
+    if (IMB) {
+        const V dm = vmul(p.B2, h);
+        if constexpr (cxv(i) != 0) imb[0] = K == 0 ? dm : vadd(imb[0], dm);
+        if constexpr (cyv(i) != 0) imb[1] = K == 1 ? dm : (cyv(i) > 0 ? vadd(imb[1], dm) : vsub(imb[1], dm));
+        if constexpr (czv(i) != 0) imb[2] = K == 2 ? dm : (czv(i) > 0 ? vadd(imb[2], dm) : vsub(imb[2], dm));
+    }
+}
+
+// Collide deviations g in place.  drho = rho - 1 and irho = 1 / rho of the
+// incoming state, B solid weight, kb = (1 - B) / tau.  mom receives rho - 1
+// and the moment velocity u = (m + F/2)/rho of the incoming state when
+// want_mom; imb the node IMB momentum when IMB.
+//
+// The collision regrouped per population pair.  With geq = w drho + wrq +- asym, the solid
+// terms os_i = (g_j - g_i) + e + h, os_j = (g_i - g_j) + e - h (e = -wrq + e_s,
+// h = asym + h_s, e_s and h_s from the solid velocity), Guo's G = K cu - 3 pref w uF +- A,
+// and the fluid part relaxing the pair's symmetric half with kb and its antisymmetric half
+// with kbm (= kb for BGK; TRT: kb omega-/omega+):
+//   g_i' = a g_i + b g_j + S + T,   g_j' = a g_j + b g_i + S - T,
+//   a = 1 - (kb + kbm)/2 - B,  b = B + (kbm - kb)/2   (BGK: 1 - kb - B and B),
+//   S = K cu + (kb - B) wrq + (kb w drho - 3 pref w uF) + B e_s,
+//   T = 3 (kbm + B) w rho cu + B h_s + A,
+// and the pair's IMB momentum B (os_i - os_j) = 2 B ((g_j - g_i) + h).  With
+// wrq = w rho (4.5 cu^2 - 1.5 u^2), S without e_s is the quadratic cu (q cu + K) + b,
+// q = 4.5 (kb - B) w rho, b = kb w drho - 3 pref w uF - (kb - B) w rho 1.5 u^2: two FMAs per
+// pair.  The per-weight factors are computed once per cell.
+template <typename V, bool MOVING, bool IMB, bool TRT>
+PSC_HD void collide_v(V* g, const WinConst<V>& c, V drho, V irho, V B, V kb, V usx, V usy, V usz, V* mom, V* imb,
+                      bool want_mom) {
+    const V one = lift<V>(1.0), half = lift<V>(0.5);
+    const V rho = vadd(one, drho);
+    V mx, my, mz;
+    momentum(g, mx, my, mz);
+    if (want_mom) moments_v(c, drho, irho, mx, my, mz, mom);  // (plain steps store no moments)
+    PairTerms<V> p;
+    p.uex = vmul(vadd(mx, c.fx), irho);
+    p.uey = vmul(vadd(my, c.fy), irho);
+    p.uez = vmul(vadd(mz, c.fz), irho);
+    const V uu15 = vmul(lift<V>(1.5), vfma(p.uez, p.uez, vfma(p.uey, p.uey, vmul(p.uex, p.uex))));
+    const V uF = vfma(p.uez, c.fz, vfma(p.uey, c.fy, vmul(p.uex, c.fx)));
+    const V omk = vsub(one, kb);
+    const V rq = vmul(rho, uu15);
+    V e0 = rq;  // rho (1.5 u^2 - 1.5 us^2)
+    if (MOVING) {
+        p.usx = usx;
+        p.usy = usy;
+        p.usz = usz;
+        p.uus15 = vmul(lift<V>(1.5), vfma(usz, usz, vfma(usy, usy, vmul(usx, usx))));
+        e0 = vmul(rho, vsub(uu15, p.uus15));
+    }
+    {
+        const V geq = vmul(lift<V>(W0), vsub(drho, rq));
+        const V os = vmul(lift<V>(W0), e0);
+        g[0] = vfma(omk, g[0], vfma(kb, geq, vfma(B, os, vmul(c.npw3[0], uF))));
+    }
+    const V kbm = TRT ? vmul(kb, c.trt_ratio) : kb;
+    p.B = B;
+    p.omB = TRT ? vsub(vsub(one, vmul(half, vadd(kb, kbm))), B) : vsub(omk, B);
+    p.bB = TRT ? vfma(half, vsub(kbm, kb), B) : B;
+    p.B2 = vadd(B, B);
+    const V kmB = vsub(kb, B), kbd = vmul(kb, drho), kp3 = vmul(lift<V>(3.0), vadd(kbm, B));
+#pragma unroll
+    for (int d = 0; d < 2; ++d) {
+        const V w = lift<V>(d == 0 ? W1 : W2);
+        const V wr = vmul(w, rho), m = vmul(kmB, wr);
+        p.wr[d] = wr;
+        p.q[d] = vmul(lift<V>(4.5), m);
+        p.b[d] = vsub(vfma(w, kbd, vmul(c.npw3[1 + d], uF)), vmul(m, uu15));
+        p.t[d] = vmul(kp3, wr);
+        p.a[d] = vmul(lift<V>(3.0), wr);
+    }
+    collide_pair_v<0, MOVING, IMB>(g, c, p, imb);
+    collide_pair_v<1, MOVING, IMB>(g, c, p, imb);
+    collide_pair_v<2, MOVING, IMB>(g, c, p, imb);
+    collide_pair_v<3, MOVING, IMB>(g, c, p, imb);
+    collide_pair_v<4, MOVING, IMB>(g, c, p, imb);
+    collide_pair_v<5, MOVING, IMB>(g, c, p, imb);
+    collide_pair_v<6, MOVING, IMB>(g, c, p, imb);
+    collide_pair_v<7, MOVING, IMB>(g, c, p, imb);
+    collide_pair_v<8, MOVING, IMB>(g, c, p, imb);
+}
+
+// collide_v with the density taken from g; irho_hint: 1 / rho where the caller has it, else 0.
 template <typename R, bool MOVING, bool IMB, bool TRT = false>
 PSC_HD void collide_fast2(R* g, const WinConst<R>& c, R B, R kb, R usx, R usy, R usz, R irho_hint, R* mom,
                           R* imb, bool want_mom = true) {
-    const R kbm = kb * c.trt_ratio;
-    (void)kbm;
-    const R drho = (((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + (g[6] + g[7]))) +
-                   (((g[8] + g[9]) + (g[10] + g[11])) + ((g[12] + g[13]) + (g[14] + g[15]))) +
-                   ((g[16] + g[17]) + g[18]);
-    const R rho = R(1) + drho;
-    const R irho = irho_hint > R(0) ? irho_hint : R(1) / rho;
-    const R mx = ((g[1] - g[2]) + (g[7] - g[8])) + ((g[9] - g[10]) + (g[11] - g[12])) + (g[13] - g[14]);
-    const R my = ((g[3] - g[4]) + (g[7] - g[8])) + ((g[10] - g[9]) + (g[15] - g[16])) + (g[17] - g[18]);
-    const R mz = ((g[5] - g[6]) + (g[11] - g[12])) + ((g[14] - g[13]) + (g[15] - g[16])) + (g[18] - g[17]);
-    if (want_mom) {  // (plain steps of the throughput kernels store no moments)
-        mom[0] = drho;
-        mom[1] = (mx + R(0.5) * c.fx) * irho;
-        mom[2] = (my + R(0.5) * c.fy) * irho;
-        mom[3] = (mz + R(0.5) * c.fz) * irho;
-    }
-    const R uex = (mx + c.fx) * irho, uey = (my + c.fy) * irho, uez = (mz + c.fz) * irho;
-    const R uu15 = R(1.5) * (uex * uex + uey * uey + uez * uez);
-    const R uF = uex * c.fx + uey * c.fy + uez * c.fz;
-    const R omk = R(1) - kb;
-    R uus15 = R(0);
-    if (MOVING) uus15 = R(1.5) * (usx * usx + usy * usy + usz * usz);
-    R ax = R(0), ay = R(0), az = R(0);
-    {
-        const R w = R(W0);
-        const R geq = w * (drho - rho * uu15);
-        const R os = w * rho * (uu15 - uus15);
-        g[0] = omk * g[0] + kb * geq + B * os - c.pw3[0] * uF;
-    }
-    // The collision regrouped per population pair.  With geq = w drho + wrq +- asym, the solid
-    // terms os_i = (g_j - g_i) + e + h, os_j = (g_i - g_j) + e - h (e = -wrq + e_s,
-    // h = asym + h_s, e_s and h_s from the solid velocity), Guo's G = K cu - 3 pref w uF +- A,
-    // and the fluid part relaxing the pair's symmetric half with kb and its antisymmetric half
-    // with kbm (= kb for BGK; TRT: kb omega-/omega+):
-    //   g_i' = a g_i + b g_j + S + T,   g_j' = a g_j + b g_i + S - T,
-    //   a = 1 - (kb + kbm)/2 - B,  b = B + (kbm - kb)/2   (BGK: 1 - kb - B and B),
-    //   S = K cu + (kb - B) wrq + (kb w drho - 3 pref w uF) + B e_s,
-    //   T = 3 (kbm + B) w rho cu + B h_s + A,
-    // and the pair's IMB momentum B (os_i - os_j) = 2 B ((g_j - g_i) + h).  With
-    // wrq = w rho (4.5 cu^2 - 1.5 u^2), S without e_s is the quadratic cu (q cu + K) + b,
-    // q = 4.5 (kb - B) w rho, b = kb w drho - 3 pref w uF - (kb - B) w rho 1.5 u^2: two FMAs per
-    // pair.  The per-weight factors are computed once per cell.
-    const R omB = TRT ? R(1) - R(0.5) * (kb + kbm) - B : omk - B;
-    const R bB = TRT ? B + R(0.5) * (kbm - kb) : B;
-    const R kmB = kb - B, B2 = B + B;
-    const R kbd = kb * drho;
-    const R wr1 = R(W1) * rho, wr2 = R(W2) * rho;
-    const R m1 = kmB * wr1, m2 = kmB * wr2;
-    const R q1 = R(4.5) * m1, q2 = R(4.5) * m2;
-    const R b1 = (R(W1) * kbd - c.pw3[1] * uF) - m1 * uu15, b2 = (R(W2) * kbd - c.pw3[2] * uF) - m2 * uu15;
-    const R kp3 = R(3) * ((TRT ? kbm : kb) + B);
-    const R t1 = kp3 * wr1, t2 = kp3 * wr2;
-    const R a1 = R(3) * wr1, a2 = R(3) * wr2;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) {
-        const int i = 2 * k + 1, j = i + 1;
-        const bool axis = i < 7;
-        const R wr = axis ? wr1 : wr2;
-        const R cu = csel(cxv(i), uex) + csel(cyv(i), uey) + csel(czv(i), uez);
-        R S = cu * ((axis ? q1 : q2) * cu + c.K[k]) + (axis ? b1 : b2);
-        R T = (axis ? t1 : t2) * cu + c.A[k];
-        R h = (axis ? a1 : a2) * cu;
-        if (MOVING) {
-            const R cus = csel(cxv(i), usx) + csel(cyv(i), usy) + csel(czv(i), usz);
-            S += B * (wr * (R(4.5) * cus * cus - uus15));
-            const R hs = R(3) * wr * cus;
-            T += B * hs;
-            h += hs;
-        }
-        const R gi = g[i], gj = g[j];
-        g[i] = omB * gi + (bB * gj + (S + T));
-        g[j] = omB * gj + (bB * gi + (S - T));
-        if (IMB) {
-            const R dm = B2 * ((gj - gi) + h);
-            ax += csel(cxv(i), dm);
-            ay += csel(cyv(i), dm);
-            az += csel(czv(i), dm);
-        }
-    }
-    if (IMB) {
-        imb[0] = ax;
-        imb[1] = ay;
-        imb[2] = az;
-    }
+    const R drho = sum_populations(g);
+    const R irho = irho_hint > R(0) ? irho_hint : R(1) / (R(1) + drho);
+    collide_v<R, MOVING, IMB, TRT>(g, c, drho, irho, B, kb, usx, usy, usz, mom, imb, want_mom);
 }
 
 }  // namespace psc

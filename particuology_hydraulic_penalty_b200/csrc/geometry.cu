@@ -904,10 +904,9 @@ __global__ void __launch_bounds__(LOAD_THREADS) k_loads_list_build_multi(const L
 // Per-particle sums of the chunk partials c0 .. c1-1: one warp per particle,
 // lane l sums chunks c0 + l, c0 + l + 32, ... in order, then a fixed shuffle tree.
 __device__ __forceinline__ void particle_sums(const double* part, int64_t c0, int64_t c1, double* force,
-                                              double* torque, double (&F)[6]) {
+                                              double* torque) {
     const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) F[k] = 0.0;
+    double F[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     for (int64_t c = c0 + lane; c < c1; c += 32) {
 #pragma unroll
         for (int k = 0; k < 6; ++k) F[k] += part[c * 6 + k];
@@ -927,8 +926,7 @@ __global__ void __launch_bounds__(256) k_loads_particles(psc_geometry g, const d
                                                          double* torques) {
     const int p = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
     if (p >= g.nparticles) return;  // warp-uniform
-    double F[6];
-    particle_sums(part, g.chunk_off[p], g.chunk_off[p + 1], forces + (size_t)p * 3, torques + (size_t)p * 3, F);
+    particle_sums(part, g.chunk_off[p], g.chunk_off[p + 1], forces + (size_t)p * 3, torques + (size_t)p * 3);
 }
 
 __device__ __forceinline__ void write_loads_diag(const double (&r)[5], const double* imb_sums, double* diag,
@@ -986,39 +984,66 @@ __device__ __forceinline__ void loads_diag_block(int P, const double* imb_sums, 
     }
 }
 
-// Per-particle sums and the diagnostics of one window by one cluster, a warp per particle in turn: one
-// launch where a kernel over the particles and a one-block kernel over the forces were two (2.1 + 3.4 us
-// with 128 particles, 3.2 + 5.4 us with 1136).  For windows of up to FINAL_PARTICLES particles: beyond, a
-// cluster's 256 warps take more turns than the whole GPU's.
+// Per-particle sums and the diagnostics of one window by one cluster: one launch where a kernel over
+// the particles and a one-block kernel over the forces were two (2.1 + 3.4 us with 128 particles,
+// 3.2 + 5.4 us with 1136).  Eight lanes add a particle's chunks c0 + l, c0 + l + 8, ... in order and
+// then by a shuffle tree: most particles own one chunk, the largest of a packed window some forty
+// (a warp per particle took 14 us with 1136).  For windows of up to FINAL_PARTICLES particles: beyond,
+// one cluster takes more turns than the whole GPU.
 constexpr int FINAL_CTAS = 8;
-constexpr int FINAL_THREADS = 1024;
+constexpr int FINAL_THREADS = 512;
+constexpr int FINAL_LANES = 8;
 constexpr int FINAL_PARTICLES = 4096;
 
 __device__ __forceinline__ void loads_final_cluster(int P, const int64_t* chunk_off, const double* part,
                                                     const double* imb_sums, double* forces, double* torques,
                                                     double* diag, double* host_diag) {
     namespace cg = cooperative_groups;
-    __shared__ double s_w[FINAL_THREADS / 32][5];
+    constexpr int kWarps = FINAL_THREADS / 32, kGroups = FINAL_CTAS * FINAL_THREADS / FINAL_LANES;
+    __shared__ double s_w[kWarps][5];
     __shared__ double s_cta[5];
     cg::cluster_group cluster = cg::this_cluster();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % FINAL_LANES;
     double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // sum Fx, Fy, Fz, max |F|^2, max |T|^2
-    for (int p = (int)cluster.block_rank() * (FINAL_THREADS / 32) + warp; p < P; p += FINAL_CTAS * (FINAL_THREADS / 32)) {
-        double F[6];
-        particle_sums(part, chunk_off[p], chunk_off[p + 1], forces + (size_t)p * 3, torques + (size_t)p * 3, F);
-        v[0] += F[0];
-        v[1] += F[1];
-        v[2] += F[2];
-        v[3] = fmax(v[3], F[0] * F[0] + F[1] * F[1] + F[2] * F[2]);
-        v[4] = fmax(v[4], F[3] * F[3] + F[4] * F[4] + F[5] * F[5]);
-    }
-    if (lane == 0) {
+    const int first = ((int)cluster.block_rank() * FINAL_THREADS + (int)threadIdx.x) / FINAL_LANES;
+    for (int p0 = first - first % (32 / FINAL_LANES); p0 < P; p0 += kGroups) {  // warp-uniform
+        const int p = p0 + lane / FINAL_LANES;
+        const int64_t c0 = p < P ? chunk_off[p] : 0, c1 = p < P ? chunk_off[p + 1] : 0;
+        double F[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        for (int64_t c = c0 + sub; c < c1; c += FINAL_LANES) {
 #pragma unroll
-        for (int k = 0; k < 5; ++k) s_w[warp][k] = v[k];
+            for (int k = 0; k < 6; ++k) F[k] += part[c * 6 + k];
+        }
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+#pragma unroll
+            for (int o = FINAL_LANES / 2; o > 0; o >>= 1) F[k] += __shfl_xor_sync(0xffffffffu, F[k], o);
+        }
+        if (p < P) {
+            const double mine = sub == 0 ? F[0] : (sub == 1 ? F[1] : (sub == 2 ? F[2] : (sub == 3 ? F[3] : (sub == 4 ? F[4] : F[5]))));
+            if (sub < 3) forces[(size_t)p * 3 + sub] = mine;
+            else if (sub < 6) torques[(size_t)p * 3 + sub - 3] = mine;
+            if (sub == 0) {
+                v[0] += F[0];
+                v[1] += F[1];
+                v[2] += F[2];
+                v[3] = fmax(v[3], F[0] * F[0] + F[1] * F[1] + F[2] * F[2]);
+                v[4] = fmax(v[4], F[3] * F[3] + F[4] * F[4] + F[5] * F[5]);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {  // the warp's groups (their first lanes hold the values)
+#pragma unroll
+        for (int o = 16; o >= FINAL_LANES; o >>= 1) {
+            const double y = __shfl_xor_sync(0xffffffffu, v[k], o);
+            v[k] = k < 3 ? v[k] + y : fmax(v[k], y);
+        }
+        if (lane == 0) s_w[warp][k] = v[k];
     }
     __syncthreads();
     if (warp < 5) {  // a warp per value: the CTA's warps by a shuffle tree
-        double x = s_w[lane][warp];
+        double x = lane < kWarps ? s_w[lane % kWarps][warp] : 0.0;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             const double y = __shfl_xor_sync(0xffffffffu, x, o);
@@ -1152,9 +1177,8 @@ __global__ void __launch_bounds__(256) k_loads_particles_multi(const LoadsJob* j
     const int k = owner_of(particle_base, njobs, gp);
     const LoadsJob& J = jobs[k];
     const int p = (int)(gp - particle_base[k]);
-    double F[6];
     particle_sums(part + chunk_base[k] * 6, J.g.chunk_off[p], J.g.chunk_off[p + 1], J.forces + (size_t)p * 3,
-                  J.torques + (size_t)p * 3, F);
+                  J.torques + (size_t)p * 3);
 }
 
 __global__ void __launch_bounds__(1024) k_loads_diag_multi(const LoadsJob* jobs) {

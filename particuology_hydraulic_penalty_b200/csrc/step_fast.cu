@@ -14,6 +14,7 @@
 
 namespace psc {
 
+
 // Resident CTAs the register allocation aims for: four (64 registers) for
 // FP32/FP16/BF16 storage, three with moving particles (the solid-velocity
 // terms), two for FP64, whose arithmetic needs about twice the registers, and
@@ -40,15 +41,24 @@ __global__ void __launch_bounds__(STEP_THREADS, (StepOccupancy<STORE, MOVING, RE
     const int64_t t0 = (total_tiles * (int64_t)blockIdx.x) / gridDim.x;
     const int64_t t1 = (total_tiles * ((int64_t)blockIdx.x + 1)) / gridDim.x;
     int64_t win_end = -1;
-    double red[PSC_NRED];  // this thread's sums over the CTA's cells of the current window
+    // FP64: two CTAs' registers do not hold the sums too (160^3 with IMB: 247 us against 260); FP32 runs as
+    // fast either way at 97^3 and slower at 49^3 (10.5 against 9.3 us)
+    constexpr bool SHARED = RED && STORE == PSC_STORE_F64;
+    __shared__ double s_red[SHARED ? PSC_NRED : 1][STEP_THREADS];
+    CellSums<SHARED> red;  // this thread's sums over the CTA's cells of the current window
+    red.s = s_red;
+    if (RED) red.clear();
+    const auto flush = [&]() {
+        double v[PSC_NRED];
 #pragma unroll
-    for (int q = 0; q < PSC_NRED; ++q) red[q] = 0.0;
+        for (int q = 0; q < PSC_NRED; ++q) v[q] = red.at(q);
+        flush_segment<PSC_NRED>(v, sw.partials, sw.tile_begin, sw.tile_end - sw.tile_begin, total_tiles, gridDim.x);
+        red.clear();
+    };
     bool have = false;  // block-uniform: red holds cells of the window in sw
     for (int64_t t = t0; t < t1; ++t) {
         if (t >= win_end) {  // block-uniform: entering a new window
-            if (do_red && have)
-                flush_segment<PSC_NRED>(red, sw.partials, sw.tile_begin, sw.tile_end - sw.tile_begin, total_tiles,
-                                        gridDim.x);
+            if (do_red && have) flush();
             have = false;
             __syncthreads();
             const int wi = find_window(wins, nullptr, nwin, t);
@@ -130,8 +140,7 @@ __global__ void __launch_bounds__(STEP_THREADS, (StepOccupancy<STORE, MOVING, RE
             }
         }
     }
-    if (do_red && have)
-        flush_segment<PSC_NRED>(red, sw.partials, sw.tile_begin, sw.tile_end - sw.tile_begin, total_tiles, gridDim.x);
+    if (do_red && have) flush();
 }
 
 template <int STORE, bool MOVING, int CPT, bool RED>

@@ -10,10 +10,13 @@
 // accesses at two CTAs per SM move 6.5 TB/s against 5.1-5.9 TB/s for scalar
 // ones.  The per-cell arithmetic is fast_cell(), the same function as the
 // one-cell kernel's, so both produce identical populations.
+#include <type_traits>
+
 #include "fast_cell.cuh"
 #include "internal.cuh"
 
 namespace psc {
+
 
 // Set (once) when a launch met a window it cannot run: 0x201 odd nz,
 // 0x202 tiles not planned by psc_plan_pair_tiles.  Such windows are skipped.
@@ -68,7 +71,13 @@ __global__ void __launch_bounds__(STEP_THREADS, (PairOccupancy<STORE, MOVING, RE
     using T = typename TR::T;
     using R = typename TR::R;
     using O = typename TR::O;
-    __shared__ FastWin<T, R, O> sw;
+        // Both cells in packed FP32 where the arithmetic bounds the kernel: 16-bit storage (160^3: 90 -> 82 us
+    // plain, 107 -> 99 with IMB and sums; 378 -> 261 instructions per cell).  FP32 storage is bound by HBM,
+    // and there the packed form was slower (114 against 108 us: its shorter bursts of arithmetic leave
+    // reads and writes less spread).  FP64 has no packed form.
+    constexpr bool PACKED = sizeof(T) == 2;
+    using V = std::conditional_t<PACKED, F2, R>;
+    __shared__ FastWin<T, R, O, V> sw;
     static_assert(STEP_THREADS / 32 == PSC_PARTIAL_ROWS, "one partial row per warp");
     const bool do_collide = flags & PSC_STEP_COLLIDE;
     const bool do_imb = do_collide && (flags & PSC_STEP_IMB);
@@ -77,9 +86,18 @@ __global__ void __launch_bounds__(STEP_THREADS, (PairOccupancy<STORE, MOVING, RE
     const int64_t t0 = (total_tiles * (int64_t)blockIdx.x) / gridDim.x;
     const int64_t t1 = (total_tiles * ((int64_t)blockIdx.x + 1)) / gridDim.x;
     int64_t win_end = -1;
-    double red[PSC_NRED];
+    constexpr bool SHARED = RED && PACKED;  // (107 -> 104 us with the sums in registers, 99 in shared memory)
+    __shared__ double s_red[SHARED ? PSC_NRED : 1][STEP_THREADS];
+    CellSums<SHARED> red;  // this thread's sums over the CTA's cells of the current window
+    red.s = s_red;
+    if (RED) red.clear();
+    const auto flush = [&]() {
+        double v[PSC_NRED];
 #pragma unroll
-    for (int q = 0; q < PSC_NRED; ++q) red[q] = 0.0;
+        for (int q = 0; q < PSC_NRED; ++q) v[q] = red.at(q);
+        flush_segment<PSC_NRED>(v, sw.partials, sw.tile_begin, sw.tile_end - sw.tile_begin, total_tiles, gridDim.x);
+        red.clear();
+    };
     bool have = false;
     bool skip = false;  // block-uniform: the window in sw cannot run here
     // this thread's first cell (ix, iy, iz) in the current tile: divided out when the CTA enters a
@@ -88,9 +106,7 @@ __global__ void __launch_bounds__(STEP_THREADS, (PairOccupancy<STORE, MOVING, RE
     uint32_t ix = 0, iy = 0, iz = 0;
     for (int64_t t = t0; t < t1; ++t) {
         if (t >= win_end) {  // block-uniform: entering a new window
-            if (do_red && have)
-                flush_segment<PSC_NRED>(red, sw.partials, sw.tile_begin, sw.tile_end - sw.tile_begin, total_tiles,
-                                        gridDim.x);
+            if (do_red && have) flush();
             have = false;
             __syncthreads();
             const int wi = find_window(wins, nullptr, nwin, t);
@@ -121,7 +137,6 @@ __global__ void __launch_bounds__(STEP_THREADS, (PairOccupancy<STORE, MOVING, RE
             ix += sw.tstep_x + cy;
         }
         if (c0 >= N) continue;  // N is even: c0 + 1 < N as well (the window's last tile)
-        const uint32_t c1 = c0 + 1;
         const bool open_x = sw.open_x;
         const bool inlet = open_x && ix == 0;
         const int32_t nyz = (int32_t)(ny * nz);
@@ -134,48 +149,76 @@ __global__ void __launch_bounds__(STEP_THREADS, (PairOccupancy<STORE, MOVING, RE
         const int32_t zm0 = iz == 0 ? (int32_t)nz - 1 : -1;
         const int32_t zp1 = iz + 2 == nz ? -(int32_t)(nz - 1) : 1;
         const T* src = sw.src;
-        R g0[Q], g1[Q];
+        V g[PACKED ? 1 : 2][Q], mom[PACKED ? 1 : 2][4], imb[PACKED ? 1 : 2][3];
         uint32_t plane = 0;
 #pragma unroll
         for (int i = 0; i < Q; ++i) {
             const int32_t oxy = (cxv(i) == 1 ? xm : (cxv(i) == -1 ? xp : 0)) + (cyv(i) == 1 ? ym : (cyv(i) == -1 ? yp : 0));
             const T* p = src + (int64_t)(int32_t)(plane + c0 + (uint32_t)oxy);
+            R a, b;
             if (czv(i) == 0) {
-                ld_pair(p, g0[i], g1[i]);  // c0 even, oxy a multiple of nz (even): aligned
+                ld_pair(p, a, b);  // c0 even, oxy a multiple of nz (even): aligned
             } else if (czv(i) == 1) {
-                g0[i] = ld_pop(p + zm0);
-                g1[i] = ld_pop(p);
+                a = ld_pop(p + zm0);
+                b = ld_pop(p);
             } else {
-                g0[i] = ld_pop(p + 1);
-                g1[i] = ld_pop(p + 1 + zp1);
+                a = ld_pop(p + 1);
+                b = ld_pop(p + 1 + zp1);
+            }
+            if constexpr (PACKED) {
+                g[0][i] = f2(a, b);
+            } else {
+                g[0][i] = a;
+                g[1][i] = b;
             }
             plane += N;
         }
-        R mom0[4], imb0[3], mom1[4], imb1[3];
-        fast_cell<TR, MOVING, RED>(sw, g0, c0, N, inlet, do_collide, do_imb, mom0, imb0, red, do_mom);
-        fast_cell<TR, MOVING, RED>(sw, g1, c1, N, inlet, do_collide, do_imb, mom1, imb1, red, do_mom);
+        if constexpr (PACKED) {
+            fast_cell_pair<TR, MOVING, RED>(sw, g[0], c0, N, inlet, do_collide, do_imb, mom[0], imb[0], red, do_mom);
+        } else {
+            fast_cell<TR, MOVING, RED>(sw, g[0], c0, N, inlet, do_collide, do_imb, mom[0], imb[0], red, do_mom);
+            fast_cell<TR, MOVING, RED>(sw, g[1], c0 + 1, N, inlet, do_collide, do_imb, mom[1], imb[1], red, do_mom);
+        }
+        // the two cells' values of one V (packed) or of the two scalars
+        const auto both = [](const auto& v, int k, R& x, R& y) {
+            if constexpr (PACKED) {
+                f2_get(v[0][k], x, y);
+            } else {
+                x = v[0][k];
+                y = v[1][k];
+            }
+        };
         if (do_collide) {
             T* dst = sw.dst + c0;
             uint32_t pl = 0;
 #pragma unroll
             for (int i = 0; i < Q; ++i) {
-                if (TR::scaled) st_pair(dst + pl, g0[i] * sw.scale, g1[i] * sw.scale);
-                else st_pair(dst + pl, g0[i], g1[i]);
+                if constexpr (PACKED && TR::scaled) g[0][i] = vmul(g[0][i], f2(sw.scale, sw.scale));
+                R x, y;
+                both(g, i, x, y);
+                st_pair(dst + pl, x, y);
                 pl += N;
             }
             if (do_imb) {
 #pragma unroll
-                for (int k = 0; k < 3; ++k) st_pair(sw.imb + (size_t)k * N + c0, (O)imb0[k], (O)imb1[k]);
+                for (int k = 0; k < 3; ++k) {
+                    R x, y;
+                    both(imb, k, x, y);
+                    st_pair(sw.imb + (size_t)k * N + c0, (O)x, (O)y);
+                }
             }
         }
         if (do_mom) {
-            st_pair(sw.mom + c0, (O)(R(1) + mom0[0]), (O)(R(1) + mom1[0]));
 #pragma unroll
-            for (int k = 1; k < 4; ++k) st_pair(sw.mom + (size_t)k * N + c0, (O)mom0[k], (O)mom1[k]);
+            for (int k = 0; k < 4; ++k) {
+                R x, y;
+                both(mom, k, x, y);
+                if (k == 0) st_pair(sw.mom + c0, (O)(R(1) + x), (O)(R(1) + y));
+                else st_pair(sw.mom + (size_t)k * N + c0, (O)x, (O)y);
+            }
         }
     }
-    if (do_red && have)
-        flush_segment<PSC_NRED>(red, sw.partials, sw.tile_begin, sw.tile_end - sw.tile_begin, total_tiles, gridDim.x);
+    if (do_red && have) flush();
 }
 
 template <int STORE, bool MOVING, bool RED>
