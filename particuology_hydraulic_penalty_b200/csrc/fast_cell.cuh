@@ -22,7 +22,7 @@ struct FastWin {
     int64_t tile_end;
     uint32_t nx, ny, nz, N;
     uint32_t step_x, step_y, step_z;     // blockDim cells as a mixed-radix (x, y, z) increment
-    uint32_t tstep_x, tstep_y, tstep_z;  // tile_cells cells (one tile on) likewise
+    uint32_t tstep_x, tstep_y, tstep_z;  // a CTA's next tile (tile_cells * stride cells on) likewise
     int32_t tile_cells;
     int32_t moving;
     int32_t inactive;
@@ -37,8 +37,25 @@ struct FastWin {
     R tau;
 };
 
+// What the level tables and the collision constants depend on.
+struct FastKey {
+    double tau, tau_minus, f[3];
+    int32_t S, level;
+    __device__ __forceinline__ bool operator==(const FastKey& o) const {
+        return tau == o.tau && tau_minus == o.tau_minus && f[0] == o.f[0] && f[1] == o.f[1] && f[2] == o.f[2] &&
+               S == o.S && level == o.level;
+    }
+};
+__device__ __forceinline__ FastKey fast_key(const psc_window& W) {
+    return {W.tau, W.tau_minus, {W.force[0], W.force[1], W.force[2]}, W.subsamples, W.level != nullptr ? 1 : 0};
+}
+
+// stride: tiles from one of the CTA's tiles to its next.  prev: the window loaded before, or null.  The windows of a batch mostly share their relaxation time
+// and force: their tables and constants stay.
 template <typename T, typename R, typename O, typename V>
-__device__ void load_fast_win(FastWin<T, R, O, V>& s, const psc_window& W, bool moving_launch) {
+__device__ void load_fast_win(FastWin<T, R, O, V>& s, const psc_window& W, bool moving_launch, int32_t stride,
+                              const psc_window* prev) {
+    const bool same = prev && fast_key(*prev) == fast_key(W);
     // one warp fills the scalar part, all threads the level tables
     if (threadIdx.x == 0) {
         s.src = reinterpret_cast<const T*>(W.f_src);
@@ -59,9 +76,9 @@ __device__ void load_fast_win(FastWin<T, R, O, V>& s, const psc_window& W, bool 
         s.step_z = blockDim.x % (uint32_t)W.nz;
         s.step_y = q % (uint32_t)W.ny;
         s.step_x = q / (uint32_t)W.ny;
-        const uint32_t tc = W.tile_cells > 0 ? (uint32_t)W.tile_cells : 0u;
-        const uint32_t tq = tc / (uint32_t)W.nz;
-        s.tstep_z = tc % (uint32_t)W.nz;
+        const uint64_t tc = W.tile_cells > 0 ? (uint64_t)W.tile_cells * stride : 0u;
+        const uint32_t tq = tc < s.N ? (uint32_t)tc / (uint32_t)W.nz : 0u;  // (a longer step leaves the window)
+        s.tstep_z = tc < s.N ? (uint32_t)tc % (uint32_t)W.nz : 0u;
         s.tstep_y = tq % (uint32_t)W.ny;
         s.tstep_x = tq / (uint32_t)W.ny;
         s.tile_cells = W.tile_cells;
@@ -71,17 +88,17 @@ __device__ void load_fast_win(FastWin<T, R, O, V>& s, const psc_window& W, bool 
         s.inv_scale = (R)(1.0 / W.store_scale);
         s.tau = (R)W.tau;
         s.inv_tau = (R)(1.0 / W.tau);
-        make_win_const(s.c, W.tau, W.force[0], W.force[1], W.force[2], W.tau_minus);
         s.trt = W.tau_minus > 0.0 ? 1 : 0;
         s.open_x = (W.flags & PSC_WIN_OPEN_X) ? 1 : 0;
     }
+    if (threadIdx.x == 32 && !same) make_win_const(s.c, W.tau, W.force[0], W.force[1], W.force[2], W.tau_minus);
     if ((W.flags & PSC_WIN_OPEN_X) && threadIdx.x < Q) {
         const int i = threadIdx.x;
         s.corr[i] = (R)inlet_correction_exact(i, W.inlet_rho, W.inlet_u[0], W.inlet_u[1], W.inlet_u[2]);
     }
     const int S = W.subsamples;
     const int S3 = S * S * S;
-    if (W.level) {
+    if (W.level && !same) {
         for (int l = threadIdx.x; l <= S3 && l < 256; l += blockDim.x) {
             const double al = (double)l / (double)S3;
             const double B = al / (al + W.tau * (1.0 - al) + 1.0e-14);

@@ -170,6 +170,82 @@ __device__ __forceinline__ void flush_segment(double (&red)[NV], double* partial
     for (int k = 0; k < NV; ++k) red[k] = 0.0;
 }
 
+// The next window at or after wi that holds tile t (a CTA's tiles ascend).
+__device__ __forceinline__ int advance_window(const psc_window* wins, int nwin, int wi, int64_t t) {
+    while (wi + 1 < nwin && t >= wins[wi].tile_begin + wins[wi].tile_count) ++wi;
+    return wi;
+}
+
+// How the tiles of a launch fall to its CTAs: CTA c has the share [start(c), start(c + 1)) of the
+// tiles, groups of 2^lg consecutive CTAs pool their shares, and the CTAs of a group take the group's
+// tiles in turn.
+//
+// In turn, a group's CTAs read and write each population plane in one moving front (DRAM pages stay
+// open: 200^3 FP32 step 213 -> 197 us with one group; exact 160^3 with sums 292 -> 270 us); with a run
+// of its own, a CTA enters fewer windows.  So one window is one group, and a batch gets groups in which
+// a CTA takes 32 to 64 tiles per window on average (24 windows, FP32: 871 -> 835 us a step; one group
+// for windows of 24^3 to 40^3 took 31 us instead of 19.5).
+struct TilePlan {
+    uint32_t q, r;  // total tiles = q * grid + r: the first r CTAs have q + 1
+    int32_t lg;
+};
+// (a launch has fewer than 2^31 tiles: as many of 256 cells would hold more than any GPU's memory)
+inline TilePlan tile_plan(int64_t total, int nwin, int grid) {
+    TilePlan p = {(uint32_t)(total / grid), (uint32_t)(total % grid), 0};
+    if (nwin <= 1) {
+        p.lg = 30;  // one group
+        return p;
+    }
+    const int64_t size = total / ((int64_t)nwin * 32);
+    while (p.lg < 30 && ((int64_t)2 << p.lg) <= size) ++p.lg;
+    return p;
+}
+
+struct TileWalk {
+    uint32_t begin, end;  // the group's tiles
+    uint32_t c0, size;    // its first CTA, its CTAs
+    // this CTA's first tile; its next ones are `size` further on
+    __device__ __forceinline__ uint32_t first() const { return begin + (blockIdx.x - c0); }
+};
+__device__ __forceinline__ uint32_t tile_start(const TilePlan& p, uint32_t c) { return p.q * c + min(c, p.r); }
+__device__ __forceinline__ TileWalk group_walk(const TilePlan& p, uint32_t c) {  // the group of CTA c
+    TileWalk w;
+    w.c0 = (c >> p.lg) << p.lg;
+    const uint32_t c1 = min(w.c0 + (1u << p.lg), gridDim.x);
+    w.size = c1 - w.c0;
+    w.begin = tile_start(p, w.c0);
+    w.end = tile_start(p, c1);
+    return w;
+}
+__device__ __forceinline__ TileWalk tile_walk(const TilePlan& p) { return group_walk(p, blockIdx.x); }
+__device__ __forceinline__ TileWalk walk_of_tile(const TilePlan& p, uint32_t t) {
+    const uint32_t wide = p.r * (p.q + 1);
+    return group_walk(p, t < wide ? t / (p.q + 1) : p.r + (t - wide) / p.q);
+}
+
+// End of this CTA's tiles inside the window [tb, te), the first of them t_in: each warp writes the sums
+// of its threads as one row of the window's partials (after the header row), the rows of a group's CTAs
+// in the order in which they enter the window, group after group; the owner of the window's first tile
+// writes the row count into the header.
+template <int NV>
+__device__ __forceinline__ void flush_walk(double (&red)[NV], double* partials, uint32_t tb, uint32_t te, uint32_t t_in,
+                                           const TileWalk& w, const TilePlan& p) {
+    uint32_t row = t_in - max(tb, w.begin);
+    if (tb < w.begin) {  // the window began in an earlier group: that group's rows and those between
+        const TileWalk a = walk_of_tile(p, tb);
+        row += min(a.size, a.end - tb) + (w.c0 - (a.c0 + a.size));
+    }
+    warp_reduce_store<NV>(red, partials + (1 + (int64_t)row * PSC_PARTIAL_ROWS) * NV);
+    if (row == 0 && threadIdx.x == 0) {
+        uint32_t rows = min(w.size, min(te, w.end) - tb);
+        if (te > w.end) {
+            const TileWalk b = walk_of_tile(p, te - 1);
+            rows += (b.c0 - (w.c0 + w.size)) + min(b.size, te - b.begin);
+        }
+        partials[0] = (double)((int64_t)rows * PSC_PARTIAL_ROWS);
+    }
+}
+
 template <int NV>
 __device__ __forceinline__ void block_reduce_store(double (&v)[NV], double (*s_red)[NV], double* out) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

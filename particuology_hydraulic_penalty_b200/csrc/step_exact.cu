@@ -8,7 +8,7 @@
 //   write     f*_i(x) to the other buffer, optional IMB momentum   (:234-236)
 //   reduce    FP64 partial sums (flux, porosity, IMB, NaN count)
 //
-// Each persistent CTA owns a contiguous run of 256-cell tiles; a thread owns
+// Each persistent CTA takes its share of the 256-cell tiles (TilePlan); a thread owns
 // one cell of a tile, so every population plane is read and written with
 // consecutive addresses and crosses HBM once per step.  The window's constants
 // sit in shared memory, built when the CTA enters the window.
@@ -28,14 +28,15 @@ struct ExactShared {
     double* partials;
     int64_t tile_begin, tile_end;
     uint32_t nx, ny, nz, N;
-    uint32_t tstep_x, tstep_y, tstep_z;  // tile_cells cells as a mixed-radix (x, y, z) increment
+    uint32_t tstep_x, tstep_y, tstep_z;  // a CTA's next tile (tile_cells * stride cells on) as (x, y, z) digits
     int32_t tile_cells;
     int32_t moving, inactive, open_x;
     ExactWin c;
     double corr[Q];  // open_x: bounce-back inlet term 2 w_i rho_in (c_i . u_in) / cs^2
 };
 
-__device__ void load_exact_win(ExactShared& s, const psc_window& W, bool moving_launch) {
+// stride: tiles from one of the CTA's tiles to its next.
+__device__ void load_exact_win(ExactShared& s, const psc_window& W, bool moving_launch, int32_t stride) {
     if (threadIdx.x == 0) {
         s.src = reinterpret_cast<const double*>(W.f_src);
         s.dst = reinterpret_cast<double*>(W.f_dst);
@@ -50,9 +51,9 @@ __device__ void load_exact_win(ExactShared& s, const psc_window& W, bool moving_
         s.ny = W.ny;
         s.nz = W.nz;
         s.N = (uint32_t)W.nx * W.ny * W.nz;
-        const uint32_t tc = (uint32_t)W.tile_cells;
-        const uint32_t tq = tc / (uint32_t)W.nz;
-        s.tstep_z = tc % (uint32_t)W.nz;
+        const uint64_t tc = (uint64_t)W.tile_cells * stride;
+        const uint32_t tq = tc < s.N ? (uint32_t)tc / (uint32_t)W.nz : 0u;  // (a longer step leaves the window)
+        s.tstep_z = tc < s.N ? (uint32_t)tc % (uint32_t)W.nz : 0u;
         s.tstep_y = tq % (uint32_t)W.ny;
         s.tstep_x = tq / (uint32_t)W.ny;
         s.tile_cells = W.tile_cells;
@@ -143,42 +144,44 @@ __device__ __noinline__ void exact_cell_general(const ExactShared& s, uint32_t c
 // Two CTAs per SM (128 registers; three at 80 registers spill).  Bounds, on a 160^3 window: HBM
 // (312 B/cell, 196 us at the measured copy rate) and the FP64 pipe (one warp instruction every other
 // cycle and SM quarter, about 575 per cell: 130 us).  Measured with branch-free divisions, one window
-// set-up per CTA run and range tests in integer instructions: 232 us plain, 268 with IMB and sums (553
-// and 608 with a branch per division and a window look-up per tile); 96^3: 56 and 62 (126 and 137);
-// 24^3: 4.7 and 6.2 (8.9 and 9.8).  Staging the next tile's populations in shared memory by cp.async
-// took another 1 to 4 %, at one more kernel per variant: not used.
+// set-up per CTA and window, and range tests in integer instructions: 232 us plain, 270 to 282 with IMB
+// and sums (553 and 608 with a branch per division and a window look-up per tile); 96^3: 56 and 62 (126
+// and 137); 24^3: 4.7 and 6.1 (8.9 and 9.8).  Staging the next tile's populations in shared memory by
+// cp.async took another 1 to 4 %, at one more kernel per variant: not used.
 template <bool MOVING, bool RED>
-__global__ void __launch_bounds__(STEP_THREADS, 2) k_step_exact(const psc_window* __restrict__ wins, int nwin,
-                                                                int64_t total_tiles, unsigned flags) {
+__global__ void __launch_bounds__(STEP_THREADS, 2)
+    k_step_exact(const psc_window* __restrict__ wins, int nwin, unsigned flags, const __grid_constant__ TilePlan plan) {
     __shared__ ExactShared sw;
     __shared__ double s_red[RED ? PSC_NRED : 1][STEP_THREADS];  // running sums per thread (in registers they would spill)
     static_assert(STEP_THREADS / 32 == PSC_PARTIAL_ROWS, "one partial row per warp");
     const bool do_collide = flags & PSC_STEP_COLLIDE;
     const bool do_imb = do_collide && (flags & PSC_STEP_IMB);
     const bool do_mom = flags & PSC_STEP_MOMENTS;
-    const int64_t t0 = (total_tiles * (int64_t)blockIdx.x) / gridDim.x;
-    const int64_t t1 = (total_tiles * ((int64_t)blockIdx.x + 1)) / gridDim.x;
-    int64_t win_end = -1;
+    const TileWalk walk = tile_walk(plan);
+    uint32_t win_end = 0, t_in = 0;  // the window's end, the CTA's first tile in it
+    int wi = -1;
     bool have = false;  // block-uniform: s_red holds cells of the window in sw
     ExactAt at = {0, 0, 0};
     auto flush = [&]() {
         double red[PSC_NRED];
 #pragma unroll
         for (int q = 0; q < PSC_NRED; ++q) red[q] = s_red[RED ? q : 0][threadIdx.x];
-        flush_segment<PSC_NRED>(red, sw.partials, sw.tile_begin, sw.tile_end - sw.tile_begin, total_tiles, gridDim.x);
+        flush_walk<PSC_NRED>(red, sw.partials, (uint32_t)sw.tile_begin, (uint32_t)sw.tile_end, t_in, walk, plan);
     };
-    for (int64_t t = t0; t < t1; ++t) {
+    for (uint32_t t = walk.first(); t < walk.end; t += walk.size) {
         if (t >= win_end) {  // block-uniform: entering a new window
             if (RED && have) flush();
             have = false;
             __syncthreads();
-            load_exact_win(sw, wins[find_window(wins, nullptr, nwin, t)], MOVING);
+            wi = wi < 0 ? find_window(wins, nullptr, nwin, t) : advance_window(wins, nwin, wi, t);
+            load_exact_win(sw, wins[wi], MOVING, (int32_t)walk.size);
             if (RED) {
 #pragma unroll
                 for (int q = 0; q < (RED ? PSC_NRED : 1); ++q) s_red[q][threadIdx.x] = 0.0;
             }
             __syncthreads();
-            win_end = sw.tile_end;
+            win_end = (uint32_t)sw.tile_end;
+            t_in = t;
             at = exact_decode(sw, (uint32_t)((t - sw.tile_begin) * sw.tile_cells) + threadIdx.x);
         }
         if (sw.inactive) continue;  // block-uniform
@@ -289,7 +292,8 @@ static cudaError_t launch_exact_t(const psc_window* d_windows, int nwin, int64_t
     }
     if ((int64_t)grid_ctas > total_tiles) grid_ctas = (int)total_tiles;  // every CTA owns >= 1 tile
     if (grid_ctas <= 0) return cudaSuccess;
-    k_step_exact<MOVING, RED><<<grid_ctas, STEP_THREADS, 0, stream>>>(d_windows, nwin, total_tiles, flags);
+    k_step_exact<MOVING, RED><<<grid_ctas, STEP_THREADS, 0, stream>>>(
+        d_windows, nwin, flags, tile_plan(total_tiles, nwin, grid_ctas));
     return cudaGetLastError();
 }
 

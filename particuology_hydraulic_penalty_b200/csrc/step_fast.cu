@@ -2,7 +2,7 @@
 //
 // The step of psc_step_windows (pull-stream + PSC-IMB collide, src/lbm_dem/psc3d.py:
 // 208-246), organised to keep the SM's issue slots for the collision:
-//  * each persistent CTA owns a CONTIGUOUS run of tiles, so it meets a new
+//  * each persistent CTA takes its share of the tiles (TilePlan) and meets a new
 //    window only a few times; per-window constants (Guo terms, 1/tau, the
 //    solid-level -> B and (1-B)/tau tables, mixed-radix tile stride) are built
 //    once in shared memory when the window changes;
@@ -26,8 +26,8 @@ struct StepOccupancy {
 };
 
 template <int STORE, bool MOVING, int CPT, bool RED>
-__global__ void __launch_bounds__(STEP_THREADS, (StepOccupancy<STORE, MOVING, RED>::value)) k_step_fast(const psc_window* __restrict__ wins, int nwin,
-                                                             int64_t total_tiles, unsigned flags) {
+__global__ void __launch_bounds__(STEP_THREADS, (StepOccupancy<STORE, MOVING, RED>::value))
+    k_step_fast(const psc_window* __restrict__ wins, int nwin, unsigned flags, const __grid_constant__ TilePlan plan) {
     using TR = StoreTraits<STORE>;
     using T = typename TR::T;
     using R = typename TR::R;
@@ -38,9 +38,9 @@ __global__ void __launch_bounds__(STEP_THREADS, (StepOccupancy<STORE, MOVING, RE
     const bool do_imb = do_collide && (flags & PSC_STEP_IMB);
     const bool do_mom = flags & PSC_STEP_MOMENTS;
     constexpr bool do_red = RED;
-    const int64_t t0 = (total_tiles * (int64_t)blockIdx.x) / gridDim.x;
-    const int64_t t1 = (total_tiles * ((int64_t)blockIdx.x + 1)) / gridDim.x;
-    int64_t win_end = -1;
+    const TileWalk walk = tile_walk(plan);
+    uint32_t win_end = 0, t_in = 0;  // the window's end, the CTA's first tile in it
+    int wi = -1, prev = -1;
     // FP64: two CTAs' registers do not hold the sums too (160^3 with IMB: 247 us against 260); FP32 runs as
     // fast either way at 97^3 and slower at 49^3 (10.5 against 9.3 us)
     constexpr bool SHARED = RED && STORE == PSC_STORE_F64;
@@ -52,19 +52,21 @@ __global__ void __launch_bounds__(STEP_THREADS, (StepOccupancy<STORE, MOVING, RE
         double v[PSC_NRED];
 #pragma unroll
         for (int q = 0; q < PSC_NRED; ++q) v[q] = red.at(q);
-        flush_segment<PSC_NRED>(v, sw.partials, sw.tile_begin, sw.tile_end - sw.tile_begin, total_tiles, gridDim.x);
+        flush_walk<PSC_NRED>(v, sw.partials, (uint32_t)sw.tile_begin, (uint32_t)sw.tile_end, t_in, walk, plan);
         red.clear();
     };
     bool have = false;  // block-uniform: red holds cells of the window in sw
-    for (int64_t t = t0; t < t1; ++t) {
+    for (uint32_t t = walk.first(); t < walk.end; t += walk.size) {
         if (t >= win_end) {  // block-uniform: entering a new window
             if (do_red && have) flush();
             have = false;
             __syncthreads();
-            const int wi = find_window(wins, nullptr, nwin, t);
-            load_fast_win(sw, wins[wi], MOVING);
+            wi = wi < 0 ? find_window(wins, nullptr, nwin, t) : advance_window(wins, nwin, wi, t);
+            load_fast_win(sw, wins[wi], MOVING, (int32_t)walk.size, prev >= 0 ? wins + prev : nullptr);
+            prev = wi;
             __syncthreads();
-            win_end = sw.tile_end;
+            win_end = (uint32_t)sw.tile_end;
+            t_in = t;
         }
         if (sw.inactive) continue;  // block-uniform
         have = true;
@@ -162,7 +164,8 @@ static cudaError_t launch_fast_t(const psc_window* d_windows, int nwin, int64_t 
     }
     if ((int64_t)grid_ctas > total_tiles) grid_ctas = (int)total_tiles;  // every CTA owns >= 1 tile
     if (grid_ctas <= 0) return cudaSuccess;
-    k_step_fast<STORE, MOVING, CPT, RED><<<grid_ctas, STEP_THREADS, 0, stream>>>(d_windows, nwin, total_tiles, flags);
+    k_step_fast<STORE, MOVING, CPT, RED><<<grid_ctas, STEP_THREADS, 0, stream>>>(
+        d_windows, nwin, flags, tile_plan(total_tiles, nwin, grid_ctas));
     return cudaGetLastError();
 }
 

@@ -66,7 +66,7 @@ struct PairOccupancy {
 
 template <int STORE, bool MOVING, bool RED>
 __global__ void __launch_bounds__(STEP_THREADS, (PairOccupancy<STORE, MOVING, RED>::value))
-    k_step_pair(const psc_window* __restrict__ wins, int nwin, int64_t total_tiles, unsigned flags) {
+    k_step_pair(const psc_window* __restrict__ wins, int nwin, unsigned flags, const __grid_constant__ TilePlan plan) {
     using TR = StoreTraits<STORE>;
     using T = typename TR::T;
     using R = typename TR::R;
@@ -83,9 +83,9 @@ __global__ void __launch_bounds__(STEP_THREADS, (PairOccupancy<STORE, MOVING, RE
     const bool do_imb = do_collide && (flags & PSC_STEP_IMB);
     const bool do_mom = flags & PSC_STEP_MOMENTS;
     constexpr bool do_red = RED;
-    const int64_t t0 = (total_tiles * (int64_t)blockIdx.x) / gridDim.x;
-    const int64_t t1 = (total_tiles * ((int64_t)blockIdx.x + 1)) / gridDim.x;
-    int64_t win_end = -1;
+    const TileWalk walk = tile_walk(plan);
+    uint32_t win_end = 0, t_in = 0;  // the window's end, the CTA's first tile in it
+    int wi = -1, prev = -1;
     constexpr bool SHARED = RED && PACKED;  // (107 -> 104 us with the sums in registers, 99 in shared memory)
     __shared__ double s_red[SHARED ? PSC_NRED : 1][STEP_THREADS];
     CellSums<SHARED> red;  // this thread's sums over the CTA's cells of the current window
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(STEP_THREADS, (PairOccupancy<STORE, MOVING, RE
         double v[PSC_NRED];
 #pragma unroll
         for (int q = 0; q < PSC_NRED; ++q) v[q] = red.at(q);
-        flush_segment<PSC_NRED>(v, sw.partials, sw.tile_begin, sw.tile_end - sw.tile_begin, total_tiles, gridDim.x);
+        flush_walk<PSC_NRED>(v, sw.partials, (uint32_t)sw.tile_begin, (uint32_t)sw.tile_end, t_in, walk, plan);
         red.clear();
     };
     bool have = false;
@@ -104,15 +104,17 @@ __global__ void __launch_bounds__(STEP_THREADS, (PairOccupancy<STORE, MOVING, RE
     // window, then advanced tile by tile (consecutive tiles, tile_cells apart) by a carry-add
     bool fresh = true;
     uint32_t ix = 0, iy = 0, iz = 0;
-    for (int64_t t = t0; t < t1; ++t) {
+    for (uint32_t t = walk.first(); t < walk.end; t += walk.size) {
         if (t >= win_end) {  // block-uniform: entering a new window
             if (do_red && have) flush();
             have = false;
             __syncthreads();
-            const int wi = find_window(wins, nullptr, nwin, t);
-            load_fast_win(sw, wins[wi], MOVING);
+            wi = wi < 0 ? find_window(wins, nullptr, nwin, t) : advance_window(wins, nwin, wi, t);
+            load_fast_win(sw, wins[wi], MOVING, (int32_t)walk.size, prev >= 0 ? wins + prev : nullptr);
+            prev = wi;
             __syncthreads();
-            win_end = sw.tile_end;
+            win_end = (uint32_t)sw.tile_end;
+            t_in = t;
             skip = (sw.nz & 1u) != 0 || sw.tile_cells != PAIR_CELLS * (int32_t)blockDim.x;
             fresh = true;
             if (skip && threadIdx.x == 0) atomicCAS(&g_pair_status, 0, (sw.nz & 1u) ? 0x201 : 0x202);
@@ -127,7 +129,7 @@ __global__ void __launch_bounds__(STEP_THREADS, (PairOccupancy<STORE, MOVING, RE
             iy = rr % ny;
             ix = rr / ny;
             fresh = false;
-        } else {  // one tile on: += the tile step, single carries (each step component < its extent)
+        } else {  // this CTA's next tile: += its step, single carries (each step component < its extent)
             iz += sw.tstep_z;
             const uint32_t cz = iz >= nz;
             iz -= cz ? nz : 0u;
@@ -240,7 +242,8 @@ static cudaError_t launch_pair_t(const psc_window* d_windows, int nwin, int64_t 
     }
     if ((int64_t)grid_ctas > total_tiles) grid_ctas = (int)total_tiles;  // every CTA owns >= 1 tile
     if (grid_ctas <= 0) return cudaSuccess;
-    k_step_pair<STORE, MOVING, RED><<<grid_ctas, STEP_THREADS, 0, stream>>>(d_windows, nwin, total_tiles, flags);
+    k_step_pair<STORE, MOVING, RED><<<grid_ctas, STEP_THREADS, 0, stream>>>(
+        d_windows, nwin, flags, tile_plan(total_tiles, nwin, grid_ctas));
     return cudaGetLastError();
 }
 
