@@ -15,8 +15,12 @@
 //   dK/dB(x)        += lambda_{t+1}(x) . dC/dB(f_t(x))
 // Each reverse step reads S_t (pulled) and lambda_{t+1}, writes lambda_t and
 // updates one FP64 accumulator per cell: ~1.6x the bytes of a forward step.
+#include <cooperative_groups.h>
+
 #include "collide.cuh"
 #include "internal.cuh"
+#include "smooth.cuh"
+#include "step_common.cuh"
 
 namespace psc {
 
@@ -124,14 +128,140 @@ __global__ void k_adjoint_seed(psc_adjoint_args a) {
     }
 }
 
+// J_C(f)^T lambda of one cell (or two in packed FP32), by hand.  g: the pulled deviations; lam: lambda_{t+1}
+// on entry, mu on exit; returns dC/dB . lambda.  Per direction pair with L = l_i + l_j, D = l_i - l_j:
+//   the sensitivities to feq_i +- feq_j are P = (kb - B) L and M = (kb + B) D, so with
+//   x = 4.5 cu P and y = 3 M
+//     d/d(rho - 1) += w cu (x + y)          (and kb sum w L - 1.5 u^2 (kb - B) sum w L once)
+//     d/du         += c (w rho (2 x + y) + 9 pref w (c . F) L)
+//   (and u by - sum w L (3 rho (kb - B) u + 3 pref F) once), and
+//     dC/dB . lambda += L ((gs/2 - sym)/tau - w rho q) + D ((gd/2 - asym)/tau - gd + asym),
+//   gs = g_i + g_j, gd = g_i - g_j, feq = sym +- asym, sym = w (drho + rho q), q = 4.5 cu^2 - 1.5 u^2;
+//   mu_i = (1 - kb - B) l_i + B l_j + d/d(rho - 1) + c . d/dm.
+template <typename V>
+struct AdjointConst {
+    V inv_tau, fx, fy, fz, pref3;  // pref3 = 3 pref
+    V K9[9];                       // 9 pref w_k (c_k . F)
+};
+
+template <typename V>
+__device__ __forceinline__ void make_adjoint_const(AdjointConst<V>& c, const psc_adjoint_args& a) {
+    const double pref = 1.0 - 0.5 / a.tau;
+    c.inv_tau = lift<V>(1.0 / a.tau);
+    c.fx = lift<V>(a.force[0]);
+    c.fy = lift<V>(a.force[1]);
+    c.fz = lift<V>(a.force[2]);
+    c.pref3 = lift<V>(3.0 * pref);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        const int i = 2 * k + 1;
+        c.K9[k] = lift<V>(9.0 * pref * wgt(i) * (cxv(i) * a.force[0] + cyv(i) * a.force[1] + czv(i) * a.force[2]));
+    }
+}
+
+template <typename V>
+struct AdjointTerms {
+    V ux, uy, uz, uu15, rho, drho, kmB, kpB3;  // kb - B, 3 (kb + B)
+    V Vx, Vy, Vz, E, dB, Lw;
+};
+
+template <int K, typename V>
+__device__ __forceinline__ void adjoint_pair(const V* g, const V* lam, const AdjointConst<V>& c, AdjointTerms<V>& p) {
+    constexpr int i = 2 * K + 1, j = i + 1;
+    const V w = lift<V>(wgt(i)), wr = vmul(w, p.rho);
+    const V L = vadd(lam[i], lam[j]), D = vsub(lam[i], lam[j]);
+    const V cu = cdot_v<K>(p.ux, p.uy, p.uz), c45 = vmul(lift<V>(4.5), cu);
+    const V x = vmul(c45, vmul(p.kmB, L)), y = vmul(p.kpB3, D);
+    p.E = vfma(vmul(w, cu), vadd(x, y), p.E);
+    const V vc = vfma(wr, vfma(lift<V>(2.0), x, y), vmul(c.K9[K], L));
+    if constexpr (cxv(i) != 0) p.Vx = K == 0 ? vc : vadd(p.Vx, vc);
+    if constexpr (cyv(i) != 0) p.Vy = K == 1 ? vc : (cyv(i) > 0 ? vadd(p.Vy, vc) : vsub(p.Vy, vc));
+    if constexpr (czv(i) != 0) p.Vz = K == 2 ? vc : (czv(i) > 0 ? vadd(p.Vz, vc) : vsub(p.Vz, vc));
+    p.Lw = vfma(w, L, p.Lw);
+    const V rq = vmul(p.rho, vsub(vmul(c45, cu), p.uu15));
+    const V sym = vmul(w, vadd(p.drho, rq)), asym = vmul(lift<V>(3.0), vmul(wr, cu));
+    const V half = lift<V>(0.5), gd = vsub(g[i], g[j]);
+    const V es = vsub(vmul(half, vadd(g[i], g[j])), sym), ea = vsub(vmul(half, gd), asym);
+    p.dB = vfma(L, vsub(vmul(es, c.inv_tau), vmul(w, rq)), p.dB);
+    p.dB = vfma(D, vadd(vmul(ea, c.inv_tau), vsub(asym, gd)), p.dB);
+}
+
+template <int K, typename V>
+__device__ __forceinline__ void adjoint_mu(V* lam, V direct, V B, V rb, V mx, V my, V mz) {
+    constexpr int i = 2 * K + 1, j = i + 1;
+    const V cm = cdot_v<K>(mx, my, mz), li = lam[i], lj = lam[j];
+    lam[i] = vfma(direct, li, vfma(B, lj, vadd(rb, cm)));
+    lam[j] = vfma(direct, lj, vfma(B, li, vsub(rb, cm)));
+}
+
+template <typename V>
+__device__ __forceinline__ V adjoint_cell(const V* g, V* lam, V B, V irho, V drho, const AdjointConst<V>& c) {
+    const V one = lift<V>(1.0);
+    AdjointTerms<V> p;
+    p.drho = drho;
+    p.rho = vadd(one, drho);
+    V mx, my, mz;
+    momentum(g, mx, my, mz);
+    p.ux = vmul(vadd(mx, c.fx), irho);
+    p.uy = vmul(vadd(my, c.fy), irho);
+    p.uz = vmul(vadd(mz, c.fz), irho);
+    p.uu15 = vmul(lift<V>(1.5), vfma(p.uz, p.uz, vfma(p.uy, p.uy, vmul(p.ux, p.ux))));
+    const V kb = vmul(vsub(one, B), c.inv_tau);
+    p.kmB = vsub(kb, B);
+    p.kpB3 = vmul(lift<V>(3.0), vadd(kb, B));
+    // rest population: cu = 0
+    const V w0 = lift<V>(W0), l0 = lam[0];
+    const V rq0 = vmul(p.rho, p.uu15), geq0 = vmul(w0, vsub(drho, rq0));
+    p.dB = vmul(l0, vfma(vsub(g[0], geq0), c.inv_tau, vmul(w0, rq0)));
+    p.E = lift<V>(0.0);
+    p.Lw = vmul(w0, l0);
+    adjoint_pair<0>(g, lam, c, p);
+    adjoint_pair<1>(g, lam, c, p);
+    adjoint_pair<2>(g, lam, c, p);
+    adjoint_pair<3>(g, lam, c, p);
+    adjoint_pair<4>(g, lam, c, p);
+    adjoint_pair<5>(g, lam, c, p);
+    adjoint_pair<6>(g, lam, c, p);
+    adjoint_pair<7>(g, lam, c, p);
+    adjoint_pair<8>(g, lam, c, p);
+    const V PL = vmul(p.kmB, p.Lw);  // sum of w P
+    const V s1 = vmul(vmul(lift<V>(3.0), p.rho), PL), s2 = vmul(c.pref3, p.Lw);
+    const V ubx = vsub(vsub(p.Vx, vmul(s1, p.ux)), vmul(s2, c.fx));
+    const V uby = vsub(vsub(p.Vy, vmul(s1, p.uy)), vmul(s2, c.fy));
+    const V ubz = vsub(vsub(p.Vz, vmul(s1, p.uz)), vmul(s2, c.fz));
+    V rb = vadd(vsub(vmul(kb, p.Lw), vmul(p.uu15, PL)), p.E);
+    rb = vsub(rb, vmul(vfma(ubz, p.uz, vfma(uby, p.uy, vmul(ubx, p.ux))), irho));
+    const V mbx = vmul(ubx, irho), mby = vmul(uby, irho), mbz = vmul(ubz, irho);
+    const V direct = vsub(vsub(one, kb), B);
+    lam[0] = vfma(vsub(one, kb), l0, rb);
+    adjoint_mu<0>(lam, direct, B, rb, mbx, mby, mbz);
+    adjoint_mu<1>(lam, direct, B, rb, mbx, mby, mbz);
+    adjoint_mu<2>(lam, direct, B, rb, mbx, mby, mbz);
+    adjoint_mu<3>(lam, direct, B, rb, mbx, mby, mbz);
+    adjoint_mu<4>(lam, direct, B, rb, mbx, mby, mbz);
+    adjoint_mu<5>(lam, direct, B, rb, mbx, mby, mbz);
+    adjoint_mu<6>(lam, direct, B, rb, mbx, mby, mbz);
+    adjoint_mu<7>(lam, direct, B, rb, mbx, mby, mbz);
+    adjoint_mu<8>(lam, direct, B, rb, mbx, mby, mbz);
+    return p.dB;
+}
+
 template <typename R>
-__global__ void __launch_bounds__(256) k_adjoint_step(psc_adjoint_args a) {
+__device__ __forceinline__ R adjoint_B(double solid, R tau) {
+    const R al = (R)solid;
+    return al / (al + tau * (R(1) - al) + R(1.0e-14));
+}
+
+// One cell per thread.
+template <typename R>
+__global__ void __launch_bounds__(256) k_adjoint_step(const __grid_constant__ psc_adjoint_args a) {
+    __shared__ AdjointConst<R> c;
+    if (threadIdx.x == 0) make_adjoint_const(c, a);
+    __syncthreads();
     const uint32_t N = (uint32_t)a.nx * a.ny * a.nz;
     const R* S = reinterpret_cast<const R*>(a.state);
     const R* lin = reinterpret_cast<const R*>(a.lam_in);
     R* lout = reinterpret_cast<R*>(a.lam_out);
-    const R tau = (R)a.tau, inv_tau = R(1) / tau, pref = R(1) - R(0.5) / tau;
-    const R Fx = (R)a.force[0], Fy = (R)a.force[1], Fz = (R)a.force[2];
     const uint32_t stride = gridDim.x * blockDim.x;
     StrideWalk at(blockIdx.x * blockDim.x + threadIdx.x, stride, a.nx, a.ny, a.nz);
     for (uint32_t cell = blockIdx.x * blockDim.x + threadIdx.x; cell < N; cell += stride, at.next()) {
@@ -140,82 +270,109 @@ __global__ void __launch_bounds__(256) k_adjoint_step(psc_adjoint_args a) {
         R g[Q], lam[Q];
 #pragma unroll
         for (int i = 0; i < Q; ++i) {
-            g[i] = S[(size_t)i * N + (size_t)((int64_t)cell + off[i])];
-            lam[i] = lin[(size_t)i * N + cell];
+            g[i] = ld_pop(S + (size_t)i * N + (size_t)((int64_t)cell + off[i]));
+            lam[i] = ld_pop(lin + (size_t)i * N + cell);
         }
-        const R al = (R)a.solid[cell];
-        const R B = al / (al + tau * (R(1) - al) + R(1.0e-14));
-        const FastMoments<R> mo = moments_fast(g);
-        const R rho = mo.rho, drho = mo.drho, irho = R(1) / rho;
-        const R uex = (mo.mx + Fx) * irho, uey = (mo.my + Fy) * irho, uez = (mo.mz + Fz) * irho;
-        const R uu = uex * uex + uey * uey + uez * uez;
-        const R kb = (R(1) - B) * inv_tau;
-        const R direct = R(1) - kb - B;
-        R mu[Q];
-        R dB = R(0), drho_bar = R(0), s1 = R(0), s2 = R(0);
-        R Vx = R(0), Vy = R(0), Vz = R(0);
-        {  // rest population
-            const R w = R(W0);
-            const R geq = w * (drho - R(1.5) * rho * uu);
-            const R os = w * drho - geq;
-            dB += lam[0] * ((g[0] - geq) * inv_tau + os);
-            const R a0 = (kb - B) * lam[0];
-            mu[0] = (R(1) - kb) * lam[0];
-            drho_bar += B * w * lam[0] + a0 * w * (R(1) - R(1.5) * uu);
-            s1 += R(3) * w * rho * a0;
-            s2 += R(3) * pref * w * lam[0];
-        }
+        const R drho = sum_populations(g);
+        const R dB = adjoint_cell<R>(g, lam, adjoint_B<R>(a.solid[cell], (R)a.tau), fast_rcp<R>(R(1) + drho), drho, c);
 #pragma unroll
-        for (int k = 0; k < 9; ++k) {
-            const int i = 2 * k + 1, j = i + 1;
-            const R w = R(wgt(i));
-            const R cu = csel(cxv(i), uex) + csel(cyv(i), uey) + csel(czv(i), uez);
-            const R cF = csel(cxv(i), Fx) + csel(cyv(i), Fy) + csel(czv(i), Fz);
-            const R q2 = R(4.5) * cu * cu - R(1.5) * uu;
-            const R sym = w * (drho + rho * q2);
-            const R asym = R(3) * w * rho * cu;
-            const R geq_i = sym + asym, geq_j = sym - asym;
-            const R os_i = g[j] - g[i] + w * drho - geq_j;
-            const R os_j = g[i] - g[j] + w * drho - geq_i;
-            const R li = lam[i], lj = lam[j];
-            dB += li * ((g[i] - geq_i) * inv_tau + os_i) + lj * ((g[j] - geq_j) * inv_tau + os_j);
-            const R ai = kb * li - B * lj, aj = kb * lj - B * li;
-            mu[i] = direct * li + B * lj;
-            mu[j] = direct * lj + B * li;
-            drho_bar += B * w * (li + lj) + w * (ai * (R(1) + R(3) * cu + q2) + aj * (R(1) - R(3) * cu + q2));
-            const R vc = w * rho * (ai * (R(3) + R(9) * cu) - aj * (R(3) - R(9) * cu)) + R(9) * pref * w * cF * (li + lj);
-            Vx += csel(cxv(i), vc);
-            Vy += csel(cyv(i), vc);
-            Vz += csel(czv(i), vc);
-            s1 += R(3) * w * rho * (ai + aj);
-            s2 += R(3) * pref * w * (li + lj);
-        }
-        const R ubx = Vx - s1 * uex - s2 * Fx;
-        const R uby = Vy - s1 * uey - s2 * Fy;
-        const R ubz = Vz - s1 * uez - s2 * Fz;
-        const R mbx = ubx * irho, mby = uby * irho, mbz = ubz * irho;
-        drho_bar -= (ubx * uex + uby * uey + ubz * uez) * irho;
+        for (int i = 0; i < Q; ++i) lout[(size_t)i * N + (size_t)((int64_t)cell + off[i])] = lam[i];
+        a.dKdB[cell] += (double)dB;
+    }
+}
+
+// Two consecutive z cells per thread in packed FP32 (nz even, pointers aligned): the accesses of
+// k_step_pair, half the arithmetic instructions.  Bound by HBM: 252 B per cell, 34 us on 96^3.  Twelve
+// warps per SM at 168 registers: 96^3 48.5 -> 39.8 us, 64^3 14.1 -> 9.6 us (sixteen warps at 128 registers
+// spill: 49 us; eight at 255: 46 us; one cell per thread: 45 us).
+constexpr int ADJ_THREADS = 128, ADJ_CTAS = 3;
+__global__ void __launch_bounds__(ADJ_THREADS, ADJ_CTAS) k_adjoint_pair(const __grid_constant__ psc_adjoint_args a) {
+    __shared__ AdjointConst<F2> c;
+    if (threadIdx.x == 0) make_adjoint_const(c, a);
+    __syncthreads();
+    const uint32_t N = (uint32_t)a.nx * a.ny * a.nz, nz = (uint32_t)a.nz;
+    const float* S = reinterpret_cast<const float*>(a.state);
+    const float* lin = reinterpret_cast<const float*>(a.lam_in);
+    float* lout = reinterpret_cast<float*>(a.lam_out);
+    const float tau = (float)a.tau;
+    const uint32_t stride = 2 * gridDim.x * blockDim.x;
+    uint32_t c0 = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+    StrideWalk at(c0, stride, a.nx, a.ny, a.nz);
+    for (; c0 < N; c0 += stride, at.next()) {
+        const int32_t nyz = a.ny * a.nz;
+        const int32_t xm = at.ix == 0 ? (a.nx - 1) * nyz : -nyz, xp = at.ix + 1 == (uint32_t)a.nx ? -(a.nx - 1) * nyz : nyz;
+        const int32_t ym = at.iy == 0 ? (a.ny - 1) * a.nz : -a.nz;
+        const int32_t yp = at.iy + 1 == (uint32_t)a.ny ? -(a.ny - 1) * a.nz : a.nz;
+        const int32_t zm0 = at.iz == 0 ? (int32_t)nz - 1 : -1;           // c0's z - 1
+        const int32_t zp1 = at.iz + 2 == nz ? 2 - (int32_t)nz : 2;       // c0 + 1's z + 1, from c0
+        F2 g[Q], lam[Q];
 #pragma unroll
         for (int i = 0; i < Q; ++i) {
-            const R v = mu[i] + drho_bar + csel(cxv(i), mbx) + csel(cyv(i), mby) + csel(czv(i), mbz);
-            lout[(size_t)i * N + (size_t)((int64_t)cell + off[i])] = v;
+            const int32_t oxy = (cxv(i) == 1 ? xm : (cxv(i) == -1 ? xp : 0)) + (cyv(i) == 1 ? ym : (cyv(i) == -1 ? yp : 0));
+            const float* p = S + (size_t)i * N + (size_t)((int64_t)c0 + oxy);
+            if (czv(i) == 0) {
+                const float2 v = __ldg(reinterpret_cast<const float2*>(p));
+                g[i] = f2(v.x, v.y);
+            } else if (czv(i) == 1) {
+                g[i] = f2(ld_pop(p + zm0), ld_pop(p));
+            } else {
+                g[i] = f2(ld_pop(p + 1), ld_pop(p + zp1));
+            }
+            const float2 l = __ldg(reinterpret_cast<const float2*>(lin + (size_t)i * N + c0));
+            lam[i] = f2(l.x, l.y);
         }
-        a.dKdB[cell] += (double)dB;
+        const double2 solid = *reinterpret_cast<const double2*>(a.solid + c0);
+        const F2 drho = sum_populations(g);
+        float d0, d1;
+        f2_get(drho, d0, d1);
+        const F2 dB = adjoint_cell<F2>(g, lam, f2(adjoint_B<float>(solid.x, tau), adjoint_B<float>(solid.y, tau)),
+                                       f2(fast_rcp<float>(1.0f + d0), fast_rcp<float>(1.0f + d1)), drho, c);
+#pragma unroll
+        for (int i = 0; i < Q; ++i) {
+            const int32_t oxy = (cxv(i) == 1 ? xm : (cxv(i) == -1 ? xp : 0)) + (cyv(i) == 1 ? ym : (cyv(i) == -1 ? yp : 0));
+            float* p = lout + (size_t)i * N + (size_t)((int64_t)c0 + oxy);
+            float x, y;
+            f2_get(lam[i], x, y);
+            if (czv(i) == 0) {
+                *reinterpret_cast<float2*>(p) = make_float2(x, y);
+            } else if (czv(i) == 1) {
+                p[zm0] = x;
+                p[0] = y;
+            } else {
+                p[1] = x;
+                p[zp1] = y;
+            }
+        }
+        float b0, b1;
+        f2_get(dB, b0, b1);
+        double2 acc = *reinterpret_cast<double2*>(a.dKdB + c0);
+        acc.x += (double)b0;
+        acc.y += (double)b1;
+        *reinterpret_cast<double2*>(a.dKdB + c0) = acc;
     }
 }
 
 // Per-cell dK/d(alpha_sum) = (dK/dB dB/dalpha + dK/dsolid) [0 < alpha_sum < 1], then
 // per-particle sums over bbox entries of dK/dalpha_sum * d alpha_p / d(x, y, z, r).
-constexpr int GRAD_THREADS = 256;
+constexpr int GRAD_THREADS = 128;
+constexpr int GRAD_CTAS = 8;
 
-__global__ void __launch_bounds__(GRAD_THREADS) k_adjoint_geom_chunks(psc_geometry g, psc_adjoint_args a,
-                                                                       double* part) {
+// One cluster per chunk: an entry near a sphere's surface costs S^3 FP64 exponentials, one away from it none,
+// and the chunks differ as much.  64 spheres, S = 4: 33^3 194 -> 80 us and 96^3 478 -> 391 us against a block
+// per chunk (clusters of 256-thread CTAs: 497 us; a tanh for every sample of every entry: 1215 us).  Bound by
+// the exponentials.  The CTAs' sums are added in order.
+template <int S>
+__global__ void __cluster_dims__(GRAD_CTAS, 1, 1) __launch_bounds__(GRAD_THREADS)
+    k_adjoint_geom_chunks(const __grid_constant__ psc_geometry g, const __grid_constant__ psc_adjoint_args a, double* part) {
+    namespace cg = cooperative_groups;
     __shared__ double s[GRAD_THREADS / 32][4];
+    __shared__ double s_cta[4];
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t rank = cluster.block_rank();
     const int64_t C = g.totals[1];
-    const int S = g.subsamples;
-    const double Sd = (double)S, eps = g.smooth_eps, tau = a.tau;
+    const double Sd = (double)g.subsamples, inv_eps = 1.0 / g.smooth_eps, tau = a.tau;
     const double inv_s3 = 1.0 / (Sd * Sd * Sd);
-    for (int64_t chunk = blockIdx.x; chunk < C; chunk += gridDim.x) {
+    for (int64_t chunk = blockIdx.x / GRAD_CTAS; chunk < C; chunk += gridDim.x / GRAD_CTAS) {
         // owner particle of this chunk (largest p with chunk_off[p] <= chunk)
         int lo = 0, hi = g.nparticles - 1;
         while (lo < hi) {
@@ -230,7 +387,7 @@ __global__ void __launch_bounds__(GRAD_THREADS) k_adjoint_geom_chunks(psc_geomet
         const int32_t* bb = g.bbox + (size_t)p * 6;
         const int64_t eyz = (int64_t)bb[4] * bb[5];
         double acc[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int64_t e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
+        for (int64_t e = e0 + rank * GRAD_THREADS + threadIdx.x; e < e1; e += GRAD_CTAS * GRAD_THREADS) {
             const int64_t local = e - g.ent_off[p];
             const int32_t ia = (int32_t)(local / eyz);
             const int64_t rem = local - (int64_t)ia * eyz;
@@ -242,24 +399,8 @@ __global__ void __launch_bounds__(GRAD_THREADS) k_adjoint_geom_chunks(psc_geomet
             if (!(as > 0.0 && as < 1.0)) continue;  // clip: zero derivative outside (0, 1)
             const double D = as + tau * (1.0 - as) + 1.0e-14;
             const double gcell = a.dKdB[cell] * (tau + 1.0e-14) / (D * D) + a.dKdsolid[cell];
-            double gx = 0.0, gy = 0.0, gz = 0.0, gr = 0.0;
-            for (int sa = 0; sa < S; ++sa) {
-                const double dx = ((double)ix + ((double)sa + 0.5) / Sd) - q[0];
-                for (int sb = 0; sb < S; ++sb) {
-                    const double dy = ((double)iy + ((double)sb + 0.5) / Sd) - q[1];
-                    for (int sc = 0; sc < S; ++sc) {
-                        const double dz = ((double)iz + ((double)sc + 0.5) / Sd) - q[2];
-                        const double d = sqrt(dx * dx + dy * dy + dz * dz);
-                        const double sg = 0.5 * (1.0 + tanh(0.5 * (q[3] - d) / eps));
-                        const double ds = sg * (1.0 - sg) / eps;
-                        const double dinv = d > 1.0e-12 ? 1.0 / d : 0.0;
-                        gr += ds;
-                        gx += ds * dx * dinv;
-                        gy += ds * dy * dinv;
-                        gz += ds * dz * dinv;
-                    }
-                }
-            }
+            double gx, gy, gz, gr;
+            smooth_gradient<S>(ix, iy, iz, q[0], q[1], q[2], q[3], g.subsamples, inv_eps, gx, gy, gz, gr);
             const double f = gcell * inv_s3;
             acc[0] += f * gx;
             acc[1] += f * gy;
@@ -278,9 +419,15 @@ __global__ void __launch_bounds__(GRAD_THREADS) k_adjoint_geom_chunks(psc_geomet
         if (threadIdx.x < 4) {
             double t = 0.0;
             for (int w = 0; w < nw; ++w) t += s[w][threadIdx.x];
+            s_cta[threadIdx.x] = t;
+        }
+        cluster.sync();
+        if (rank == 0 && threadIdx.x < 4) {
+            double t = 0.0;
+            for (int r = 0; r < GRAD_CTAS; ++r) t += cluster.map_shared_rank(s_cta, r)[threadIdx.x];
             part[chunk * 4 + threadIdx.x] = t;
         }
-        __syncthreads();
+        cluster.sync();  // s and s_cta stay in place until they are read
     }
 }
 
@@ -310,8 +457,14 @@ cudaError_t launch_adjoint_seed(const psc_adjoint_args& a, cudaStream_t stream) 
 
 cudaError_t launch_adjoint_step(const psc_adjoint_args& a, cudaStream_t stream) {
     const int64_t N = (int64_t)a.nx * a.ny * a.nz;
-    if (a.store == PSC_STORE_F64) k_adjoint_step<double><<<cap_grid(N, 256, 8), 256, 0, stream>>>(a);
-    else k_adjoint_step<float><<<cap_grid(N, 256, 8), 256, 0, stream>>>(a);
+    const auto aligned = [](const void* p, uintptr_t n) { return reinterpret_cast<uintptr_t>(p) % n == 0; };
+    if (a.store == PSC_STORE_F64)
+        k_adjoint_step<double><<<cap_grid(N, 256, 8), 256, 0, stream>>>(a);
+    else if (a.nz % 2 == 0 && aligned(a.state, 8) && aligned(a.lam_in, 8) && aligned(a.lam_out, 8) &&
+             aligned(a.solid, 16) && aligned(a.dKdB, 16))
+        k_adjoint_pair<<<cap_grid(N / 2, ADJ_THREADS, ADJ_CTAS), ADJ_THREADS, 0, stream>>>(a);  // (the resident CTAs)
+    else
+        k_adjoint_step<float><<<cap_grid(N, 256, 8), 256, 0, stream>>>(a);
     return cudaGetLastError();
 }
 
@@ -319,9 +472,9 @@ cudaError_t launch_adjoint_geometry_grad(const psc_geometry& g, const psc_adjoin
                                          double* grad, cudaStream_t stream) {
     if (g.nparticles <= 0) return cudaSuccess;
     if (g.capacity_chunks > 0) {
-        const int64_t cap = (int64_t)sm_count() * 8;
-        const unsigned grid = (unsigned)(g.capacity_chunks < cap ? g.capacity_chunks : cap);
-        k_adjoint_geom_chunks<<<grid, GRAD_THREADS, 0, stream>>>(g, a, part);
+        const int64_t cap = (int64_t)sm_count() * 16;
+        const unsigned grid = GRAD_CTAS * (unsigned)(g.capacity_chunks < cap ? g.capacity_chunks : cap);
+        PSC_BY_SUBSAMPLES(g.subsamples, k_adjoint_geom_chunks, <<<grid, GRAD_THREADS, 0, stream>>>(g, a, part));
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }

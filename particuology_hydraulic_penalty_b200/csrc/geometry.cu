@@ -25,6 +25,7 @@
 
 #include "collide.cuh"
 #include "internal.cuh"
+#include "smooth.cuh"
 
 namespace psc {
 
@@ -158,27 +159,6 @@ __device__ __forceinline__ int sample_count(int32_t ix, int32_t iy, int32_t iz, 
     return cnt;
 }
 
-// Smooth surrogate of sample_count / S^3: every sample contributes
-// sigma((r - d_s) / eps) (logistic via tanh), the differentiable solid
-// fraction used by the adjoint.  Same boxes and sample offsets as the count.
-__device__ __forceinline__ double smooth_alpha(int32_t ix, int32_t iy, int32_t iz, double px, double py, double pz,
-                                               double r, int S, double eps) {
-    const double Sd = (double)S;
-    double acc = 0.0;
-    for (int a = 0; a < S; ++a) {
-        const double dx = ((double)ix + ((double)a + 0.5) / Sd) - px;
-        for (int b = 0; b < S; ++b) {
-            const double dy = ((double)iy + ((double)b + 0.5) / Sd) - py;
-            for (int c = 0; c < S; ++c) {
-                const double dz = ((double)iz + ((double)c + 0.5) / Sd) - pz;
-                const double d = sqrt(dx * dx + dy * dy + dz * dz);
-                acc += 0.5 * (1.0 + tanh(0.5 * (r - d) / eps));
-            }
-        }
-    }
-    return acc / (Sd * Sd * Sd);
-}
-
 // Descriptor of one load-reduction chunk, computed by k_chunk_desc (one
 // thread per chunk, so the lookups of many chunks overlap) into an array that
 // is kept with the geometry, or into the chunk's own partial row (6 doubles):
@@ -210,6 +190,11 @@ __device__ __forceinline__ ChunkDesc make_chunk_desc(const psc_geometry& g, int6
     d.ez = bb[5];
     d.pad = 0;
     return d;
+}
+
+// Chunk c's descriptor: read where the geometry has them, else looked up.
+__device__ __forceinline__ ChunkDesc chunk_desc(const psc_geometry& g, const double* desc, int64_t c) {
+    return desc ? *reinterpret_cast<const ChunkDesc*>(desc + c * 6) : make_chunk_desc(g, c);
 }
 
 // sample_count for a compile-time S: the same IEEE operations on the same
@@ -250,18 +235,26 @@ __device__ __forceinline__ int sample_count_t(int32_t ix, int32_t iy, int32_t iz
 // offsets, one lookup per chunk instead of one per entry); thread t takes the
 // chunk's entries t, t + blockDim.x, ... and steps their bbox-local
 // coordinates by a carry-add.
-template <int S>
-__global__ void __launch_bounds__(256, 2) k_geometry_count(psc_geometry g) {
+// SMOOTH: the smooth solid fraction of the adjoint instead (psc_geometry.smooth_eps > 0).
+// PARTS: blocks per chunk, each with an equal run of its entries (SMOOTH: an entry near a sphere's surface
+// costs S^3 exponentials and one away from it none, so a chunk per block left the GPU waiting for the costly
+// ones: 96^3 with 64 spheres, S = 4, 490 us against 333; with a tanh per sample of every entry 1034 us).
+template <int S, bool SMOOTH, int PARTS>
+__device__ __forceinline__ void geometry_count(const psc_geometry& g, const double* desc) {
     const int64_t E = min(g.totals[0], g.capacity_entries);
     const int64_t C = g.totals[1];
-    const bool smooth = g.smooth_eps > 0.0;
+    const double inv_eps = SMOOTH ? 1.0 / g.smooth_eps : 0.0;
     double o[S > 0 ? S : 1];
 #pragma unroll
     for (int k = 0; k < (S > 0 ? S : 1); ++k) o[k] = xdiv((double)k + 0.5, (double)(S > 0 ? S : 1));  // (k + 0.5) / S
     const uint32_t ny = (uint32_t)g.ny, nz = (uint32_t)g.nz;
-    for (int64_t chunk = blockIdx.x; chunk < C; chunk += gridDim.x) {
-        const ChunkDesc dsc = make_chunk_desc(g, chunk);
-        const int64_t e1 = min(dsc.e1, E);
+    const int64_t run = (g.chunk_entries + PARTS - 1) / PARTS;
+    for (int64_t item = blockIdx.x; item < C * PARTS; item += gridDim.x) {
+        ChunkDesc dsc = chunk_desc(g, desc, item / PARTS);
+        const int64_t shift = (item % PARTS) * run;
+        dsc.e0 += shift;
+        dsc.local0 += (int32_t)shift;
+        const int64_t e1 = min(PARTS > 1 ? min(dsc.e1, dsc.e0 + run) : dsc.e1, E);
         int64_t e = dsc.e0 + threadIdx.x;
         if (e >= e1) continue;
         const double* q = g.particles + (size_t)dsc.p * PF;
@@ -279,8 +272,8 @@ __global__ void __launch_bounds__(256, 2) k_geometry_count(psc_geometry g) {
         for (; e < e1; e += blockDim.x) {
             const int32_t ix = dsc.x0 + (int32_t)a, iy = dsc.y0 + (int32_t)b, iz = dsc.z0 + (int32_t)k;
             int cnt;
-            if (smooth) {
-                const double al = smooth_alpha(ix, iy, iz, px, py, pz, r, g.subsamples, g.smooth_eps);
+            if constexpr (SMOOTH) {
+                const double al = smooth_alpha<S>(ix, iy, iz, px, py, pz, r, g.subsamples, inv_eps);
                 g.ent_alpha[e] = al;
                 cnt = al > 0.0 ? 1 : 0;  // membership of the cell list
             } else if constexpr (S > 0) {
@@ -302,15 +295,25 @@ __global__ void __launch_bounds__(256, 2) k_geometry_count(psc_geometry g) {
     }
 }
 
+template <int S>
+__global__ void __launch_bounds__(256, 2) k_geometry_count(const __grid_constant__ psc_geometry g, const double* desc) {
+    geometry_count<S, false, 1>(g, desc);
+}
+constexpr int SMOOTH_PARTS = 16;
+template <int S>
+__global__ void __launch_bounds__(256, 2) k_geometry_smooth(const __grid_constant__ psc_geometry g, const double* desc) {
+    geometry_count<S, true, SMOOTH_PARTS>(g, desc);
+}
+
 // The cell lists: every entry with a non-zero count appends (particle, count)
 // to its cell's list (the order within a list is fixed by k_geometry_final's
 // sort).  Walks the chunks as k_geometry_count does.
-__global__ void __launch_bounds__(256) k_geometry_fill(psc_geometry g) {
+__global__ void __launch_bounds__(256) k_geometry_fill(const __grid_constant__ psc_geometry g, const double* desc) {
     const int64_t E = min(g.totals[0], g.capacity_entries);
     const int64_t C = g.totals[1];
     const uint32_t ny = (uint32_t)g.ny, nz = (uint32_t)g.nz;
     for (int64_t chunk = blockIdx.x; chunk < C; chunk += gridDim.x) {
-        const ChunkDesc dsc = make_chunk_desc(g, chunk);
+        const ChunkDesc dsc = chunk_desc(g, desc, chunk);
         const int64_t e1 = min(dsc.e1, E);
         int64_t e = dsc.e0 + threadIdx.x;
         if (e >= e1) continue;
@@ -828,8 +831,8 @@ __device__ __forceinline__ void chunk_list_build(const ChunkDesc& dsc, const uin
                                                  uint32_t* labk, int64_t slot_chunk, uint8_t* load_n_chunk) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t ey = (uint32_t)dsc.ey, ez = (uint32_t)dsc.ez, eyz = ey * ez;
-    const int passes = chunk_entries / LOAD_THREADS;
     const int64_t e1 = min(dsc.e1, E);
+    const int passes = e1 > dsc.e0 ? (int)((e1 - dsc.e0 + LOAD_THREADS - 1) / LOAD_THREADS) : 0;
     const uint32_t below = (1u << lane) - 1u;  // lanes before this one
     uint32_t base = 0;                          // non-zero entries of the warp so far
 #pragma unroll 4
@@ -1285,28 +1288,34 @@ cudaError_t launch_geometry_plan(const psc_geometry& g, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_geometry_build(const psc_geometry& g, cudaStream_t stream) {
+cudaError_t launch_chunk_desc(const psc_geometry& g, double* desc, cudaStream_t stream) {
+    const int64_t cap = (int64_t)sm_count() * 16, cg = (g.capacity_chunks + 255) / 256;
+    k_chunk_desc<<<(unsigned)(cg < 1 ? 1 : (cg < cap ? cg : cap)), 256, 0, stream>>>(g, desc);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_geometry_build(const psc_geometry& g, cudaStream_t stream, double* desc) {
     const int64_t N = (int64_t)g.nx * g.ny * g.nz;
     cudaError_t e = cudaMemsetAsync(g.cell_n, 0, (size_t)N * sizeof(int32_t), stream);
     if (e != cudaSuccess) return e;
+    // a block per chunk: most particles own one small chunk (a grid of entries / 4096 blocks took the small
+    // ones in turns: 21 us for the 1136 particles of a 64^3 window)
+    const int64_t full = g.capacity_entries / (g.chunk_entries > 0 ? g.chunk_entries : 4096);
+    const unsigned grid = grid_cap(g.capacity_chunks > full ? g.capacity_chunks : full, 1);
     if (g.capacity_entries > 0) {
-        const unsigned grid = grid_cap(g.capacity_entries, g.chunk_entries > 0 ? g.chunk_entries : 4096);  // ~ one block per chunk
-        switch (g.smooth_eps > 0.0 ? 0 : g.subsamples) {  // the count kernel for a compile-time S
-            case 1: k_geometry_count<1><<<grid, 256, 0, stream>>>(g); break;
-            case 2: k_geometry_count<2><<<grid, 256, 0, stream>>>(g); break;
-            case 3: k_geometry_count<3><<<grid, 256, 0, stream>>>(g); break;
-            case 4: k_geometry_count<4><<<grid, 256, 0, stream>>>(g); break;
-            case 5: k_geometry_count<5><<<grid, 256, 0, stream>>>(g); break;
-            case 6: k_geometry_count<6><<<grid, 256, 0, stream>>>(g); break;
-            default: k_geometry_count<0><<<grid, 256, 0, stream>>>(g); break;
+        if (desc && (e = launch_chunk_desc(g, desc, stream)) != cudaSuccess) return e;
+        if (g.smooth_eps > 0.0) {
+            const unsigned parts = grid_cap(g.capacity_chunks * SMOOTH_PARTS, 1);
+            PSC_BY_SUBSAMPLES(g.subsamples, k_geometry_smooth, <<<parts, 256, 0, stream>>>(g, desc));
+        } else {
+            PSC_BY_SUBSAMPLES(g.subsamples, k_geometry_count, <<<grid, 256, 0, stream>>>(g, desc));
         }
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     if ((e = scan_exclusive_i32(g.cell_n, g.cell_off, N, g.scan_tmp, stream)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(g.cell_n, 0, (size_t)N * sizeof(int32_t), stream)) != cudaSuccess) return e;
     if (g.capacity_entries > 0) {
-        k_geometry_fill<<<grid_cap(g.capacity_entries, g.chunk_entries > 0 ? g.chunk_entries : 4096), 256, 0,
-                          stream>>>(g);
+        k_geometry_fill<<<grid, 256, 0, stream>>>(g, desc);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     k_geometry_final<<<grid_cap(N, 256), 256, 0, stream>>>(g);
@@ -1352,12 +1361,6 @@ static cudaError_t loads_smem_optin() {
         return e;
     done[dev] = 1;
     return cudaSuccess;
-}
-
-cudaError_t launch_chunk_desc(const psc_geometry& g, double* desc, cudaStream_t stream) {
-    const int64_t cap = (int64_t)sm_count() * 16, cg = (g.capacity_chunks + 255) / 256;
-    k_chunk_desc<<<(unsigned)(cg < 1 ? 1 : (cg < cap ? cg : cap)), 256, 0, stream>>>(g, desc);
-    return cudaGetLastError();
 }
 
 cudaError_t launch_particle_loads(const psc_geometry& g, int imb_type, const void* imb, double* chunk_partials,

@@ -64,7 +64,8 @@ cudaError_t launch_stream_pull_store(int store, double scale, const double* src,
                                      cudaStream_t stream, bool open_x = false, const double* inlet = nullptr);
 
 cudaError_t launch_geometry_plan(const psc_geometry& g, cudaStream_t stream);
-cudaError_t launch_geometry_build(const psc_geometry& g, cudaStream_t stream);
+// desc: room for the geometry's load-chunk descriptors (launch_chunk_desc), written here, or null.
+cudaError_t launch_geometry_build(const psc_geometry& g, cudaStream_t stream, double* desc = nullptr);
 cudaError_t launch_solid_velocity(const psc_geometry& g, int us_type, void* us, cudaStream_t stream);
 // desc: the chunk descriptors of this geometry (launch_chunk_desc), or null: made on every call in the
 // chunks' partial rows.  host_diag: page-locked copy of diag, or null.

@@ -554,13 +554,13 @@ int window_rebuild_finish(Window& w, cudaStream_t s, const int64_t* tot4, const 
         }
         w.cap_chunks = cap;
     }
-    psc_geometry g = w.geometry();
-    PSC_TRY(psc_geometry_build(&g, s));
+    const psc_geometry g = w.geometry();
+    PSC_CUDA(launch_geometry_build(g, s, w.cap_chunks > 0 ? w.chunk_desc.p : nullptr), who);
     w.built = true;
     ++w.builds;
     w.built_version = w.pversion;
     w.list_version = 0;
-    w.desc_built = 0;
+    w.desc_built = w.cap_entries > 0 && w.cap_chunks > 0 ? w.built_version : 0;  // (made with the build)
     w.us_version = 0;
     w.loads_ready = false;
     w.diag_ready = false;
@@ -1096,6 +1096,7 @@ int solver_report_step(psc_solver& h) {
         PSC_TRY(report_step_work(h, par, kind));
         h.report_seen[par][kind] = std::move(key);
     }
+    w.loads_enqueued();  // (a replayed graph enqueued them too)
     w.cur ^= 1;
     w.imb_par = w.cur;
     w.stepped = true;
@@ -1472,6 +1473,7 @@ struct psc_batch {
     std::vector<uint64_t> built_desc;  // descriptor versions the tables were built from
     bool moving_any = false;
     Lanes lanes;  // particle loads of the windows beside the post-stream reduction pass
+    Lanes build_lanes;  // geometry rebuilds of the windows beside one another
     HArray<double> up_host;    // every window's particles, staged for one upload
     DArray<double> up_dev;
     // The upload runs on its own stream beside the step kernels, which do not
@@ -1699,9 +1701,26 @@ int batch_prepare(psc_batch& b, bool imb, bool moments) {
     if (!plan.empty()) {
         PSC_TRY(batch_upload_join(b, who));
         PSC_CUDA(b.tot.ensure(4 * (int64_t)b.w.size()), who);
-        for (size_t k : plan) PSC_TRY(window_rebuild_plan(*b.w[k], b.stream, b.tot.p + 4 * k, who));
-        PSC_CUDA(cudaStreamSynchronize(b.stream), who);
-        for (size_t k : plan) PSC_TRY(window_rebuild_finish(*b.w[k], b.stream, b.tot.p + 4 * k, who));
+        // one window's kernels are too small for the GPU: the windows' chains run beside one another, the
+        // solid velocity of a moving window at its end (6 moving windows of 64^3, a
+        // call of two steps: 1.09 ms one after the other, 0.93 ms on four streams)
+        Lanes& lanes = b.build_lanes;
+        PSC_CUDA(lanes.begin(b.stream), who);
+        int st = PSC_OK;
+        for (size_t i = 0; i < plan.size() && st == PSC_OK; ++i)
+            st = window_rebuild_plan(*b.w[plan[i]], lanes.lane((int)i), b.tot.p + 4 * plan[i], who);
+        for (int i = 0; i < lanes.n; ++i) {  // (also after a failure: no lane reads what a later call changes)
+            const cudaError_t e = cudaStreamSynchronize(lanes.s[i]);
+            if (st == PSC_OK && e != cudaSuccess) st = cuda_fail(e, who);
+        }
+        for (size_t i = 0; i < plan.size() && st == PSC_OK; ++i) {
+            Window& w = *b.w[plan[i]];
+            st = window_rebuild_finish(w, lanes.lane((int)i), b.tot.p + 4 * plan[i], who);
+            if (st == PSC_OK && window_needs_solid_velocity(w)) st = window_solid_velocity(w, lanes.lane((int)i));
+        }
+        const cudaError_t e = lanes.end(b.stream);
+        if (st != PSC_OK) return st;
+        PSC_CUDA(e, who);
     }
     for (size_t k = 0; k < b.w.size(); ++k) {
         Window& w = *b.w[k];
@@ -1863,6 +1882,7 @@ int psc_batch_create(const psc_config* h_cfgs, int nwin, const psc_launch* h_lau
         if (e == cudaSuccess) e = b->diag.ensure((int64_t)nwin * PSC_NDIAG, true, b->stream);
         if (e == cudaSuccess) e = b->host.ensure((int64_t)nwin * kOutLen);
         if (e == cudaSuccess) e = b->lanes.init(1);
+        if (e == cudaSuccess) e = b->build_lanes.init(Lanes::kMax);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->up_done, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->up_ready, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->up_stream, cudaStreamNonBlocking);
