@@ -1198,6 +1198,18 @@ __global__ void __cluster_dims__(FINAL_CTAS, 1, 1) __launch_bounds__(FINAL_THREA
 }
 
 // ---------------------------------------------------------------------------
+// results of many windows to the host
+// ---------------------------------------------------------------------------
+struct RowCopies {
+    RowCopy r[kRowCopies];
+};
+// Four CTAs per array, 128-byte stores: bound by the bus.
+__global__ void __launch_bounds__(256) k_copy_rows(const __grid_constant__ RowCopies rows, double* dst) {
+    const RowCopy& r = rows.r[blockIdx.y];
+    for (int64_t k = blockIdx.x * blockDim.x + threadIdx.x; k < r.n; k += gridDim.x * blockDim.x) dst[r.at + k] = r.src[k];
+}
+
+// ---------------------------------------------------------------------------
 // exclusive scan (int32), three passes over blocks of SCAN_ITEMS elements
 // ---------------------------------------------------------------------------
 constexpr int SCAN_THREADS = 256;
@@ -1286,6 +1298,18 @@ static unsigned grid_cap(int64_t work, int threads) {
 cudaError_t launch_geometry_plan(const psc_geometry& g, cudaStream_t stream) {
     k_geometry_plan<<<1, 1024, 0, stream>>>(g);
     return cudaGetLastError();
+}
+
+cudaError_t launch_copy_rows(const RowCopy* rows, int count, double* dst, cudaStream_t stream) {
+    for (int k0 = 0; k0 < count; k0 += kRowCopies) {
+        RowCopies a = {};
+        const int m = count - k0 < kRowCopies ? count - k0 : kRowCopies;
+        for (int k = 0; k < m; ++k) a.r[k] = rows[k0 + k];
+        k_copy_rows<<<dim3(4, (unsigned)m), 256, 0, stream>>>(a, dst);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 cudaError_t launch_chunk_desc(const psc_geometry& g, double* desc, cudaStream_t stream) {

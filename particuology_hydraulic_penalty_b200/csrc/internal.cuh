@@ -75,6 +75,15 @@ cudaError_t launch_particle_loads(const psc_geometry& g, int imb_type, const voi
 // The load-chunk descriptors of one geometry, 6 doubles per chunk.
 cudaError_t launch_chunk_desc(const psc_geometry& g, double* desc, cudaStream_t stream);
 
+// Arrays of doubles to consecutive places of one array (page-locked host memory), in one launch per
+// kRowCopies of them.
+struct RowCopy {
+    const double* src;
+    int64_t at, n;
+};
+constexpr int kRowCopies = 128;
+cudaError_t launch_copy_rows(const RowCopy* rows, int count, double* dst, cudaStream_t stream);
+
 // One window of a many-window particle-loads launch (a device table).
 struct LoadsJob {
     psc_geometry g;

@@ -8,6 +8,7 @@ path: constructing anything here without a CUDA device raises.
 from __future__ import annotations
 
 import ctypes
+import marshal
 import operator
 from dataclasses import dataclass
 
@@ -50,6 +51,7 @@ DEFAULT_STORE_SCALE = {
 Q = 19
 PARTICLE_FIELDS = ("x", "y", "z", "r", "vx", "vy", "vz", "wx", "wy", "wz")
 _particle_row = operator.attrgetter(*PARTICLE_FIELDS)
+_TUPLE_HEAD = np.frombuffer(b"(" + len(PARTICLE_FIELDS).to_bytes(4, "little"), np.uint8)
 
 
 def trt_tau_minus(tau: float, magic: float = 3.0 / 16.0) -> float:
@@ -100,6 +102,30 @@ def stream_handle(device: torch.device | None = None):
     return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
 
 
+def _float_rows(rows: list) -> np.ndarray | None:
+    """(P, 10) array of a list of 10-tuples whose items are all Python floats, else None.
+
+    numpy looks at every item's type twice (1136 rows: 0.40 ms).  marshal writes a float as "g" and its
+    8 bytes and a tuple as "(", its length in 4 bytes and its items, so the rows are records of one size
+    (0.19 ms); any other item changes a tag or the size.
+    """
+    width, n = len(PARTICLE_FIELDS), len(rows)
+    if n == 0 or set(map(type, rows[0])) != {float}:
+        return None
+    try:
+        raw = marshal.dumps(rows, 2)
+    except ValueError:  # an item that marshal has no form for
+        return None
+    size = 5 + 9 * width
+    if len(raw) != 5 + n * size:
+        return None
+    heads = np.ndarray((n, 5), np.uint8, raw, 5, (size, 1))
+    tags = np.ndarray((n, width), np.uint8, raw, 10, (size, 9))
+    if not ((heads == _TUPLE_HEAD).all() and (tags == ord("g")).all()):
+        return None
+    return np.ndarray((n, width), "<f8", raw, 11, (size, 9)).copy()
+
+
 def particles_array(particles) -> np.ndarray:
     """(P, 10) float64 [x, y, z, r, vx, vy, vz, wx, wy, wz] from Particle3D-like objects or an array.
 
@@ -116,7 +142,10 @@ def particles_array(particles) -> np.ndarray:
             raise ValueError("a particle array must have shape (P, 10)")
     else:
         # one attribute tuple per particle (callers mutate Particle3D fields in place between steps)
-        arr = np.array(list(map(_particle_row, particles)), dtype=np.float64).reshape(-1, 10)
+        rows = list(map(_particle_row, particles))
+        arr = _float_rows(rows)
+        if arr is None:
+            arr = np.array(rows, dtype=np.float64).reshape(-1, 10)
     if not np.all(np.isfinite(arr)):
         raise ValueError("particle state contains NaN or Inf")
     return arr
