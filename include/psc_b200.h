@@ -64,6 +64,8 @@ extern "C" {
 #define PSC_STEP_MOMENTS 4u /* write rho, ux, uy, uz of the pulled state */
 #define PSC_STEP_REDUCE 8u  /* write per-tile FP64 reduction partials */
 #define PSC_STEP_MOVING 16u /* some window has PSC_WIN_MOVING: compile in the u_s path */
+#define PSC_STEP_CHAINED 32u /* the kernel before this call on the stream does not write d_windows: the step
+                              * may read it before that kernel has ended */
 
 /* ---- kernel variants of the deviation modes ----------------------------- */
 #define PSC_KERNEL_AUTO 0   /* psc_step_windows_ex: the direct kernel; the handle layer picks the pair
@@ -331,6 +333,10 @@ int psc_voxelize_spheres(const double* d_points, int M, const double* h_lo, cons
  * PSC_STEP_MOMENTS (rho, ux, uy, uz [4][N]). */
 int psc_bounceback_step(const double* f_src, double* f_dst, const uint8_t* solid, int nx, int ny, int nz, double tau,
                         double fx, double fy, double fz, unsigned flags, double* moments, void* stream);
+/* `steps` >= 0 such steps (:99-124), f0 to f1 to f0 ...: the state is in f0 after an even number of them, else in
+ * f1; then its moments, where moments is not NULL. */
+int psc_bounceback_steps(double* f0, double* f1, const uint8_t* solid, int nx, int ny, int nz, double tau, double fx,
+                         double fy, double fz, int64_t steps, double* moments, void* stream);
 
 /* ---- particle loads without caller scratch (no counterpart in the reference)
  * For callers that cannot allocate device memory -- a solver embedded in a

@@ -36,6 +36,7 @@ STEP_IMB = 2
 STEP_MOMENTS = 4
 STEP_REDUCE = 8
 STEP_MOVING = 16
+STEP_CHAINED = 32
 
 WIN_MOVING = 1
 WIN_INACTIVE = 2
@@ -177,6 +178,8 @@ SIGNATURES = {
                                      c_int, c_void_p, c_void_p]),
     "psc_bounceback_step": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_double, c_double, c_double,
                                     c_double, c_uint, c_void_p, c_void_p]),
+    "psc_bounceback_steps": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_double, c_double, c_double,
+                                     c_double, c_int64, c_void_p, c_void_p]),
     "psc_stream_push": (c_int, [c_int, c_double, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "psc_stream_pull_store": (c_int, [c_int, c_double, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "psc_stream_push_open": (c_int, [c_int, c_double, c_void_p, c_void_p, c_int, c_int, c_int, c_double,

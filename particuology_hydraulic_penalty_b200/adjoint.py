@@ -116,7 +116,7 @@ class PermeabilityProblem:
             size = ctypes.sizeof(nat.PscWindow)
             for k in range(L - 1):
                 nat.call("psc_step_windows", self.store, ctypes.c_void_p(table.data_ptr() + k * size), 1, per,
-                         nat.STEP_COLLIDE, 0, stream_handle(self.device))
+                         nat.STEP_COLLIDE | nat.STEP_CHAINED, 0, stream_handle(self.device))
         return buf
 
     def backward(self) -> np.ndarray:

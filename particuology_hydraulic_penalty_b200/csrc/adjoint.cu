@@ -140,6 +140,7 @@ __global__ void k_adjoint_seed(psc_adjoint_args a) {
 //   mu_i = (1 - kb - B) l_i + B l_j + d/d(rho - 1) + c . d/dm.
 template <typename V>
 struct AdjointConst {
+    const void *state, *lam;
     V inv_tau, fx, fy, fz, pref3;  // pref3 = 3 pref
     V K9[9];                       // 9 pref w_k (c_k . F)
 };
@@ -257,10 +258,15 @@ template <typename R>
 __global__ void __launch_bounds__(256) k_adjoint_step(const __grid_constant__ psc_adjoint_args a) {
     __shared__ AdjointConst<R> c;
     if (threadIdx.x == 0) make_adjoint_const(c, a);
+    chain_wait();
+    if (threadIdx.x == 0) {
+        c.state = a.state;
+        c.lam = a.lam_in;
+    }
     __syncthreads();
     const uint32_t N = (uint32_t)a.nx * a.ny * a.nz;
-    const R* S = reinterpret_cast<const R*>(a.state);
-    const R* lin = reinterpret_cast<const R*>(a.lam_in);
+    const R* S = reinterpret_cast<const R*>(c.state);
+    const R* lin = reinterpret_cast<const R*>(c.lam);
     R* lout = reinterpret_cast<R*>(a.lam_out);
     const uint32_t stride = gridDim.x * blockDim.x;
     StrideWalk at(blockIdx.x * blockDim.x + threadIdx.x, stride, a.nx, a.ny, a.nz);
@@ -289,10 +295,15 @@ constexpr int ADJ_THREADS = 128, ADJ_CTAS = 3;
 __global__ void __launch_bounds__(ADJ_THREADS, ADJ_CTAS) k_adjoint_pair(const __grid_constant__ psc_adjoint_args a) {
     __shared__ AdjointConst<F2> c;
     if (threadIdx.x == 0) make_adjoint_const(c, a);
+    chain_wait();
+    if (threadIdx.x == 0) {
+        c.state = a.state;
+        c.lam = a.lam_in;
+    }
     __syncthreads();
     const uint32_t N = (uint32_t)a.nx * a.ny * a.nz, nz = (uint32_t)a.nz;
-    const float* S = reinterpret_cast<const float*>(a.state);
-    const float* lin = reinterpret_cast<const float*>(a.lam_in);
+    const float* S = reinterpret_cast<const float*>(c.state);
+    const float* lin = reinterpret_cast<const float*>(c.lam);
     float* lout = reinterpret_cast<float*>(a.lam_out);
     const float tau = (float)a.tau;
     const uint32_t stride = 2 * gridDim.x * blockDim.x;
@@ -459,13 +470,13 @@ cudaError_t launch_adjoint_step(const psc_adjoint_args& a, cudaStream_t stream) 
     const int64_t N = (int64_t)a.nx * a.ny * a.nz;
     const auto aligned = [](const void* p, uintptr_t n) { return reinterpret_cast<uintptr_t>(p) % n == 0; };
     if (a.store == PSC_STORE_F64)
-        k_adjoint_step<double><<<cap_grid(N, 256, 8), 256, 0, stream>>>(a);
+        return launch_chained(k_adjoint_step<double>, cap_grid(N, 256, 8), 256, 0, stream, true, a);
     else if (a.nz % 2 == 0 && aligned(a.state, 8) && aligned(a.lam_in, 8) && aligned(a.lam_out, 8) &&
              aligned(a.solid, 16) && aligned(a.dKdB, 16))
-        k_adjoint_pair<<<cap_grid(N / 2, ADJ_THREADS, ADJ_CTAS), ADJ_THREADS, 0, stream>>>(a);  // (the resident CTAs)
+        return launch_chained(k_adjoint_pair, cap_grid(N / 2, ADJ_THREADS, ADJ_CTAS), ADJ_THREADS, 0, stream, true,
+                              a);  // (the resident CTAs)
     else
-        k_adjoint_step<float><<<cap_grid(N, 256, 8), 256, 0, stream>>>(a);
-    return cudaGetLastError();
+        return launch_chained(k_adjoint_step<float>, cap_grid(N, 256, 8), 256, 0, stream, true, a);
 }
 
 cudaError_t launch_adjoint_geometry_grad(const psc_geometry& g, const psc_adjoint_args& a, double* part,

@@ -389,6 +389,23 @@ int psc_bounceback_step(const double* f_src, double* f_dst, const uint8_t* solid
     return e == cudaSuccess ? PSC_OK : cuda_fail(e, "psc_bounceback_step");
 }
 
+int psc_bounceback_steps(double* f0, double* f1, const uint8_t* solid, int nx, int ny, int nz, double tau, double fx,
+                         double fy, double fz, int64_t steps, double* moments, void* stream) {
+    int st = check_extent(nx, ny, nz, "psc_bounceback_steps");
+    if (st) return st;
+    if (!f0 || !solid || steps < 0 || (steps > 0 && (!f1 || f1 == f0)))
+        return fail(PSC_E_INVALID, "psc_bounceback_steps: bad arguments");
+    if (!(tau > 0.5)) return fail(PSC_E_INVALID, "psc_bounceback_steps: tau must exceed 0.5");
+    cudaError_t e = cudaSuccess;
+    for (int64_t k = 0; k < steps && e == cudaSuccess; ++k)
+        e = launch_bb_step(k % 2 ? f1 : f0, k % 2 ? f0 : f1, solid, nx, ny, nz, tau, fx, fy, fz, PSC_STEP_COLLIDE, nullptr,
+                           as_stream(stream));
+    if (moments && e == cudaSuccess)
+        e = launch_bb_step(steps % 2 ? f1 : f0, nullptr, solid, nx, ny, nz, tau, fx, fy, fz, PSC_STEP_MOMENTS, moments,
+                           as_stream(stream));
+    return e == cudaSuccess ? PSC_OK : cuda_fail(e, "psc_bounceback_steps");
+}
+
 int psc_stream_push(int store, double store_scale, const void* src, double* dst, int nx, int ny, int nz,
                     void* stream) {
     if (!valid_store(store) || !src || !dst) return fail(PSC_E_INVALID, "psc_stream_push: bad arguments");

@@ -786,6 +786,7 @@ __global__ void __launch_bounds__(LOAD_THREADS, 3) k_loads_chunks_list(psc_geome
                                                                          const double* desc, double* part) {
     __shared__ ChunkRing rows;
     extern __shared__ __align__(16) unsigned char list_stage[];
+    chain_wait();
     chunk_ring_init(rows);
     const int64_t C = g.totals[1];
     const uint32_t N = (uint32_t)g.nx * g.ny * g.nz;
@@ -1071,6 +1072,7 @@ __device__ __forceinline__ void loads_final_cluster(int P, const int64_t* chunk_
 __global__ void __cluster_dims__(FINAL_CTAS, 1, 1) __launch_bounds__(FINAL_THREADS)
     k_loads_final(const __grid_constant__ psc_geometry g, const double* part, const double* imb_sums, double* forces,
                   double* torques, double* diag, double* host_diag) {
+    chain_wait();
     loads_final_cluster(g.nparticles, g.chunk_off, part, imb_sums, forces, torques, diag, host_diag);
 }
 
@@ -1137,6 +1139,7 @@ __global__ void __launch_bounds__(LOAD_THREADS, 3) k_loads_chunks_list_multi(con
                                                                            const double* desc, double* part) {
     __shared__ ChunkRing rows;
     extern __shared__ __align__(16) unsigned char list_stage[];
+    chain_wait();
     chunk_ring_init(rows);
     const int64_t C = chunk_base[njobs];
     ListCursor cur{};
@@ -1191,6 +1194,7 @@ __global__ void __launch_bounds__(1024) k_loads_diag_multi(const LoadsJob* jobs)
 
 __global__ void __cluster_dims__(FINAL_CTAS, 1, 1) __launch_bounds__(FINAL_THREADS)
     k_loads_final_multi(const LoadsJob* jobs, const int64_t* chunk_base, const double* part) {
+    chain_wait();
     const int k = blockIdx.x / FINAL_CTAS;
     const LoadsJob& J = jobs[k];
     loads_final_cluster(J.g.nparticles, J.g.chunk_off, part + chunk_base[k] * 6, J.imb_sums, J.forces, J.torques, J.diag,
@@ -1418,9 +1422,8 @@ cudaError_t launch_particle_loads(const psc_geometry& g, int imb_type, const voi
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     if (g.nparticles > 0 && g.nparticles <= FINAL_PARTICLES) {
-        k_loads_final<<<FINAL_CTAS, FINAL_THREADS, 0, stream>>>(g, chunk_partials, imb_sums, forces, torques, diag,
-                                                               host_diag);
-        return cudaGetLastError();
+        return launch_chained(k_loads_final, FINAL_CTAS, FINAL_THREADS, 0, stream, true, g, chunk_partials, imb_sums, forces,
+                              torques, diag, host_diag);
     }
     if (g.nparticles > 0) {
         k_loads_particles<<<(g.nparticles + 7) / 8, 256, 0, stream>>>(g, chunk_partials, forces, torques);
@@ -1461,8 +1464,8 @@ cudaError_t launch_particle_loads_multi(const LoadsJob* d_jobs, const int64_t* d
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     if (max_particles <= FINAL_PARTICLES) {
-        k_loads_final_multi<<<(unsigned)(njobs * FINAL_CTAS), FINAL_THREADS, 0, stream>>>(d_jobs, d_chunk_base, part);
-        return cudaGetLastError();
+        return launch_chained(k_loads_final_multi, (unsigned)(njobs * FINAL_CTAS), FINAL_THREADS, 0, stream, true, d_jobs,
+                              d_chunk_base, part);
     }
     if (total_particles > 0) {
         k_loads_particles_multi<<<(unsigned)((total_particles + 7) / 8), 256, 0, stream>>>(

@@ -60,6 +60,35 @@ cudaError_t launch_init_equilibrium(int store, double scale, void* f, int64_t nc
 // inlet = {rho, ux, uy, uz} when open_x (PSC_WIN_OPEN_X faces), else unused
 cudaError_t launch_stream_push(int store, double scale, const void* src, double* dst, int nx, int ny, int nz,
                                cudaStream_t stream, bool open_x = false, const double* inlet = nullptr);
+// A launch that may start before the kernel ahead of it on its stream has ended (chained): its CTAs take the
+// SMs as they fall free and set up what that kernel does not write; then every CTA waits (chain_wait) before
+// it touches anything else, and lets its own successor in only then, so at most two kernels
+// of a stream overlap.  A pointer that is read through the read-only path after the wait goes through
+// shared memory, so that no such load is moved above it.  A step in a row of steps: 64^3 FP32 8.9 -> 7.7 us,
+// 75^3 FP32 12.0 -> 10.5, 24^3 exact 4.65 -> 3.86, 96^3 exact 55.8 -> 54.1 us.
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream,
+                                  bool chained, A... args) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = stream;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = chained ? 1 : 0;
+    cudaLaunchKernelEx(&c, kernel, P(args)...);
+    return cudaGetLastError();
+}
+// Waits until the kernels ahead on the stream have ended and their results are visible; then the next one may
+// take the SMs that this one leaves.
+__device__ __forceinline__ void chain_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 cudaError_t launch_stream_pull_store(int store, double scale, const double* src, void* dst, int nx, int ny, int nz,
                                      cudaStream_t stream, bool open_x = false, const double* inlet = nullptr);
 

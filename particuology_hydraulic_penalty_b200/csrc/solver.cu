@@ -632,7 +632,7 @@ int launch_solo(Window& w, unsigned flags, cudaStream_t s) {
     PSC_TRY(window_upload_solo(w, s));
     if (w.moving) flags |= PSC_STEP_MOVING;
     psc_launch c = {0, 1, w.solo_kernel, 0, 0};
-    return psc_step_windows_ex(w.cfg.store, w.solo[w.cur].p, 1, w.solo_tiles, flags, &c, s);
+    return psc_step_windows_ex(w.cfg.store, w.solo[w.cur].p, 1, w.solo_tiles, flags | PSC_STEP_CHAINED, &c, s);
 }
 
 double* red_pre(Window& w) { return w.out.p; }
@@ -1073,7 +1073,7 @@ std::vector<uint64_t> solver_step_inputs(const psc_solver& h) {
 int report_step_work(psc_solver& h, int par, int kind) {
     Window& w = h.w;
     cudaStream_t s = h.stream;
-    const unsigned mv = w.moving ? PSC_STEP_MOVING : 0u;
+    const unsigned mv = (w.moving ? PSC_STEP_MOVING : 0u) | PSC_STEP_CHAINED;
     const psc_launch c = {0, 1, w.solo_kernel, 0, 0};
     const unsigned full = PSC_STEP_COLLIDE | PSC_STEP_IMB | PSC_STEP_REDUCE | mv;
     const double* pre = h.ahead_red.p + (par ^ 1) * PSC_NRED;
@@ -1198,7 +1198,7 @@ int solver_converge(psc_solver& h, int nsteps, double tol, int min_steps, int ch
     for (auto& e : h.conv_ev)
         if (!e) PSC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), who);
     PSC_CUDA(cudaMemsetAsync(h.conv.p, 0, kConvState * sizeof(double), s), who);
-    const unsigned mv = w.moving ? PSC_STEP_MOVING : 0u;
+    const unsigned mv = w.moving ? PSC_STEP_MOVING : 0u;  // (not chained: the criterion ends the window in its table)
     const psc_launch c = {0, 1, w.solo_kernel, 0, 0};
     const int start = w.cur;
     const auto row = [&](int u) { return h.conv.p + kConvState + (2 + (u & 1)) * PSC_NRED; };
@@ -1754,8 +1754,8 @@ bool batch_may_run_ahead(const psc_batch& b, bool fields, const std::vector<uint
 
 int batch_launch(psc_batch& b, unsigned flags) {
     if (b.moving_any) flags |= PSC_STEP_MOVING;
-    return psc_step_windows_ex(b.store, b.table[b.parity].p, (int)b.w.size(), b.total_tiles, flags, &b.launch,
-                               b.stream);
+    return psc_step_windows_ex(b.store, b.table[b.parity].p, (int)b.w.size(), b.total_tiles, flags | PSC_STEP_CHAINED,
+                               &b.launch, b.stream);
 }
 
 // The main stream waits for a pending particle upload (psc_batch_set_particles_all):
@@ -2392,7 +2392,8 @@ int adj_segment(psc_adjoint& a, int t0, int t1) {
              "psc_adjoint_backward");
     psc_launch c = {0, 1, PSC_KERNEL_AUTO, 0, 0};
     for (int k = 0; k < L - 1; ++k)
-        PSC_TRY(psc_step_windows_ex(w.cfg.store, a.seg_tab.p + k, 1, tab[(size_t)k].tile_count, PSC_STEP_COLLIDE, &c, s));
+        PSC_TRY(psc_step_windows_ex(w.cfg.store, a.seg_tab.p + k, 1, tab[(size_t)k].tile_count,
+                                    PSC_STEP_COLLIDE | PSC_STEP_CHAINED, &c, s));
     PSC_CUDA(cudaStreamSynchronize(s), "psc_adjoint_backward");  // tab lives on this frame
     return PSC_OK;
 }

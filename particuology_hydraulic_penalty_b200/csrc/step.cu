@@ -65,6 +65,7 @@ __global__ void __cluster_dims__(REDUCE_CTAS, 1, 1) __launch_bounds__(REDUCE_THR
     k_reduce_windows(const psc_window* __restrict__ wins, double* __restrict__ out, double* __restrict__ out2,
                      const __grid_constant__ ConvergeCheck cc) {
     namespace cg = cooperative_groups;
+    chain_wait();
     __shared__ double s_g[REDUCE_GROUPS * PSC_NRED];
     __shared__ double s_cta[PSC_NRED];
     cg::cluster_group cluster = cg::this_cluster();
@@ -213,15 +214,14 @@ __global__ void k_stream_pull_store(const double* src, void* dst, int nx, int ny
 // ---------------------------------------------------------------------------
 cudaError_t launch_reduce_windows(const psc_window* d_windows, int nwin, double* out, cudaStream_t stream,
                                   double* out2) {
-    k_reduce_windows<false>
-        <<<nwin * REDUCE_CTAS, REDUCE_THREADS, 0, stream>>>(d_windows, out, out2, ConvergeCheck{});
-    return cudaGetLastError();
+    return launch_chained(k_reduce_windows<false>, nwin * REDUCE_CTAS, REDUCE_THREADS, 0, stream, true, d_windows, out, out2,
+                          ConvergeCheck{});
 }
 
 cudaError_t launch_reduce_converge(const psc_window* d_window, double* out, const ConvergeCheck& cc,
                                    cudaStream_t stream) {
-    k_reduce_windows<true><<<REDUCE_CTAS, REDUCE_THREADS, 0, stream>>>(d_window, out, nullptr, cc);
-    return cudaGetLastError();
+    return launch_chained(k_reduce_windows<true>, REDUCE_CTAS, REDUCE_THREADS, 0, stream, true, d_window, out,
+                          static_cast<double*>(nullptr), cc);
 }
 
 static int grid_for(int64_t work, int threads) {

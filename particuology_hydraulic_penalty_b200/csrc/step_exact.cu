@@ -154,6 +154,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 2)
     __shared__ ExactShared sw;
     __shared__ double s_red[RED ? PSC_NRED : 1][STEP_THREADS];  // running sums per thread (in registers they would spill)
     static_assert(STEP_THREADS / 32 == PSC_PARTIAL_ROWS, "one partial row per warp");
+    if (!(flags & PSC_STEP_CHAINED)) chain_wait();  // (the table may be what it waits for)
     const bool do_collide = flags & PSC_STEP_COLLIDE;
     const bool do_imb = do_collide && (flags & PSC_STEP_IMB);
     const bool do_mom = flags & PSC_STEP_MOMENTS;
@@ -173,8 +174,10 @@ __global__ void __launch_bounds__(STEP_THREADS, 2)
             if (RED && have) flush();
             have = false;
             __syncthreads();
-            wi = wi < 0 ? find_window(wins, nullptr, nwin, t) : advance_window(wins, nwin, wi, t);
+            const bool first = wi < 0;
+            wi = first ? find_window(wins, nullptr, nwin, t) : advance_window(wins, nwin, wi, t);
             load_exact_win(sw, wins[wi], MOVING, (int32_t)walk.size);
+            if (first && (flags & PSC_STEP_CHAINED)) chain_wait();
             if (RED) {
 #pragma unroll
                 for (int q = 0; q < (RED ? PSC_NRED : 1); ++q) s_red[q][threadIdx.x] = 0.0;
@@ -292,9 +295,8 @@ static cudaError_t launch_exact_t(const psc_window* d_windows, int nwin, int64_t
     }
     if ((int64_t)grid_ctas > total_tiles) grid_ctas = (int)total_tiles;  // every CTA owns >= 1 tile
     if (grid_ctas <= 0) return cudaSuccess;
-    k_step_exact<MOVING, RED><<<grid_ctas, STEP_THREADS, 0, stream>>>(
-        d_windows, nwin, flags, tile_plan(total_tiles, nwin, grid_ctas));
-    return cudaGetLastError();
+    return launch_chained(k_step_exact<MOVING, RED>, grid_ctas, STEP_THREADS, 0, stream, true, d_windows,
+                          nwin, flags, tile_plan(total_tiles, nwin, grid_ctas));
 }
 
 cudaError_t launch_step_exact(const psc_window* d_windows, int nwin, int64_t total_tiles, unsigned flags, bool moving,

@@ -63,6 +63,7 @@ __global__ void __launch_bounds__(STEP_THREADS, (StepOccupancy<STORE, MOVING, RE
             __syncthreads();
             wi = wi < 0 ? find_window(wins, nullptr, nwin, t) : advance_window(wins, nwin, wi, t);
             load_fast_win(sw, wins[wi], MOVING, (int32_t)walk.size, prev >= 0 ? wins + prev : nullptr);
+            if (prev < 0) chain_wait();
             prev = wi;
             __syncthreads();
             win_end = (uint32_t)sw.tile_end;
@@ -164,9 +165,8 @@ static cudaError_t launch_fast_t(const psc_window* d_windows, int nwin, int64_t 
     }
     if ((int64_t)grid_ctas > total_tiles) grid_ctas = (int)total_tiles;  // every CTA owns >= 1 tile
     if (grid_ctas <= 0) return cudaSuccess;
-    k_step_fast<STORE, MOVING, CPT, RED><<<grid_ctas, STEP_THREADS, 0, stream>>>(
-        d_windows, nwin, flags, tile_plan(total_tiles, nwin, grid_ctas));
-    return cudaGetLastError();
+    return launch_chained(k_step_fast<STORE, MOVING, CPT, RED>, grid_ctas, STEP_THREADS, 0, stream, flags & PSC_STEP_CHAINED,
+                          d_windows, nwin, flags, tile_plan(total_tiles, nwin, grid_ctas));
 }
 
 template <int STORE, bool RED>

@@ -17,7 +17,6 @@
 
 namespace psc {
 
-
 // Set (once) when a launch met a window it cannot run: 0x201 odd nz,
 // 0x202 tiles not planned by psc_plan_pair_tiles.  Such windows are skipped.
 __device__ int g_pair_status = 0;
@@ -71,7 +70,7 @@ __global__ void __launch_bounds__(STEP_THREADS, (PairOccupancy<STORE, MOVING, RE
     using T = typename TR::T;
     using R = typename TR::R;
     using O = typename TR::O;
-        // Both cells in packed FP32 where the arithmetic bounds the kernel: 16-bit storage (160^3: 90 -> 82 us
+    // Both cells in packed FP32 where the arithmetic bounds the kernel: 16-bit storage (160^3: 90 -> 82 us
     // plain, 107 -> 99 with IMB and sums; 378 -> 261 instructions per cell).  FP32 storage is bound by HBM,
     // and there the packed form was slower (114 against 108 us: its shorter bursts of arithmetic leave
     // reads and writes less spread).  FP64 has no packed form.
@@ -111,6 +110,7 @@ __global__ void __launch_bounds__(STEP_THREADS, (PairOccupancy<STORE, MOVING, RE
             __syncthreads();
             wi = wi < 0 ? find_window(wins, nullptr, nwin, t) : advance_window(wins, nwin, wi, t);
             load_fast_win(sw, wins[wi], MOVING, (int32_t)walk.size, prev >= 0 ? wins + prev : nullptr);
+            if (prev < 0) chain_wait();
             prev = wi;
             __syncthreads();
             win_end = (uint32_t)sw.tile_end;
@@ -242,9 +242,8 @@ static cudaError_t launch_pair_t(const psc_window* d_windows, int nwin, int64_t 
     }
     if ((int64_t)grid_ctas > total_tiles) grid_ctas = (int)total_tiles;  // every CTA owns >= 1 tile
     if (grid_ctas <= 0) return cudaSuccess;
-    k_step_pair<STORE, MOVING, RED><<<grid_ctas, STEP_THREADS, 0, stream>>>(
-        d_windows, nwin, flags, tile_plan(total_tiles, nwin, grid_ctas));
-    return cudaGetLastError();
+    return launch_chained(k_step_pair<STORE, MOVING, RED>, grid_ctas, STEP_THREADS, 0, stream, flags & PSC_STEP_CHAINED,
+                          d_windows, nwin, flags, tile_plan(total_tiles, nwin, grid_ctas));
 }
 
 template <int STORE>

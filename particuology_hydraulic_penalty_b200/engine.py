@@ -475,7 +475,8 @@ class LatticeWindow:
         self.ensure_fields(imb=bool(flags & nat.STEP_IMB), moments=bool(flags & nat.STEP_MOMENTS))
         if self.solid_ptr is None:
             raise RuntimeError("geometry not bound")
-        fl = flags | nat.STEP_COLLIDE | (nat.STEP_MOVING if self.moving else 0)
+        # (chained: the window tables are copied from the host, not written by a kernel)
+        fl = flags | nat.STEP_COLLIDE | nat.STEP_CHAINED | (nat.STEP_MOVING if self.moving else 0)
         nat.call("psc_step_windows", self.store, vp(self.windows(self.cur)), 1, self.tiles, fl, 0,
                  stream_handle(self.device))
         self.cur = 1 - self.cur
@@ -486,7 +487,7 @@ class LatticeWindow:
     def moments_pass(self, reduce_out: torch.Tensor | None = None, write_fields: bool = True) -> None:
         """Moments (and reductions) of the current post-stream state, no collision."""
         self.ensure_fields(imb=False, moments=write_fields)
-        fl = (nat.STEP_MOMENTS if write_fields else 0) | (nat.STEP_REDUCE if reduce_out is not None else 0)
+        fl = (nat.STEP_MOMENTS if write_fields else 0) | (nat.STEP_REDUCE if reduce_out is not None else 0) | nat.STEP_CHAINED
         nat.call("psc_step_windows", self.store, vp(self.windows(self.cur)), 1, self.tiles, fl, 0,
                  stream_handle(self.device))
         if reduce_out is not None:

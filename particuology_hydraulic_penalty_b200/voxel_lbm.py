@@ -3,7 +3,7 @@
 ``voxelize`` and ``run_lbm`` keep the names, arguments and results of
 scripts/run_3d_window_lbm.py (:73-92, :95-146) -- the drag-proxy solver the
 older coupled loop uses -- and run in libpscb200.so (psc_voxelize_spheres,
-psc_bounceback_step) in exact FP64, bit-identical to the reference.
+psc_bounceback_steps) in exact FP64, bit-identical to the reference.
 """
 
 from __future__ import annotations
@@ -54,13 +54,8 @@ def run_lbm(solid, tau: float, force_z: float, steps: int, return_fields: bool =
         mom = torch.empty(4 * N, dtype=torch.float64, device=dev)
         st = stream_handle(dev)
         nat.call("psc_init_equilibrium", nat.STORE_F64_EXACT, 1.0, vp(f[0]), N, st)
-        cur = 0
-        for _ in range(int(steps)):
-            nat.call("psc_bounceback_step", vp(f[cur]), vp(f[1 - cur]), vp(s), nx, ny, nz, float(tau), 0.0, 0.0,
-                     float(force_z), nat.STEP_COLLIDE, None, st)
-            cur = 1 - cur
-        nat.call("psc_bounceback_step", vp(f[cur]), None, vp(s), nx, ny, nz, float(tau), 0.0, 0.0, float(force_z),
-                 nat.STEP_MOMENTS, vp(mom), st)
+        nat.call("psc_bounceback_steps", vp(f[0]), vp(f[1]), vp(s), nx, ny, nz, float(tau), 0.0, 0.0, float(force_z),
+                 max(int(steps), 0), vp(mom), st)
         m = mom.view(4, nx, ny, nz).cpu().numpy()
     ux, uy, uz = m[1], m[2], m[3]
     fluid = ~solid_np
