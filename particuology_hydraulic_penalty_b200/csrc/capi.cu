@@ -197,7 +197,8 @@ int psc_init_equilibrium(int store, double store_scale, void* f, int64_t ncells,
 int psc_geometry_plan(const psc_geometry* h_geo, void* stream) {
     int st = check_geometry(h_geo, "psc_geometry_plan");
     if (st) return st;
-    cudaError_t e = launch_geometry_plan(*h_geo, as_stream(stream));
+    const GeoJob job = {*h_geo};
+    cudaError_t e = launch_geometry_plan(&job, 1, as_stream(stream));
     return e == cudaSuccess ? PSC_OK : cuda_fail(e, "psc_geometry_plan");
 }
 
@@ -217,7 +218,8 @@ int psc_geometry_build(const psc_geometry* h_geo, void* stream) {
         return fail(PSC_E_INVALID, "psc_geometry_build: smooth mode needs ent_alpha and cl_ent");
     if (g.smooth_eps > 0.0 && g.level)
         return fail(PSC_E_INVALID, "psc_geometry_build: smooth mode has no integer level (pass level = NULL)");
-    cudaError_t e = launch_geometry_build(g, as_stream(stream));
+    const GeoJob job = {g};
+    cudaError_t e = launch_geometry_build(&job, 1, as_stream(stream));
     return e == cudaSuccess ? PSC_OK : cuda_fail(e, "psc_geometry_build");
 }
 
@@ -225,7 +227,8 @@ int psc_solid_velocity(const psc_geometry* h_geo, int us_type, void* us, void* s
     int st = check_geometry(h_geo, "psc_solid_velocity");
     if (st) return st;
     if (!us || (us_type != 0 && us_type != 1)) return fail(PSC_E_INVALID, "psc_solid_velocity: bad output");
-    cudaError_t e = launch_solid_velocity(*h_geo, us_type, us, as_stream(stream));
+    const GeoJob job = {*h_geo, nullptr, nullptr, us, us_type};
+    cudaError_t e = launch_solid_velocity(&job, 1, as_stream(stream));
     return e == cudaSuccess ? PSC_OK : cuda_fail(e, "psc_solid_velocity");
 }
 

@@ -72,8 +72,17 @@ __device__ __forceinline__ T block_exclusive_scan(T v, T* s_warp, T& total) {
     return warp_prefix + x - v;
 }
 
-// One block: boxes, entry offsets, chunk offsets, totals.
-__global__ void __launch_bounds__(1024) k_geometry_plan(psc_geometry g) {
+// The kernels of a rebuild take up to kGeoJobs windows, one per row of the grid (blockIdx.y): one window's
+// kernels are too small for the GPU and a window took eleven launches and three copies of its own (two steps
+// of six moving 64^3 windows, rebuilt every call: 0.69 ms with the windows' launches on four streams,
+// 0.58 ms so).
+struct GeoJobs {
+    GeoJob j[kGeoJobs];
+};
+
+// One block per window: boxes, entry offsets, chunk offsets, totals.
+__global__ void __launch_bounds__(1024) k_geometry_plan(const __grid_constant__ GeoJobs jobs) {
+    const psc_geometry& g = jobs.j[blockIdx.y].g;
     __shared__ int64_t s_warp[32];
     __shared__ int64_t s_carry[2];
     const int P = g.nparticles;
@@ -123,6 +132,10 @@ __global__ void __launch_bounds__(1024) k_geometry_plan(psc_geometry g) {
         g.totals[1] = s_carry[1];
         g.totals[2] = 0;
         g.totals[3] = (s_carry[0] > g.capacity_entries || s_carry[1] > g.capacity_chunks) ? 1 : 0;
+        if (int64_t* host = jobs.j[blockIdx.y].host_totals) {
+            host[0] = s_carry[0];
+            host[1] = s_carry[1];
+        }
     }
 }
 
@@ -296,19 +309,21 @@ __device__ __forceinline__ void geometry_count(const psc_geometry& g, const doub
 }
 
 template <int S>
-__global__ void __launch_bounds__(256, 2) k_geometry_count(const __grid_constant__ psc_geometry g, const double* desc) {
-    geometry_count<S, false, 1>(g, desc);
+__global__ void __launch_bounds__(256, 2) k_geometry_count(const __grid_constant__ GeoJobs jobs) {
+    geometry_count<S, false, 1>(jobs.j[blockIdx.y].g, jobs.j[blockIdx.y].desc);
 }
 constexpr int SMOOTH_PARTS = 16;
 template <int S>
 __global__ void __launch_bounds__(256, 2) k_geometry_smooth(const __grid_constant__ psc_geometry g, const double* desc) {
-    geometry_count<S, true, SMOOTH_PARTS>(g, desc);
+    geometry_count<S, true, SMOOTH_PARTS>(g, desc);  // (a window of its own: from a table 333 -> 372 us)
 }
 
 // The cell lists: every entry with a non-zero count appends (particle, count)
 // to its cell's list (the order within a list is fixed by k_geometry_final's
 // sort).  Walks the chunks as k_geometry_count does.
-__global__ void __launch_bounds__(256) k_geometry_fill(const __grid_constant__ psc_geometry g, const double* desc) {
+__global__ void __launch_bounds__(256) k_geometry_fill(const __grid_constant__ GeoJobs jobs) {
+    const psc_geometry& g = jobs.j[blockIdx.y].g;
+    const double* desc = jobs.j[blockIdx.y].desc;
     const int64_t E = min(g.totals[0], g.capacity_entries);
     const int64_t C = g.totals[1];
     const uint32_t ny = (uint32_t)g.ny, nz = (uint32_t)g.nz;
@@ -350,7 +365,8 @@ __global__ void __launch_bounds__(256) k_geometry_fill(const __grid_constant__ p
     }
 }
 
-__global__ void k_geometry_final(psc_geometry g) {
+__global__ void k_geometry_final(const __grid_constant__ GeoJobs jobs) {
+    const psc_geometry& g = jobs.j[blockIdx.y].g;
     const uint32_t N = (uint32_t)g.nx * g.ny * g.nz;
     const int S = g.subsamples;
     const int S3 = S * S * S;
@@ -395,7 +411,9 @@ __global__ void k_geometry_final(psc_geometry g) {
 }
 
 template <typename O>
-__global__ void k_solid_velocity(psc_geometry g, O* us) {
+__global__ void k_solid_velocity(const __grid_constant__ GeoJobs jobs) {
+    const psc_geometry& g = jobs.j[blockIdx.y].g;
+    O* us = reinterpret_cast<O*>(jobs.j[blockIdx.y].us);
     const uint32_t N = (uint32_t)g.nx * g.ny * g.nz;
     const double S3d = (double)(g.subsamples * g.subsamples * g.subsamples);
     for (uint32_t cell = blockIdx.x * blockDim.x + threadIdx.x; cell < N; cell += gridDim.x * blockDim.x) {
@@ -513,6 +531,17 @@ __global__ void __launch_bounds__(256) k_chunk_desc(psc_geometry g, double* part
     const int64_t C = g.totals[1];
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < C; c += (int64_t)gridDim.x * blockDim.x)
         *reinterpret_cast<ChunkDesc*>(part + c * 6) = make_chunk_desc(g, c);
+}
+
+// The start of a build: no cell has an entry; the chunk descriptors, where they are kept.
+__global__ void __launch_bounds__(256) k_geometry_begin(const __grid_constant__ GeoJobs jobs) {
+    const psc_geometry& g = jobs.j[blockIdx.y].g;
+    const int64_t N = (int64_t)g.nx * g.ny * g.nz, stride = (int64_t)gridDim.x * blockDim.x;
+    const int64_t first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    double* desc = jobs.j[blockIdx.y].desc;
+    const int64_t C = desc ? g.totals[1] : 0;
+    for (int64_t c = first; c < C; c += stride) *reinterpret_cast<ChunkDesc*>(desc + c * 6) = make_chunk_desc(g, c);
+    for (int64_t c = first; c < N; c += stride) g.cell_n[c] = 0;
 }
 
 // The block's table of inside / S^3 for every sample count (S <= 16) holds
@@ -1214,32 +1243,74 @@ __global__ void __launch_bounds__(256) k_copy_rows(const __grid_constant__ RowCo
 }
 
 // ---------------------------------------------------------------------------
-// exclusive scan (int32), three passes over blocks of SCAN_ITEMS elements
+// exclusive scan of the cells' entry counts, over blocks of SCAN_ITEMS cells
 // ---------------------------------------------------------------------------
 constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_PER_THREAD = 8;
 constexpr int SCAN_ITEMS = SCAN_THREADS * SCAN_PER_THREAD;
+// Up to SCAN_DIRECT blocks each adds up the blocks before it by itself; beyond, where that would read more
+// than the cells do, k_scan_top does it once.
+constexpr int SCAN_DIRECT = 2048;
 
 size_t scan_tmp_bytes(int64_t n) {
     const int64_t nb = (n + SCAN_ITEMS - 1) / SCAN_ITEMS;
     return (size_t)(nb + 1) * sizeof(int32_t) + 256;
 }
 
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_partial(const int32_t* in, int64_t n, int32_t* bsum) {
-    __shared__ int32_t s_warp[32];
-    const int64_t base = (int64_t)blockIdx.x * SCAN_ITEMS + (int64_t)threadIdx.x * SCAN_PER_THREAD;
-    int32_t acc = 0;
-#pragma unroll
-    for (int k = 0; k < SCAN_PER_THREAD; ++k)
-        if (base + k < n) acc += in[base + k];
-    int32_t total;
-    block_exclusive_scan<int32_t>(acc, s_warp, total);
-    if (threadIdx.x == 0) bsum[blockIdx.x] = total;
+__device__ __forceinline__ int64_t scan_blocks(const psc_geometry& g) {
+    return ((int64_t)g.nx * g.ny * g.nz + SCAN_ITEMS - 1) / SCAN_ITEMS;
 }
 
-__global__ void __launch_bounds__(1024) k_scan_top(int32_t* bsum, int64_t nb) {
+// This thread's SCAN_PER_THREAD values from base on (0 beyond n).
+__device__ __forceinline__ void scan_load(const int32_t* in, int64_t base, int64_t n, int32_t (&v)[SCAN_PER_THREAD]) {
+    if (base + SCAN_PER_THREAD <= n && reinterpret_cast<uintptr_t>(in) % 16 == 0) {
+#pragma unroll
+        for (int k = 0; k < SCAN_PER_THREAD; k += 4) {
+            const int4 q = *reinterpret_cast<const int4*>(in + base + k);
+            v[k] = q.x;
+            v[k + 1] = q.y;
+            v[k + 2] = q.z;
+            v[k + 3] = q.w;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < SCAN_PER_THREAD; ++k) v[k] = base + k < n ? in[base + k] : 0;
+    }
+}
+__device__ __forceinline__ void scan_store(int32_t* out, int64_t base, int64_t n, const int32_t (&v)[SCAN_PER_THREAD]) {
+    if (base + SCAN_PER_THREAD <= n && reinterpret_cast<uintptr_t>(out) % 16 == 0) {
+#pragma unroll
+        for (int k = 0; k < SCAN_PER_THREAD; k += 4)
+            *reinterpret_cast<int4*>(out + base + k) = make_int4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < SCAN_PER_THREAD; ++k)
+            if (base + k < n) out[base + k] = v[k];
+    }
+}
+
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_partial(const __grid_constant__ GeoJobs jobs) {
+    __shared__ int32_t s_warp[32];
+    const psc_geometry& g = jobs.j[blockIdx.y].g;
+    const int64_t n = (int64_t)g.nx * g.ny * g.nz;
+    if (blockIdx.x >= scan_blocks(g)) return;  // (a smaller window)
+    int32_t v[SCAN_PER_THREAD];
+    scan_load(g.cell_n, (int64_t)blockIdx.x * SCAN_ITEMS + (int64_t)threadIdx.x * SCAN_PER_THREAD, n, v);
+    int32_t acc = 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_PER_THREAD; ++k) acc += v[k];
+    int32_t total;
+    block_exclusive_scan<int32_t>(acc, s_warp, total);
+    if (threadIdx.x == 0) reinterpret_cast<int32_t*>(g.scan_tmp)[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(1024) k_scan_top(const __grid_constant__ GeoJobs jobs) {
     __shared__ int32_t s_warp[32];
     __shared__ int32_t s_carry;
+    const psc_geometry& g = jobs.j[blockIdx.y].g;
+    const int64_t nb = scan_blocks(g);
+    if (nb <= SCAN_DIRECT) return;
+    int32_t* bsum = reinterpret_cast<int32_t*>(g.scan_tmp);
     if (threadIdx.x == 0) s_carry = 0;
     __syncthreads();
     for (int64_t base = 0; base < nb; base += blockDim.x) {
@@ -1252,40 +1323,39 @@ __global__ void __launch_bounds__(1024) k_scan_top(int32_t* bsum, int64_t nb) {
         if (threadIdx.x == 0) s_carry += total;
         __syncthreads();
     }
-    if (threadIdx.x == 0) bsum[nb] = s_carry;
 }
 
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(const int32_t* in, int32_t* out, int64_t n,
-                                                             const int32_t* bsum, int64_t nb) {
+// cell_off = the exclusive scan; cell_n is left at zero, the cursors of k_geometry_fill.
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(const __grid_constant__ GeoJobs jobs) {
     __shared__ int32_t s_warp[32];
+    const psc_geometry& g = jobs.j[blockIdx.y].g;
+    const int64_t n = (int64_t)g.nx * g.ny * g.nz, nb = scan_blocks(g);
+    if (blockIdx.x >= nb) return;
+    const int32_t* bsum = reinterpret_cast<const int32_t*>(g.scan_tmp);
+    int32_t before = 0, total;
+    if (nb > SCAN_DIRECT) {
+        before = bsum[blockIdx.x];
+    } else {
+        for (int64_t i = threadIdx.x; i < blockIdx.x; i += SCAN_THREADS) before += bsum[i];
+        block_exclusive_scan<int32_t>(before, s_warp, total);
+        before = total;
+    }
     const int64_t base = (int64_t)blockIdx.x * SCAN_ITEMS + (int64_t)threadIdx.x * SCAN_PER_THREAD;
-    int32_t v[SCAN_PER_THREAD];
+    int32_t v[SCAN_PER_THREAD], off[SCAN_PER_THREAD];
+    scan_load(g.cell_n, base, n, v);
     int32_t acc = 0;
 #pragma unroll
-    for (int k = 0; k < SCAN_PER_THREAD; ++k) {
-        v[k] = base + k < n ? in[base + k] : 0;
-        acc += v[k];
-    }
-    int32_t total;
-    int32_t run = block_exclusive_scan<int32_t>(acc, s_warp, total) + bsum[blockIdx.x];
+    for (int k = 0; k < SCAN_PER_THREAD; ++k) acc += v[k];
+    off[0] = block_exclusive_scan<int32_t>(acc, s_warp, total) + before;
 #pragma unroll
     for (int k = 0; k < SCAN_PER_THREAD; ++k) {
-        if (base + k < n) out[base + k] = run;
-        run += v[k];
+        if (k > 0) off[k] = off[k - 1] + v[k - 1];
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = bsum[nb];
-}
-
-cudaError_t scan_exclusive_i32(const int32_t* in, int32_t* out, int64_t n, void* tmp, cudaStream_t stream) {
-    const int64_t nb = (n + SCAN_ITEMS - 1) / SCAN_ITEMS;
-    int32_t* bsum = reinterpret_cast<int32_t*>(tmp);
-    if (nb == 0) {
-        return cudaMemsetAsync(out, 0, sizeof(int32_t), stream);
-    }
-    k_scan_partial<<<(unsigned)nb, SCAN_THREADS, 0, stream>>>(in, n, bsum);
-    k_scan_top<<<1, 1024, 0, stream>>>(bsum, nb);
-    k_scan_apply<<<(unsigned)nb, SCAN_THREADS, 0, stream>>>(in, out, n, bsum, nb);
-    return cudaGetLastError();
+    scan_store(g.cell_off, base, n, off);
+#pragma unroll
+    for (int k = 0; k < SCAN_PER_THREAD; ++k) v[k] = 0;
+    scan_store(g.cell_n, base, n, v);
+    if (blockIdx.x == nb - 1 && threadIdx.x == 0) g.cell_off[n] = before + total;
 }
 
 // ---------------------------------------------------------------------------
@@ -1299,9 +1369,39 @@ static unsigned grid_cap(int64_t work, int threads) {
     return (unsigned)gsz;
 }
 
-cudaError_t launch_geometry_plan(const psc_geometry& g, cudaStream_t stream) {
-    k_geometry_plan<<<1, 1024, 0, stream>>>(g);
-    return cudaGetLastError();
+// Calls launch(jobs, grid rows, first job) for runs of at most kGeoJobs consecutive windows that take the
+// same kernels (subsamples, smooth or not, velocity type).
+template <typename F>
+static cudaError_t by_geo_jobs(const GeoJob* jobs, int count, F launch) {
+    for (int k0 = 0; k0 < count;) {
+        GeoJobs a = {};
+        const GeoJob& f = jobs[k0];
+        int m = 0;
+        while (m < kGeoJobs && k0 + m < count && jobs[k0 + m].g.subsamples == f.g.subsamples &&
+               (jobs[k0 + m].g.smooth_eps > 0.0) == (f.g.smooth_eps > 0.0) && jobs[k0 + m].us_type == f.us_type) {
+            a.j[m] = jobs[k0 + m];
+            ++m;
+        }
+        launch(a, (unsigned)m, f);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+        k0 += m;
+    }
+    return cudaSuccess;
+}
+
+// The largest of the windows' own grids.
+template <typename F>
+static unsigned widest(const GeoJobs& a, unsigned m, F grid) {
+    unsigned g = 1;
+    for (unsigned k = 0; k < m; ++k) g = std::max(g, grid(a.j[k].g));
+    return g;
+}
+
+cudaError_t launch_geometry_plan(const GeoJob* jobs, int count, cudaStream_t stream) {
+    return by_geo_jobs(jobs, count, [&](const GeoJobs& a, unsigned m, const GeoJob&) {
+        k_geometry_plan<<<dim3(1, m), 1024, 0, stream>>>(a);
+    });
 }
 
 cudaError_t launch_copy_rows(const RowCopy* rows, int count, double* dst, cudaStream_t stream) {
@@ -1322,32 +1422,33 @@ cudaError_t launch_chunk_desc(const psc_geometry& g, double* desc, cudaStream_t 
     return cudaGetLastError();
 }
 
-cudaError_t launch_geometry_build(const psc_geometry& g, cudaStream_t stream, double* desc) {
-    const int64_t N = (int64_t)g.nx * g.ny * g.nz;
-    cudaError_t e = cudaMemsetAsync(g.cell_n, 0, (size_t)N * sizeof(int32_t), stream);
-    if (e != cudaSuccess) return e;
+cudaError_t launch_geometry_build(const GeoJob* jobs, int count, cudaStream_t stream) {
+    const auto cells = [](const psc_geometry& g) { return (int64_t)g.nx * g.ny * g.nz; };
     // a block per chunk: most particles own one small chunk (a grid of entries / 4096 blocks took the small
     // ones in turns: 21 us for the 1136 particles of a 64^3 window)
-    const int64_t full = g.capacity_entries / (g.chunk_entries > 0 ? g.chunk_entries : 4096);
-    const unsigned grid = grid_cap(g.capacity_chunks > full ? g.capacity_chunks : full, 1);
-    if (g.capacity_entries > 0) {
-        if (desc && (e = launch_chunk_desc(g, desc, stream)) != cudaSuccess) return e;
-        if (g.smooth_eps > 0.0) {
-            const unsigned parts = grid_cap(g.capacity_chunks * SMOOTH_PARTS, 1);
-            PSC_BY_SUBSAMPLES(g.subsamples, k_geometry_smooth, <<<parts, 256, 0, stream>>>(g, desc));
+    const auto chunks = [](const psc_geometry& g) {
+        return g.capacity_entries > 0 ? std::max(g.capacity_chunks, g.capacity_entries / g.chunk_entries) : 0;
+    };
+    return by_geo_jobs(jobs, count, [&](const GeoJobs& a, unsigned m, const GeoJob& f) {
+        const dim3 by_cell(widest(a, m, [&](const psc_geometry& g) { return grid_cap(cells(g), 256); }), m);
+        const dim3 by_chunk(widest(a, m, [&](const psc_geometry& g) { return grid_cap(chunks(g), 1); }), m);
+        const dim3 scan(widest(a, m, [&](const psc_geometry& g) { return (unsigned)((cells(g) + SCAN_ITEMS - 1) / SCAN_ITEMS); }),
+                        m);
+        k_geometry_begin<<<by_cell, 256, 0, stream>>>(a);
+        if (f.g.smooth_eps > 0.0) {
+            for (unsigned k = 0; k < m; ++k) {
+                const unsigned parts = grid_cap(chunks(a.j[k].g) * SMOOTH_PARTS, 1);
+                PSC_BY_SUBSAMPLES(f.g.subsamples, k_geometry_smooth, <<<parts, 256, 0, stream>>>(a.j[k].g, a.j[k].desc));
+            }
         } else {
-            PSC_BY_SUBSAMPLES(g.subsamples, k_geometry_count, <<<grid, 256, 0, stream>>>(g, desc));
+            PSC_BY_SUBSAMPLES(f.g.subsamples, k_geometry_count, <<<by_chunk, 256, 0, stream>>>(a));
         }
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    }
-    if ((e = scan_exclusive_i32(g.cell_n, g.cell_off, N, g.scan_tmp, stream)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(g.cell_n, 0, (size_t)N * sizeof(int32_t), stream)) != cudaSuccess) return e;
-    if (g.capacity_entries > 0) {
-        k_geometry_fill<<<grid, 256, 0, stream>>>(g, desc);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    }
-    k_geometry_final<<<grid_cap(N, 256), 256, 0, stream>>>(g);
-    return cudaGetLastError();
+        k_scan_partial<<<scan, SCAN_THREADS, 0, stream>>>(a);
+        if (scan.x > SCAN_DIRECT) k_scan_top<<<dim3(1, m), 1024, 0, stream>>>(a);
+        k_scan_apply<<<scan, SCAN_THREADS, 0, stream>>>(a);
+        k_geometry_fill<<<by_chunk, 256, 0, stream>>>(a);
+        k_geometry_final<<<by_cell, 256, 0, stream>>>(a);
+    });
 }
 
 cudaError_t read_loads_status(int* out, bool clear) {
@@ -1357,11 +1458,13 @@ cudaError_t read_loads_status(int* out, bool clear) {
     return cudaMemcpyToSymbol(g_loads_status, &zero, sizeof(int));
 }
 
-cudaError_t launch_solid_velocity(const psc_geometry& g, int us_type, void* us, cudaStream_t stream) {
-    const int64_t N = (int64_t)g.nx * g.ny * g.nz;
-    if (us_type == 0) k_solid_velocity<double><<<grid_cap(N, 256), 256, 0, stream>>>(g, reinterpret_cast<double*>(us));
-    else k_solid_velocity<float><<<grid_cap(N, 256), 256, 0, stream>>>(g, reinterpret_cast<float*>(us));
-    return cudaGetLastError();
+cudaError_t launch_solid_velocity(const GeoJob* jobs, int count, cudaStream_t stream) {
+    return by_geo_jobs(jobs, count, [&](const GeoJobs& a, unsigned m, const GeoJob& f) {
+        const dim3 by_cell(
+            widest(a, m, [&](const psc_geometry& g) { return grid_cap((int64_t)g.nx * g.ny * g.nz, 256); }), m);
+        if (f.us_type == 0) k_solid_velocity<double><<<by_cell, 256, 0, stream>>>(a);
+        else k_solid_velocity<float><<<by_cell, 256, 0, stream>>>(a);
+    });
 }
 
 // The chunk kernels hold a static staging ring and a dynamic count table of

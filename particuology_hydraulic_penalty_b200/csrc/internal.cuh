@@ -92,10 +92,21 @@ __device__ __forceinline__ void chain_wait() {
 cudaError_t launch_stream_pull_store(int store, double scale, const double* src, void* dst, int nx, int ny, int nz,
                                      cudaStream_t stream, bool open_x = false, const double* inlet = nullptr);
 
-cudaError_t launch_geometry_plan(const psc_geometry& g, cudaStream_t stream);
-// desc: room for the geometry's load-chunk descriptors (launch_chunk_desc), written here, or null.
-cudaError_t launch_geometry_build(const psc_geometry& g, cudaStream_t stream, double* desc = nullptr);
-cudaError_t launch_solid_velocity(const psc_geometry& g, int us_type, void* us, cudaStream_t stream);
+// One window of a rebuild: its geometry, room for its load-chunk descriptors (launch_chunk_desc; written by the
+// build) or null, page-locked room for its entry and chunk totals (written by the plan) or null, and
+// the solid velocity [3][N] (us_type 0 = float64, 1 = float32).
+struct GeoJob {
+    psc_geometry g;
+    double* desc;
+    int64_t* host_totals;
+    void* us;
+    int32_t us_type;
+};
+constexpr int kGeoJobs = 12;  // kernel parameters of 4 KB
+static_assert(kGeoJobs * sizeof(GeoJob) <= 4000, "kernel parameters");
+cudaError_t launch_geometry_plan(const GeoJob* jobs, int count, cudaStream_t stream);
+cudaError_t launch_geometry_build(const GeoJob* jobs, int count, cudaStream_t stream);
+cudaError_t launch_solid_velocity(const GeoJob* jobs, int count, cudaStream_t stream);
 // desc: the chunk descriptors of this geometry (launch_chunk_desc), or null: made on every call in the
 // chunks' partial rows.  host_diag: page-locked copy of diag, or null.
 cudaError_t launch_particle_loads(const psc_geometry& g, int imb_type, const void* imb, double* chunk_partials,

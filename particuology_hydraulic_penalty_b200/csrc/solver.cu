@@ -516,20 +516,23 @@ int window_set_particles(Window& w, const double* hp, int P, cudaStream_t s, con
 
 // A geometry rebuild in two halves, so that a batch reads the entry and chunk
 // counts of all its windows after one synchronisation: the plan (bounding
-// boxes, entry and chunk offsets, totals) with the totals copied into the
-// pinned slot tot4[0..3], then, once the copy has landed, the buffers grown
-// to the counts and the build enqueued.
-int window_rebuild_plan(Window& w, cudaStream_t s, int64_t* tot4, const char* who) {
-    psc_geometry g = w.geometry();
-    w.built = false;  // the plan overwrites the current geometry's offsets
-    PSC_TRY(psc_geometry_plan(&g, s));
-    PSC_CUDA(cudaMemcpyAsync(tot4, w.totals.p, 4 * sizeof(int64_t), cudaMemcpyDeviceToHost, s), who);
+// boxes, entry and chunk offsets, totals), which writes window k's entry and
+// chunk totals into the pinned slot tot[k][0..1], then, once it has ended, the
+// buffers grown to the counts and the build enqueued.
+int windows_plan(Window* const* w, int64_t* const* tot, int count, cudaStream_t s, const char* who) {
+    std::vector<GeoJob> jobs((size_t)count);
+    for (int k = 0; k < count; ++k) {
+        jobs[(size_t)k] = {w[k]->geometry(), nullptr, tot[k]};
+        w[k]->built = false;  // the plan overwrites the current geometry's offsets
+    }
+    PSC_CUDA(launch_geometry_plan(jobs.data(), count, s), who);
     return PSC_OK;
 }
 
-int window_rebuild_finish(Window& w, cudaStream_t s, const int64_t* tot4, const char* who) {
-    w.n_entries = tot4[0];
-    w.n_chunks = tot4[1];
+// Room for the planned geometry.
+int window_rebuild_room(Window& w, cudaStream_t s, const int64_t* tot, const char* who) {
+    w.n_entries = tot[0];
+    w.n_chunks = tot[1];
     if (w.n_entries >= (1ll << 31) - 1)
         return fail(PSC_E_CAPACITY, std::string(who) + ": too many bounding-box entries (>= 2^31) for one window");
     if (w.n_entries > w.cap_entries) {
@@ -554,31 +557,54 @@ int window_rebuild_finish(Window& w, cudaStream_t s, const int64_t* tot4, const 
         }
         w.cap_chunks = cap;
     }
-    const psc_geometry g = w.geometry();
-    PSC_CUDA(launch_geometry_build(g, s, w.cap_chunks > 0 ? w.chunk_desc.p : nullptr), who);
-    w.built = true;
-    ++w.builds;
-    w.built_version = w.pversion;
-    w.list_version = 0;
-    w.desc_built = w.cap_entries > 0 && w.cap_chunks > 0 ? w.built_version : 0;  // (made with the build)
-    w.us_version = 0;
-    w.loads_ready = false;
-    w.diag_ready = false;
+    return PSC_OK;
+}
+
+int window_velocity_room(Window& w, cudaStream_t s) {
+    if (w.us.p) return PSC_OK;
+    PSC_CUDA(w.us.ensure(3 * w.N * (int64_t)w.field_bytes(), true, s), "solid velocity");
+    w.touch();
+    return PSC_OK;
+}
+
+// The windows' planned geometries (window_rebuild_room each), and the solid velocity of those that move and ask
+// for it.
+int windows_build(Window* const* w, int count, cudaStream_t s, const char* who, bool velocity) {
+    std::vector<GeoJob> jobs((size_t)count);
+    for (int k = 0; k < count; ++k) jobs[(size_t)k] = {w[k]->geometry(), w[k]->cap_chunks > 0 ? w[k]->chunk_desc.p : nullptr};
+    PSC_CUDA(launch_geometry_build(jobs.data(), count, s), who);
+    std::vector<GeoJob> move;
+    for (int k = 0; k < count; ++k) {
+        Window& x = *w[k];
+        x.built = true;
+        ++x.builds;
+        x.built_version = x.pversion;
+        x.list_version = 0;
+        x.desc_built = jobs[(size_t)k].desc ? x.built_version : 0;  // (made with the build)
+        x.us_version = 0;
+        x.loads_ready = false;
+        x.diag_ready = false;
+        if (!velocity || !x.moving) continue;
+        PSC_TRY(window_velocity_room(x, s));
+        move.push_back({x.geometry(), nullptr, nullptr, x.us.p, x.field_type()});
+        x.us_version = x.pversion;
+    }
+    PSC_CUDA(launch_solid_velocity(move.data(), (int)move.size(), s), who);
     return PSC_OK;
 }
 
 int window_rebuild(Window& w, cudaStream_t s, HArray<int64_t>& tot, const char* who) {
     PSC_CUDA(tot.ensure(4), who);
-    PSC_TRY(window_rebuild_plan(w, s, tot.p, who));
+    Window* one = &w;
+    int64_t* at = tot.p;
+    PSC_TRY(windows_plan(&one, &at, 1, s, who));
     PSC_CUDA(cudaStreamSynchronize(s), who);
-    return window_rebuild_finish(w, s, tot.p, who);
+    PSC_TRY(window_rebuild_room(w, s, tot.p, who));
+    return windows_build(&one, 1, s, who, false);
 }
 
 int window_solid_velocity(Window& w, cudaStream_t s) {
-    if (!w.us.p) {
-        PSC_CUDA(w.us.ensure(3 * w.N * (int64_t)w.field_bytes(), true, s), "solid velocity");
-        w.touch();
-    }
+    PSC_TRY(window_velocity_room(w, s));
     psc_geometry g = w.geometry();
     PSC_TRY(psc_solid_velocity(&g, w.field_type(), w.us.p, s));
     w.us_version = w.pversion;
@@ -1522,7 +1548,6 @@ struct psc_batch {
     std::vector<uint64_t> built_desc;  // descriptor versions the tables were built from
     bool moving_any = false;
     Lanes lanes;  // particle loads of the windows beside the post-stream reduction pass
-    Lanes build_lanes;  // geometry rebuilds of the windows beside one another
     HArray<double> up_host;    // every window's particles, staged for one upload
     DArray<double> up_dev;
     // The upload runs on its own stream beside the step kernels, which do not
@@ -1777,26 +1802,16 @@ int batch_prepare(psc_batch& b, bool imb, bool moments) {
     if (!plan.empty()) {
         PSC_TRY(batch_upload_join(b, who));
         PSC_CUDA(b.tot.ensure(4 * (int64_t)b.w.size()), who);
-        // one window's kernels are too small for the GPU: the windows' chains run beside one another, the
-        // solid velocity of a moving window at its end (6 moving windows of 64^3, a
-        // call of two steps: 1.09 ms one after the other, 0.93 ms on four streams)
-        Lanes& lanes = b.build_lanes;
-        PSC_CUDA(lanes.begin(b.stream), who);
-        int st = PSC_OK;
-        for (size_t i = 0; i < plan.size() && st == PSC_OK; ++i)
-            st = window_rebuild_plan(*b.w[plan[i]], lanes.lane((int)i), b.tot.p + 4 * plan[i], who);
-        for (int i = 0; i < lanes.n; ++i) {  // (also after a failure: no lane reads what a later call changes)
-            const cudaError_t e = cudaStreamSynchronize(lanes.s[i]);
-            if (st == PSC_OK && e != cudaSuccess) st = cuda_fail(e, who);
+        std::vector<Window*> w;
+        std::vector<int64_t*> tot;
+        for (size_t k : plan) {
+            w.push_back(b.w[k].get());
+            tot.push_back(b.tot.p + 4 * k);
         }
-        for (size_t i = 0; i < plan.size() && st == PSC_OK; ++i) {
-            Window& w = *b.w[plan[i]];
-            st = window_rebuild_finish(w, lanes.lane((int)i), b.tot.p + 4 * plan[i], who);
-            if (st == PSC_OK && window_needs_solid_velocity(w)) st = window_solid_velocity(w, lanes.lane((int)i));
-        }
-        const cudaError_t e = lanes.end(b.stream);
-        if (st != PSC_OK) return st;
-        PSC_CUDA(e, who);
+        PSC_TRY(windows_plan(w.data(), tot.data(), (int)w.size(), b.stream, who));
+        PSC_CUDA(cudaStreamSynchronize(b.stream), who);
+        for (size_t i = 0; i < w.size(); ++i) PSC_TRY(window_rebuild_room(*w[i], b.stream, tot[i], who));
+        PSC_TRY(windows_build(w.data(), (int)w.size(), b.stream, who, true));
     }
     for (size_t k = 0; k < b.w.size(); ++k) {
         Window& w = *b.w[k];
@@ -1958,7 +1973,6 @@ int psc_batch_create(const psc_config* h_cfgs, int nwin, const psc_launch* h_lau
         if (e == cudaSuccess) e = b->diag.ensure((int64_t)nwin * PSC_NDIAG, true, b->stream);
         if (e == cudaSuccess) e = b->host.ensure((int64_t)nwin * kOutLen);
         if (e == cudaSuccess) e = b->lanes.init(1);
-        if (e == cudaSuccess) e = b->build_lanes.init(Lanes::kMax);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->up_done, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->up_ready, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->up_stream, cudaStreamNonBlocking);
