@@ -75,7 +75,7 @@ __device__ __forceinline__ T block_exclusive_scan(T v, T* s_warp, T& total) {
 // The kernels of a rebuild take up to kGeoJobs windows, one per row of the grid (blockIdx.y): one window's
 // kernels are too small for the GPU and a window took eleven launches and three copies of its own (two steps
 // of six moving 64^3 windows, rebuilt every call: 0.69 ms with the windows' launches on four streams,
-// 0.58 ms so).
+// 0.55 ms so).
 struct GeoJobs {
     GeoJob j[kGeoJobs];
 };

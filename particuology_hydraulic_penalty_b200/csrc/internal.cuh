@@ -134,7 +134,7 @@ struct LoadsJob {
     double* diag;             // [PSC_NDIAG]
     double* host_diag;        // page-locked copy of diag, or null
 };
-// Particle loads and load diagnostics of njobs windows in four launches.
+// Particle loads and load diagnostics of njobs windows, one launch per stage for all of them.
 // d_chunk_base / d_particle_base: [njobs + 1] exclusive prefix sums of the
 // jobs' chunk and particle counts (the totals are their last entries, also
 // passed by value); part: total_chunks rows of 6 doubles.  all_lists: every

@@ -90,8 +90,8 @@ __device__ __noinline__ void bb_cell_general(const BbArgs& a, uint32_t N, uint32
 }
 
 // One cell per thread of a grid-stride loop, two CTAs per SM (128 registers): bound by the FP64 pipe
-// like k_step_exact, whose branch-free forms it shares (64^3: 32.5 us a step with a branch per division, 15.2 without, 13.4 in a
-// chain of steps).
+// like k_step_exact, whose branch-free forms it shares (64^3: 32.5 us a step with a branch per division,
+// 15.0 without, in a chain of steps).
 __global__ void __launch_bounds__(256, 2) k_bb_step(const __grid_constant__ BbArgs a) {
     __shared__ ExactWin w;
     __shared__ const double* s_src;
