@@ -70,10 +70,11 @@ __global__ void __launch_bounds__(STEP_THREADS, (PairOccupancy<STORE, MOVING, RE
     using T = typename TR::T;
     using R = typename TR::R;
     using O = typename TR::O;
-    // Both cells in packed FP32 where the arithmetic bounds the kernel: 16-bit storage (160^3: 90 -> 82 us
-    // plain, 107 -> 99 with IMB and sums; 378 -> 261 instructions per cell).  FP32 storage is bound by HBM,
-    // and there the packed form was slower (114 against 108 us: its shorter bursts of arithmetic leave
-    // reads and writes less spread).  FP64 has no packed form.
+    // Both cells in packed FP32 where the arithmetic weighs: 16-bit storage (FP16 160^3 90 -> 82 us plain and
+    // 107 -> 99 with IMB and sums, 78 and 95 in a chain of steps; 311 and 394 instructions per cell).  FP32
+    // storage is bound by HBM, and there the packed form was slower (114 against 108 us, although at 261
+    // instructions per cell instead of 378: its shorter bursts of arithmetic leave reads and writes less
+    // spread).  FP64 has no packed form.
     constexpr bool PACKED = sizeof(T) == 2;
     using V = std::conditional_t<PACKED, F2, R>;
     __shared__ FastWin<T, R, O, V> sw;
