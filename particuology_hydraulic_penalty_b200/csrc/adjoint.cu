@@ -140,7 +140,6 @@ __global__ void k_adjoint_seed(psc_adjoint_args a) {
 //   mu_i = (1 - kb - B) l_i + B l_j + d/d(rho - 1) + c . d/dm.
 template <typename V>
 struct AdjointConst {
-    const void *state, *lam;
     V inv_tau, fx, fy, fz, pref3;  // pref3 = 3 pref
     V K9[9];                       // 9 pref w_k (c_k . F)
 };
@@ -259,14 +258,10 @@ __global__ void __launch_bounds__(256) k_adjoint_step(const __grid_constant__ ps
     __shared__ AdjointConst<R> c;
     if (threadIdx.x == 0) make_adjoint_const(c, a);
     chain_wait();
-    if (threadIdx.x == 0) {
-        c.state = a.state;
-        c.lam = a.lam_in;
-    }
     __syncthreads();
     const uint32_t N = (uint32_t)a.nx * a.ny * a.nz;
-    const R* S = reinterpret_cast<const R*>(c.state);
-    const R* lin = reinterpret_cast<const R*>(c.lam);
+    const R* S = reinterpret_cast<const R*>(a.state);
+    const R* lin = reinterpret_cast<const R*>(a.lam_in);
     R* lout = reinterpret_cast<R*>(a.lam_out);
     const uint32_t stride = gridDim.x * blockDim.x;
     StrideWalk at(blockIdx.x * blockDim.x + threadIdx.x, stride, a.nx, a.ny, a.nz);
@@ -296,14 +291,10 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_CTAS) k_adjoint_pair(const __
     __shared__ AdjointConst<F2> c;
     if (threadIdx.x == 0) make_adjoint_const(c, a);
     chain_wait();
-    if (threadIdx.x == 0) {
-        c.state = a.state;
-        c.lam = a.lam_in;
-    }
     __syncthreads();
     const uint32_t N = (uint32_t)a.nx * a.ny * a.nz, nz = (uint32_t)a.nz;
-    const float* S = reinterpret_cast<const float*>(c.state);
-    const float* lin = reinterpret_cast<const float*>(c.lam);
+    const float* S = reinterpret_cast<const float*>(a.state);
+    const float* lin = reinterpret_cast<const float*>(a.lam_in);
     float* lout = reinterpret_cast<float*>(a.lam_out);
     const float tau = (float)a.tau;
     const uint32_t stride = 2 * gridDim.x * blockDim.x;
@@ -322,15 +313,17 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_CTAS) k_adjoint_pair(const __
             const int32_t oxy = (cxv(i) == 1 ? xm : (cxv(i) == -1 ? xp : 0)) + (cyv(i) == 1 ? ym : (cyv(i) == -1 ? yp : 0));
             const float* p = S + (size_t)i * N + (size_t)((int64_t)c0 + oxy);
             if (czv(i) == 0) {
-                const float2 v = __ldg(reinterpret_cast<const float2*>(p));
-                g[i] = f2(v.x, v.y);
+                float x, y;
+                ld_pair(p, x, y);
+                g[i] = f2(x, y);
             } else if (czv(i) == 1) {
                 g[i] = f2(ld_pop(p + zm0), ld_pop(p));
             } else {
                 g[i] = f2(ld_pop(p + 1), ld_pop(p + zp1));
             }
-            const float2 l = __ldg(reinterpret_cast<const float2*>(lin + (size_t)i * N + c0));
-            lam[i] = f2(l.x, l.y);
+            float l0, l1;
+            ld_pair(lin + (size_t)i * N + c0, l0, l1);
+            lam[i] = f2(l0, l1);
         }
         const double2 solid = *reinterpret_cast<const double2*>(a.solid + c0);
         const F2 drho = sum_populations(g);

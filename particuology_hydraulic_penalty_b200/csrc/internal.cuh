@@ -63,8 +63,8 @@ cudaError_t launch_stream_push(int store, double scale, const void* src, double*
 // A launch that may start before the kernel ahead of it on its stream has ended (chained): its CTAs take the
 // SMs as they fall free and set up what that kernel does not write; then every CTA waits (chain_wait) before
 // it touches anything else, and lets its own successor in only then, so at most two kernels
-// of a stream overlap.  A pointer that is read through the read-only path after the wait goes through
-// shared memory, so that no such load is moved above it.  A step in a row of steps: 64^3 FP32 8.9 -> 7.7 us,
+// of a stream overlap.  What the kernel ahead writes is read after the wait by ordinary loads only: the
+// read-only path (ld.global.nc, const __restrict__) is for data that nothing in the chain writes.  A step in a row of steps: 64^3 FP32 8.9 -> 7.7 us,
 // 75^3 FP32 12.0 -> 10.5, 24^3 exact 4.65 -> 3.86, 96^3 exact 55.8 -> 54.1 us.
 template <typename... P, typename... A>
 inline cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream,

@@ -62,8 +62,7 @@ __device__ void converge_check(const ConvergeCheck& cc, const double* post) {
 
 template <bool CONV>
 __global__ void __cluster_dims__(REDUCE_CTAS, 1, 1) __launch_bounds__(REDUCE_THREADS)
-    k_reduce_windows(const psc_window* __restrict__ wins, double* __restrict__ out, double* __restrict__ out2,
-                     const __grid_constant__ ConvergeCheck cc) {
+    k_reduce_windows(const psc_window* wins, double* out, double* out2, const __grid_constant__ ConvergeCheck cc) {
     namespace cg = cooperative_groups;
     chain_wait();
     __shared__ double s_g[REDUCE_GROUPS * PSC_NRED];

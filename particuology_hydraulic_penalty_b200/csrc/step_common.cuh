@@ -49,17 +49,51 @@ struct StoreTraits<PSC_STORE_BF16> {
     static constexpr bool scaled = true;
 };
 
-__device__ __forceinline__ double ld_pop(const double* p) { return __ldg(p); }
-// FP32 pulls ask L2 to fetch the whole 256-byte line pair: consecutive tiles of
-// a CTA read consecutive rows, so the neighbouring sectors are used next
-// (measured +1.3 % on the 24-window batch).
-__device__ __forceinline__ float ld_pop(const float* p) {
-    float v;
-    asm volatile("ld.global.nc.L2::256B.f32 %0, [%1];" : "=f"(v) : "l"(p));
+// Population loads are ordinary (coherent) ones: a chained kernel (launch_chained) is resident while the kernel
+// ahead of it still writes them, and read-only (.nc) loads are defined only for data that nobody writes
+// while the kernel lives.  asm volatile keeps them behind chain_wait.  FP32 pulls ask L2 for the whole 256-byte line pair.
+__device__ __forceinline__ double ld_pop(const double* p) {
+    double v;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
     return v;
 }
-__device__ __forceinline__ float ld_pop(const __half* p) { return __half2float(__ldg(p)); }
-__device__ __forceinline__ float ld_pop(const __nv_bfloat16* p) { return __bfloat162float(__ldg(p)); }
+__device__ __forceinline__ float ld_pop(const float* p) {
+    float v;
+    asm volatile("ld.global.L2::256B.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float ld_pop(const __half* p) {
+    __half_raw v;
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(v.x) : "l"(p));
+    return __half2float(v);
+}
+__device__ __forceinline__ float ld_pop(const __nv_bfloat16* p) {
+    __nv_bfloat16_raw v;
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(v.x) : "l"(p));
+    return __bfloat162float(v);
+}
+
+// The same of two consecutive populations (p aligned to both).
+__device__ __forceinline__ void ld_pair(const float* p, float& a, float& b) {
+    asm volatile("ld.global.L2::256B.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "l"(p));
+}
+__device__ __forceinline__ void ld_pair(const double* p, double& a, double& b) {
+    asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(a), "=d"(b) : "l"(p));
+}
+__device__ __forceinline__ void ld_pair(const __half* p, float& a, float& b) {
+    __half2_raw r;
+    asm volatile("ld.global.v2.u16 {%0, %1}, [%2];" : "=h"(r.x), "=h"(r.y) : "l"(p));
+    const float2 v = __half22float2(r);
+    a = v.x;
+    b = v.y;
+}
+__device__ __forceinline__ void ld_pair(const __nv_bfloat16* p, float& a, float& b) {
+    __nv_bfloat162_raw r;
+    asm volatile("ld.global.v2.u16 {%0, %1}, [%2];" : "=h"(r.x), "=h"(r.y) : "l"(p));
+    const float2 v = __bfloat1622float2(r);
+    a = v.x;
+    b = v.y;
+}
 
 template <typename R>
 __device__ __forceinline__ R fast_rcp(R x);

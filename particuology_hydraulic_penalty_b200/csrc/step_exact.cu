@@ -150,7 +150,7 @@ __device__ __noinline__ void exact_cell_general(const ExactShared& s, uint32_t c
 // cp.async took another 1 to 4 %, at one more kernel per variant: not used.
 template <bool MOVING, bool RED>
 __global__ void __launch_bounds__(STEP_THREADS, 2)
-    k_step_exact(const psc_window* __restrict__ wins, int nwin, unsigned flags, const __grid_constant__ TilePlan plan) {
+    k_step_exact(const psc_window* wins, int nwin, unsigned flags, const __grid_constant__ TilePlan plan) {
     __shared__ ExactShared sw;
     __shared__ double s_red[RED ? PSC_NRED : 1][STEP_THREADS];  // running sums per thread (in registers they would spill)
     static_assert(STEP_THREADS / 32 == PSC_PARTIAL_ROWS, "one partial row per warp");

@@ -23,25 +23,6 @@ __device__ int g_pair_status = 0;
 
 constexpr int PAIR_CELLS = 2;
 
-__device__ __forceinline__ void ld_pair(const float* p, float& a, float& b) {
-    asm volatile("ld.global.nc.L2::256B.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "l"(p));
-}
-__device__ __forceinline__ void ld_pair(const double* p, double& a, double& b) {
-    const double2 v = __ldg(reinterpret_cast<const double2*>(p));
-    a = v.x;
-    b = v.y;
-}
-__device__ __forceinline__ void ld_pair(const __half* p, float& a, float& b) {
-    const float2 v = __half22float2(__ldg(reinterpret_cast<const __half2*>(p)));
-    a = v.x;
-    b = v.y;
-}
-__device__ __forceinline__ void ld_pair(const __nv_bfloat16* p, float& a, float& b) {
-    const float2 v = __bfloat1622float2(__ldg(reinterpret_cast<const __nv_bfloat162*>(p)));
-    a = v.x;
-    b = v.y;
-}
-
 __device__ __forceinline__ void st_pair(float* p, float a, float b) {
     *reinterpret_cast<float2*>(p) = make_float2(a, b);
 }

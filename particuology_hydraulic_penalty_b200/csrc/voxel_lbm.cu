@@ -94,12 +94,9 @@ __device__ __noinline__ void bb_cell_general(const BbArgs& a, uint32_t N, uint32
 // 15.0 without, in a chain of steps).
 __global__ void __launch_bounds__(256, 2) k_bb_step(const __grid_constant__ BbArgs a) {
     __shared__ ExactWin w;
-    __shared__ const double* s_src;
     make_exact_win_block(w, a.tau, a.fx, a.fy, a.fz);
     chain_wait();
-    if (threadIdx.x == 0) s_src = a.src;
     __syncthreads();
-    const double* src = s_src;
     const uint32_t N = (uint32_t)a.nx * a.ny * a.nz;
     const bool do_collide = a.flags & PSC_STEP_COLLIDE;
     const bool do_mom = a.flags & PSC_STEP_MOMENTS;
@@ -111,7 +108,7 @@ __global__ void __launch_bounds__(256, 2) k_bb_step(const __grid_constant__ BbAr
     for (; cell < N; cell += stride) {
         const NbrOffsets o = nbr_offsets(ix, iy, iz, a.nx, a.ny, a.nz);
         double f[Q];
-        bb_pull(src, N, cell, o, f);
+        bb_pull(a.src, N, cell, o, f);
         const bool s = a.solid[cell] != 0;
         if (s) bounce_solid_as_reference(f);
         const ExactMomentsS mo = moments_exact_s(f, w.hfx, w.hfy, w.hfz);
