@@ -319,6 +319,7 @@ struct ExactMomentsS {
     bool out;
 };
 
+// .out: the populations or rho left the range; F / 2 is ExactWin.out's to test.
 PSC_HD ExactMomentsS moments_exact_s(const double* f, double hfx, double hfy, double hfz) {
     ExactMomentsS m;
     double rho = f[0];

@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(STEP_THREADS, 2)
         if (sw.open_x && at.ix == 0) exact_inlet(sw, cell, f);
         exact_advance(sw, at);
         ExactMomentsS mo = moments_exact_s(f, sw.c.hfx, sw.c.hfy, sw.c.hfz);
-        bool out = mo.out;
+        bool out = mo.out | (sw.c.out != 0);  // (the moments divide m + F / 2)
         if (do_collide) {
             bool moves = false;
             double usx = 0.0, usy = 0.0, usz = 0.0;

@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(256, 2) k_bb_step(const __grid_constant__ BbAr
         if (s) bounce_solid_as_reference(f);
         const ExactMomentsS mo = moments_exact_s(f, w.hfx, w.hfy, w.hfz);
         double m[4] = {mo.rho, s ? 0.0 : mo.ux, s ? 0.0 : mo.uy, s ? 0.0 : mo.uz};
-        bool out = mo.out;
+        bool out = mo.out | (w.out != 0);  // (the moments divide m + F / 2)
         if (do_collide) out = w.axis >= 0 ? collide_bb_exact_s<true>(f, mo, s, w) : collide_bb_exact_s<false>(f, mo, s, w);
         if (out) {
             BbCell g;
