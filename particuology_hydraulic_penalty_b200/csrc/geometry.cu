@@ -1022,7 +1022,8 @@ __device__ __forceinline__ void loads_diag_block(int P, const double* imb_sums, 
 // 3.2 + 5.4 us with 1136).  Eight lanes add a particle's chunks c0 + l, c0 + l + 8, ... in order and
 // then by a shuffle tree: most particles own one chunk, the largest of a packed window some forty
 // (a warp per particle took 14 us with 1136).  For windows of up to FINAL_PARTICLES particles: beyond,
-// one cluster takes more turns than the whole GPU.
+// one cluster takes more turns than the whole GPU.  The window's own count decides, alone or among others:
+// the order of a particle's sum, and so its bits, do not depend on the launch it is made in.
 constexpr int FINAL_CTAS = 8;
 constexpr int FINAL_THREADS = 512;
 constexpr int FINAL_LANES = 8;
@@ -1211,6 +1212,7 @@ __global__ void __launch_bounds__(256) k_loads_particles_multi(const LoadsJob* j
     if (gp >= particle_base[njobs]) return;  // warp-uniform
     const int k = owner_of(particle_base, njobs, gp);
     const LoadsJob& J = jobs[k];
+    if (J.g.nparticles <= FINAL_PARTICLES) return;  // (k_loads_final_multi's)
     const int p = (int)(gp - particle_base[k]);
     particle_sums(part + chunk_base[k] * 6, J.g.chunk_off[p], J.g.chunk_off[p + 1], J.forces + (size_t)p * 3,
                   J.torques + (size_t)p * 3);
@@ -1218,6 +1220,7 @@ __global__ void __launch_bounds__(256) k_loads_particles_multi(const LoadsJob* j
 
 __global__ void __launch_bounds__(1024) k_loads_diag_multi(const LoadsJob* jobs) {
     const LoadsJob& J = jobs[blockIdx.x];
+    if (J.g.nparticles <= FINAL_PARTICLES) return;
     loads_diag_block(J.g.nparticles, J.imb_sums, J.forces, J.torques, J.diag, J.host_diag);
 }
 
@@ -1226,6 +1229,7 @@ __global__ void __cluster_dims__(FINAL_CTAS, 1, 1) __launch_bounds__(FINAL_THREA
     chain_wait();
     const int k = blockIdx.x / FINAL_CTAS;
     const LoadsJob& J = jobs[k];
+    if (J.g.nparticles > FINAL_PARTICLES) return;  // the whole cluster
     loads_final_cluster(J.g.nparticles, J.g.chunk_off, part + chunk_base[k] * 6, J.imb_sums, J.forces, J.torques, J.diag,
                         J.host_diag);
 }
@@ -1566,15 +1570,12 @@ cudaError_t launch_particle_loads_multi(const LoadsJob* d_jobs, const int64_t* d
             k_loads_chunks_multi<float><<<grid, LOAD_THREADS, lut, stream>>>(d_jobs, d_chunk_base, njobs, desc, part);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    if (max_particles <= FINAL_PARTICLES) {
-        return launch_chained(k_loads_final_multi, (unsigned)(njobs * FINAL_CTAS), FINAL_THREADS, 0, stream, true, d_jobs,
-                              d_chunk_base, part);
-    }
-    if (total_particles > 0) {
-        k_loads_particles_multi<<<(unsigned)((total_particles + 7) / 8), 256, 0, stream>>>(
-            d_jobs, d_chunk_base, d_particle_base, njobs, part);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    }
+    e = launch_chained(k_loads_final_multi, (unsigned)(njobs * FINAL_CTAS), FINAL_THREADS, 0, stream, true, d_jobs,
+                       d_chunk_base, part);
+    if (e != cudaSuccess || max_particles <= FINAL_PARTICLES) return e;
+    k_loads_particles_multi<<<(unsigned)((total_particles + 7) / 8), 256, 0, stream>>>(d_jobs, d_chunk_base,
+                                                                                       d_particle_base, njobs, part);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     k_loads_diag_multi<<<(unsigned)njobs, 1024, 0, stream>>>(d_jobs);
     return cudaGetLastError();
 }
