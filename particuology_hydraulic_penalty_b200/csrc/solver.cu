@@ -729,18 +729,33 @@ void fill_diag(const Window& w, const double* host_out, psc_diag& d) {
 // with four threads, which cost the smaller ones 0.1 ms).  Doubles of more than one piece go straight into
 // the caller's memory, where the driver does the same: 128^3 1.17 ms against 1.34 here; one piece goes
 // through the ring (24^3 41 -> 33 us).  ring: page-locked memory of the caller's handle, grown to
-// kRingPiece * kRingPieces bytes at most.
+// kRingPiece * kRingPieces bytes at most; where there is none to be had, floats cross into the upper half of
+// dst and are converted in place.
 constexpr int64_t kRingPiece = 256 << 10, kRingPieces = 8;
+
+// Whether the page-locked array holds n elements now; a failed allocation leaves no error behind.
+template <class T>
+bool pinned_room(HArray<T>& a, int64_t n) {
+    if (a.ensure(n) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
+
 int values_to_host(const void* src, bool f64, int64_t count, double* dst, cudaStream_t s, HArray<int64_t>& ring,
                    const char* who) {
     const int64_t el = f64 ? 8 : 4, piece = kRingPiece / el, n = (count + piece - 1) / piece;
-    if (f64 && n > 1) {
-        PSC_CUDA(cudaMemcpyAsync(dst, src, (size_t)count * 8, cudaMemcpyDeviceToHost, s), who);
+    const int64_t slots = std::min(n, kRingPieces);
+    if ((f64 && n > 1) || !pinned_room(ring, n > 1 ? slots * kRingPiece / 8 : (count * el + 7) / 8)) {
+        unsigned char* at = reinterpret_cast<unsigned char*>(dst) + (f64 ? 0 : count * 4);
+        PSC_CUDA(cudaMemcpyAsync(at, src, (size_t)(count * el), cudaMemcpyDeviceToHost, s), who);
         PSC_CUDA(cudaStreamSynchronize(s), who);
+        for (int64_t i = 0; !f64 && i < count; ++i) {  // (value i lies at or beyond the end of dst[i - 1])
+            float v;
+            std::memcpy(&v, at + i * 4, sizeof(v));
+            dst[i] = (double)v;
+        }
         return PSC_OK;
     }
-    const int64_t slots = std::min(n, kRingPieces);
-    PSC_CUDA(ring.ensure(n > 1 ? slots * kRingPiece / 8 : (count * el + 7) / 8), who);
     unsigned char* mem = reinterpret_cast<unsigned char*>(ring.p);
     cudaEvent_t ev[kRingPieces] = {};
     cudaError_t e = cudaSuccess;
@@ -783,11 +798,10 @@ int field_to_host(const Window& w, const void* src, int64_t count, double* dst, 
 int window_loads_to_host(const Window& w, double* forces, double* torques, cudaStream_t s, HArray<int64_t>& ring,
                          const char* who) {
     const int64_t n = 3 * (int64_t)w.P;
-    if (2 * n * 8 > kRingPiece * kRingPieces) {
+    if (2 * n * 8 > kRingPiece * kRingPieces || !pinned_room(ring, 2 * n)) {
         PSC_TRY(values_to_host(w.forces.p, true, n, forces, s, ring, who));
         return values_to_host(w.torques.p, true, n, torques, s, ring, who);
     }
-    PSC_CUDA(ring.ensure(2 * n), who);
     double* mem = reinterpret_cast<double*>(ring.p);
     PSC_CUDA(cudaMemcpyAsync(mem, w.forces.p, (size_t)n * 8, cudaMemcpyDeviceToHost, s), who);
     PSC_CUDA(cudaMemcpyAsync(mem + n, w.torques.p, (size_t)n * 8, cudaMemcpyDeviceToHost, s), who);
@@ -1679,9 +1693,12 @@ int batch_fetch_loads(psc_batch& b, const char* who) {
         rows.push_back({w.torques.p, total + n, n});
         total += 2 * n;
     }
-    PSC_CUDA(b.loads_host.ensure(total), who);
-    PSC_CUDA(launch_copy_rows(rows.data(), (int)rows.size(), b.loads_host.p, b.stream), who);
-    PSC_CUDA(cudaStreamSynchronize(b.stream), who);
+    if (pinned_room(b.loads_host, total)) {
+        PSC_CUDA(launch_copy_rows(rows.data(), (int)rows.size(), b.loads_host.p, b.stream), who);
+        PSC_CUDA(cudaStreamSynchronize(b.stream), who);
+    } else {  // each window's on its own
+        at.assign(b.w.size(), -1);
+    }
     b.loads_at.swap(at);
     return PSC_OK;
 }
