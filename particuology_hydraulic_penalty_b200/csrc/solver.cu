@@ -1583,11 +1583,11 @@ struct psc_batch {
     DArray<double> loads_part;  // chunk partials of all jobs
     DArray<double> loads_desc;  // chunk descriptors of all jobs, of the geometries in desc_built
     std::vector<uint64_t> desc_built;
-    // loads of the last reporting step as the host read them: where each window's lie (-1: not there), empty
-    // until a second window (after loads_first) is asked for
+    // loads of the last reporting step on the host (batch_fetch_loads): where each window's lie (-1: not there;
+    // empty: none read since the step), and how many windows the next transfer brings (0: no more of them)
     HArray<double> loads_host;
     std::vector<int64_t> loads_at;
-    int loads_first = -1;
+    size_t loads_take = 1;
     int jobs_n = 0, jobs_max_s = 1, jobs_max_p = 0;
     int64_t jobs_chunks = 0, jobs_particles = 0;
     bool jobs_list_ready = false;  // every job's loads list is current
@@ -1678,13 +1678,22 @@ std::vector<uint64_t> batch_geometries(const psc_batch& b) {
     return v;
 }
 
-// Every window's loads of the last reporting step into loads_host (as many as kLoadsHostBytes holds).
+// The loads of windows `win` and on (cyclically) into loads_host, in place of what lay there, in one launch and
+// wait: one window for the first read after a step, then eight times as many each time until a transfer is for
+// all of them (as many as kLoadsHostBytes holds; the others are read singly).  So a caller that reads two
+// windows of hundreds brings over nine, and one that reads all 24 waits three times (24 windows of 1136
+// particles: all of them 219 us, two of them 50; with a doubling 250 and 45 us, with everything on the second
+// read 206 and 71, one at a time 800 and 66 us).
 constexpr int64_t kLoadsHostBytes = 64 << 20;
-int batch_fetch_loads(psc_batch& b, const char* who) {
-    std::vector<int64_t> at(b.w.size(), -1);
+int batch_fetch_loads(psc_batch& b, size_t win, const char* who) {
+    const size_t nwin = b.w.size(), take = b.loads_take;
+    b.loads_take = take >= nwin ? 0 : 8 * take;
+    b.loads_at.assign(nwin, -1);
+    std::vector<int64_t> at(nwin, -1);
     std::vector<RowCopy> rows;
     int64_t total = 0;
-    for (size_t k = 0; k < b.w.size(); ++k) {
+    for (size_t j = 0; j < nwin && rows.size() < 2 * take; ++j) {
+        const size_t k = (win + j) % nwin;
         const Window& w = *b.w[k];
         const int64_t n = 3 * (int64_t)w.P;
         if (w.P == 0 || !w.loads_ready || (total + 2 * n) * 8 > kLoadsHostBytes) continue;
@@ -1693,12 +1702,12 @@ int batch_fetch_loads(psc_batch& b, const char* who) {
         rows.push_back({w.torques.p, total + n, n});
         total += 2 * n;
     }
-    if (pinned_room(b.loads_host, total)) {
-        PSC_CUDA(launch_copy_rows(rows.data(), (int)rows.size(), b.loads_host.p, b.stream), who);
-        PSC_CUDA(cudaStreamSynchronize(b.stream), who);
-    } else {  // each window's on its own
-        at.assign(b.w.size(), -1);
+    if (!pinned_room(b.loads_host, total)) {  // each window's on its own
+        b.loads_take = 0;
+        return PSC_OK;
     }
+    PSC_CUDA(launch_copy_rows(rows.data(), (int)rows.size(), b.loads_host.p, b.stream), who);
+    PSC_CUDA(cudaStreamSynchronize(b.stream), who);
     b.loads_at.swap(at);
     return PSC_OK;
 }
@@ -2191,7 +2200,7 @@ int psc_batch_step(psc_batch* b, int nsteps, unsigned flags, psc_status* h_statu
                  "psc_batch_step: particle loads");
         if (!desc_ready) b->desc_built.swap(geos);
         b->loads_at.clear();
-        b->loads_first = -1;
+        b->loads_take = 1;
         for (int k = 0; k < nwin; ++k)
             if (b->frozen[(size_t)k] < 0) {
                 b->w[(size_t)k]->loads_enqueued();
@@ -2320,15 +2329,8 @@ int psc_batch_get_loads(psc_batch* b, int win, double* h_forces, double* h_torqu
     if (!h_forces || !h_torques) return fail(PSC_E_INVALID, "psc_batch_get_loads: null output");
     if (!w.loads_ready) return fail(PSC_E_INVALID, "psc_batch_get_loads: no PSC_RUN_DIAG step has run since the last step");
     DeviceScope ds(b->device);
-    // The second window asked for after a step brings every window's loads in one launch (24 windows of 1136
-    // particles: 0.8 -> 0.1 ms); the first one its own.
-    if (b->loads_at.empty()) {
-        if (b->loads_first < 0 || b->loads_first == win) {
-            b->loads_first = win;
-            return window_loads_to_host(w, h_forces, h_torques, b->stream, b->tot, "psc_batch_get_loads");
-        }
-        PSC_TRY(batch_fetch_loads(*b, "psc_batch_get_loads"));
-    }
+    if (b->loads_at.empty() || (b->loads_at[(size_t)win] < 0 && b->loads_take > 0))
+        PSC_TRY(batch_fetch_loads(*b, (size_t)win, "psc_batch_get_loads"));
     const int64_t at = b->loads_at[(size_t)win], n = 3 * (int64_t)w.P;
     if (at < 0) return window_loads_to_host(w, h_forces, h_torques, b->stream, b->tot, "psc_batch_get_loads");
     std::memcpy(h_forces, b->loads_host.p + at, (size_t)n * 8);

@@ -39,3 +39,25 @@ def test_fields_arrive(run, no_pinned):
 @pytest.mark.parametrize("P", [1, 300, 60000])  # 60000: 2.9 MB of loads, more than the page-locked ring
 def test_loads_arrive(run, no_pinned, P):
     assert run("loads", no_pinned, 5, P, 0, 1, 2, 4, 3, 1, 0)["bad"] == 0
+
+
+WINDOW = 2 * 3 * 50 * 8  # bytes of one window's loads
+
+
+def test_reading_two_windows_of_many_brings_a_few(run):
+    got = run("loads", 0, 400, 50, 17, 200)
+    assert got["bad"] == 0 and got["copied"] <= 9 * WINDOW and got["pinned"] <= 9 * WINDOW
+
+
+@pytest.mark.parametrize("order", ["up", "down", "mixed", "same"])
+@pytest.mark.parametrize("nwin", [1, 2, 8, 9, 24, 200])
+def test_reading_windows_takes_few_transfers(run, nwin, order):
+    """Each transfer brings eight times as many windows as the one before (1, 8, 64, ...) until one brings all,
+    in whatever order they are asked for: bytes and waits do not grow with the reads."""
+    reads = {"up": list(range(nwin)), "down": list(range(nwin))[::-1], "mixed": [k * 7 % nwin for k in range(nwin)],
+             "same": [nwin // 2] * 5}[order]
+    got = run("loads", 0, nwin, 50, *reads, *reads)
+    transfers = 1 + sum(8 ** k < nwin for k in range(4))
+    assert got["bad"] == 0
+    assert got["waits"] <= (1 if order == "same" else transfers)
+    assert got["copied"] <= (1 if order == "same" else sum(min(8 ** k, nwin) for k in range(transfers))) * WINDOW
