@@ -17,6 +17,9 @@ from . import _native as nat
 from .engine import require_cuda, stream_handle, vp
 
 Q = 19
+# steps per library call: even (the state is back in the first buffer), and few enough that a long run
+# can be interrupted (64^3: 1 ms a call)
+_PIECE = 64
 
 
 def voxelize(points, center, size, radius: float, n: int, device=None):
@@ -54,8 +57,14 @@ def run_lbm(solid, tau: float, force_z: float, steps: int, return_fields: bool =
         mom = torch.empty(4 * N, dtype=torch.float64, device=dev)
         st = stream_handle(dev)
         nat.call("psc_init_equilibrium", nat.STORE_F64_EXACT, 1.0, vp(f[0]), N, st)
-        nat.call("psc_bounceback_steps", vp(f[0]), vp(f[1]), vp(s), nx, ny, nz, float(tau), 0.0, 0.0, float(force_z),
-                 max(int(steps), 0), vp(mom), st)
+        left = max(int(steps), 0)
+        while True:
+            k = min(left, _PIECE)
+            left -= k
+            nat.call("psc_bounceback_steps", vp(f[0]), vp(f[1]), vp(s), nx, ny, nz, float(tau), 0.0, 0.0,
+                     float(force_z), k, None if left else vp(mom), st)
+            if not left:
+                break
         m = mom.view(4, nx, ny, nz).cpu().numpy()
     ux, uy, uz = m[1], m[2], m[3]
     fluid = ~solid_np
