@@ -669,6 +669,8 @@ double* diag_dev(Window& w) { return w.out.p + 2 * PSC_NRED; }
 // descriptors are made once per geometry.
 int window_loads_from(Window& w, const void* imb, const double* imb_sums, cudaStream_t s, double* host_diag = nullptr) {
     const psc_geometry g = w.geometry();
+    // particles given since the last step to a window that has never held an entry: no geometry to reduce over
+    if (w.P > 0 && !w.built && !g.ent_cnt) return fail(PSC_E_INVALID, "psc_particle_loads: null array");
     if (w.P > 0 && w.cap_chunks > 0 && (!w.built || w.desc_built != w.built_version)) {
         PSC_CUDA(launch_chunk_desc(g, w.chunk_desc.p, s), "particle loads");
         w.desc_built = w.built ? w.built_version : 0;
