@@ -732,8 +732,10 @@ void fill_diag(const Window& w, const double* host_out, psc_diag& d) {
 // the caller's memory, where the driver does the same: 128^3 1.17 ms against 1.34 here; one piece goes
 // through the ring (24^3 41 -> 33 us).  ring: page-locked memory of the caller's handle, grown to
 // kRingPiece * kRingPieces bytes at most; where there is none to be had, floats cross into the upper half of
-// dst and are converted in place.
-constexpr int64_t kRingPiece = 256 << 10, kRingPieces = 8;
+// dst and are converted in place.  Seven pieces, since a page-locked allocation of 2 MB and more is mapped by
+// itself and smaller ones come out of the driver's pool: the first field read of a 110^3 window 2.3 to 2.7 ms with eight, 1.1 to
+// 1.3 with seven (2.2 to 3.2 through pageable memory); later reads take the same.
+constexpr int64_t kRingPiece = 256 << 10, kRingPieces = 7;
 
 // Whether the page-locked array holds n elements now; a failed allocation leaves no error behind.
 template <class T>

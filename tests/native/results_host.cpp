@@ -73,6 +73,16 @@ static int fields() {
     return bad;
 }
 
+// One float field of n values.
+static int field(int64_t n) {
+    std::vector<float> f((size_t)n, 0.25f);
+    std::vector<double> out((size_t)n, -1.0);
+    HArray<int64_t> ring;
+    int bad = values_to_host(f.data(), false, n, out.data(), nullptr, ring, "x") != PSC_OK;
+    for (double v : out) bad |= v != 0.25;
+    return bad;
+}
+
 static void make_batch(psc_batch& b, int nwin, int P) {
     for (int k = 0; k < nwin; ++k) {
         b.w.emplace_back(new Window);
@@ -96,12 +106,14 @@ static int read(psc_batch& b, int k) {
            std::memcmp(t.data(), b.w[(size_t)k]->torques.p, n * 8) != 0 || g_last != cudaSuccess;
 }
 
-// results_host fields NO_PINNED | results_host loads NO_PINNED NWIN P WINDOW...
+// results_host fields NO_PINNED | results_host field NO_PINNED VALUES | results_host loads NO_PINNED NWIN P WINDOW...
 int main(int argc, char** argv) {
     g_no_pinned = std::atoi(argv[2]) != 0;
     int bad = 0;
     if (!std::strcmp(argv[1], "fields")) {
         bad = fields();
+    } else if (!std::strcmp(argv[1], "field")) {
+        bad = field(std::atoll(argv[3]));
     } else {
         psc_batch b;
         make_batch(b, std::atoi(argv[3]), std::atoi(argv[4]));

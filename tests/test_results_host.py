@@ -41,6 +41,13 @@ def test_loads_arrive(run, no_pinned, P):
     assert run("loads", no_pinned, 5, P, 0, 1, 2, 4, 3, 1, 0)["bad"] == 0
 
 
+@pytest.mark.parametrize("values", [1, 100 ** 3, 160 ** 3])
+def test_a_field_asks_for_less_than_a_mapping_of_page_locked_memory(run, values):
+    """A page-locked allocation of 2 MB and more is mapped by itself, which costs more than a field's transfer."""
+    got = run("field", 0, values)
+    assert got["bad"] == 0 and got["pinned"] < 2 << 20
+
+
 WINDOW = 2 * 3 * 50 * 8  # bytes of one window's loads
 
 
