@@ -1592,6 +1592,7 @@ struct psc_batch {
     HArray<double> loads_host;
     std::vector<int64_t> loads_at;
     size_t loads_take = 1;
+    bool loads_again = false;  // loads of an earlier step were read
     int jobs_n = 0, jobs_max_s = 1, jobs_max_p = 0;
     int64_t jobs_chunks = 0, jobs_particles = 0;
     bool jobs_list_ready = false;  // every job's loads list is current
@@ -1686,7 +1687,7 @@ std::vector<uint64_t> batch_geometries(const psc_batch& b) {
 // wait: one window for the first read after a step, then eight times as many each time until a transfer is for
 // all of them (as many as kLoadsHostBytes holds; the others are read singly).  So a caller that reads two
 // windows of hundreds brings over nine, and one that reads all 24 waits three times (24 windows of 1136
-// particles: all of them 219 us, two of them 50; with a doubling 250 and 45 us, with everything on the second
+// particles: all of them 219 to 229 us, two of them 50 to 57; with a doubling 250 and 45 us, with everything on the second
 // read 206 and 71, one at a time 800 and 66 us).
 constexpr int64_t kLoadsHostBytes = 64 << 20;
 int batch_fetch_loads(psc_batch& b, size_t win, const char* who) {
@@ -1695,7 +1696,8 @@ int batch_fetch_loads(psc_batch& b, size_t win, const char* who) {
     b.loads_at.assign(nwin, -1);
     std::vector<int64_t> at(nwin, -1);
     std::vector<RowCopy> rows;
-    int64_t total = 0;
+    int64_t total = 0, all = 0;
+    for (const auto& w : b.w) all += 6 * (int64_t)w->P;
     for (size_t j = 0; j < nwin && rows.size() < 2 * take; ++j) {
         const size_t k = (win + j) % nwin;
         const Window& w = *b.w[k];
@@ -1706,7 +1708,9 @@ int batch_fetch_loads(psc_batch& b, size_t win, const char* who) {
         rows.push_back({w.torques.p, total + n, n});
         total += 2 * n;
     }
-    if (!pinned_room(b.loads_host, total)) {  // each window's on its own
+    // (room for all of them at once, up to the ring's size: each growth page-locks again)
+    const int64_t room = std::max(total, std::min(all, kRingPiece * kRingPieces / 8));
+    if (!pinned_room(b.loads_host, room)) {  // each window's on its own
         b.loads_take = 0;
         return PSC_OK;
     }
@@ -2333,6 +2337,13 @@ int psc_batch_get_loads(psc_batch* b, int win, double* h_forces, double* h_torqu
     if (!h_forces || !h_torques) return fail(PSC_E_INVALID, "psc_batch_get_loads: null output");
     if (!w.loads_ready) return fail(PSC_E_INVALID, "psc_batch_get_loads: no PSC_RUN_DIAG step has run since the last step");
     DeviceScope ds(b->device);
+    if (b->loads_at.empty() && !b->loads_again) {
+        // page-locking the room takes 1.5 to 3 ms, as long as reading some sixty windows one by one: not for a batch
+        // that is read after one step only
+        b->loads_again = true;
+        b->loads_at.assign(b->w.size(), -1);
+        b->loads_take = 0;
+    }
     if (b->loads_at.empty() || (b->loads_at[(size_t)win] < 0 && b->loads_take > 0))
         PSC_TRY(batch_fetch_loads(*b, (size_t)win, "psc_batch_get_loads"));
     const int64_t at = b->loads_at[(size_t)win], n = 3 * (int64_t)w.P;

@@ -106,7 +106,7 @@ static int read(psc_batch& b, int k) {
            std::memcmp(t.data(), b.w[(size_t)k]->torques.p, n * 8) != 0 || g_last != cudaSuccess;
 }
 
-// results_host fields NO_PINNED | results_host field NO_PINNED VALUES | results_host loads NO_PINNED NWIN P WINDOW...
+// results_host fields NO_PINNED | results_host field NO_PINNED VALUES | results_host loads NO_PINNED NWIN P (WINDOW | step)...
 int main(int argc, char** argv) {
     g_no_pinned = std::atoi(argv[2]) != 0;
     int bad = 0;
@@ -117,7 +117,15 @@ int main(int argc, char** argv) {
     } else {
         psc_batch b;
         make_batch(b, std::atoi(argv[3]), std::atoi(argv[4]));
-        for (int k = 5; k < argc; ++k) bad |= read(b, std::atoi(argv[k]));
+        for (int k = 5; k < argc; ++k) {
+            if (!std::strcmp(argv[k], "step")) {  // what a reporting step leaves; counted from here
+                b.loads_at.clear();
+                b.loads_take = 1;
+                g_copied = g_pinned = g_waits = 0;
+            } else {
+                bad |= read(b, std::atoi(argv[k]));
+            }
+        }
     }
     std::printf("%d %lld %lld %d\n", bad, g_copied, g_pinned, g_waits);
     return 0;

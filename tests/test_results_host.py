@@ -38,7 +38,7 @@ def test_fields_arrive(run, no_pinned):
 @pytest.mark.parametrize("no_pinned", [0, 1])
 @pytest.mark.parametrize("P", [1, 300, 60000])  # 60000: 2.9 MB of loads, more than the page-locked ring
 def test_loads_arrive(run, no_pinned, P):
-    assert run("loads", no_pinned, 5, P, 0, 1, 2, 4, 3, 1, 0)["bad"] == 0
+    assert run("loads", no_pinned, 5, P, 0, 1, 2, 4, 3, 1, 0, "step", 3, 3, 0, 1, 2, 4, 0, "step", 4, 0)["bad"] == 0
 
 
 @pytest.mark.parametrize("values", [1, 100 ** 3, 160 ** 3])
@@ -52,8 +52,20 @@ WINDOW = 2 * 3 * 50 * 8  # bytes of one window's loads
 
 
 def test_reading_two_windows_of_many_brings_a_few(run):
-    got = run("loads", 0, 400, 50, 17, 200)
-    assert got["bad"] == 0 and got["copied"] <= 9 * WINDOW and got["pinned"] <= 9 * WINDOW
+    got = run("loads", 0, 400, 2000, 17, "step", 17, 200)  # 38 MB in all
+    assert got["bad"] == 0 and got["copied"] <= 9 * 40 * WINDOW and got["pinned"] < 2 << 20
+
+
+def test_the_reads_after_a_batchs_first_step_are_single(run):
+    """No page-locked room for all windows before the loads of a second step are read."""
+    got = run("loads", 0, 24, 700, *range(24))
+    assert got["bad"] == 0 and got["pinned"] <= 14 * WINDOW and got["copied"] == 24 * 14 * WINDOW
+
+
+def test_a_batch_asks_for_page_locked_memory_once(run):
+    """Up to the size of the ring; a free and a second allocation wait for the device."""
+    got = run("loads", 0, 24, 700, 0, "step", *range(24))
+    assert got["bad"] == 0 and got["pinned"] <= 24 * 14 * WINDOW
 
 
 @pytest.mark.parametrize("order", ["up", "down", "mixed", "same"])
@@ -63,7 +75,7 @@ def test_reading_windows_takes_few_transfers(run, nwin, order):
     in whatever order they are asked for: bytes and waits do not grow with the reads."""
     reads = {"up": list(range(nwin)), "down": list(range(nwin))[::-1], "mixed": [k * 7 % nwin for k in range(nwin)],
              "same": [nwin // 2] * 5}[order]
-    got = run("loads", 0, nwin, 50, *reads, *reads)
+    got = run("loads", 0, nwin, 50, 0, "step", *reads, *reads)
     transfers = 1 + sum(8 ** k < nwin for k in range(4))
     assert got["bad"] == 0
     assert got["waits"] <= (1 if order == "same" else transfers)
