@@ -251,7 +251,7 @@ struct Window {
     DArray<uint8_t> level;
     DArray<unsigned char> scan_tmp;
     DArray<double> chunk_partials;
-    DArray<double> chunk_desc;  // load-chunk descriptors of the geometry of desc_built (window_chunk_desc)
+    DArray<double> chunk_desc;  // load-chunk descriptors of the geometry of desc_built (made with the build)
     uint64_t desc_built = 0;
     double smooth_eps = 0.0;  // > 0: smooth solid fraction (the adjoint's differentiable surrogate)
     DArray<double> ent_alpha;
@@ -732,10 +732,11 @@ void fill_diag(const Window& w, const double* host_out, psc_diag& d) {
 // the caller's memory, where the driver does the same: 128^3 1.17 ms against 1.34 here; one piece goes
 // through the ring (24^3 41 -> 33 us).  ring: page-locked memory of the caller's handle, grown to
 // kRingPiece * kRingPieces bytes at most; where there is none to be had, floats cross into the upper half of
-// dst and are converted in place.  Seven pieces, since a page-locked allocation of 2 MB and more is mapped by
-// itself and smaller ones come out of the driver's pool: the first field read of a 110^3 window 2.3 to 2.7 ms with eight, 1.1 to
-// 1.3 with seven (2.2 to 3.2 through pageable memory); later reads take the same.
-constexpr int64_t kRingPiece = 256 << 10, kRingPieces = 7;
+// dst and are converted in place.  512 KB in all, since page-locking takes 1.3 to 3 ms per 2 MB, in which the
+// driver places smaller allocations: the first reads of eight 110^3 windows take 1.2 ms each on the average with four
+// pieces of 128 KB, 2.0 with seven of 256 and 3.2 through pageable memory, later ones 0.61, 0.57 and 2.7; 75^3
+// 0.69, 1.54 and 1.12, later 0.21, 0.20 and 0.93 (four of 64 KB: 110^3 0.74, 75^3 0.24).
+constexpr int64_t kRingPiece = 128 << 10, kRingPieces = 4;
 
 // Whether the page-locked array holds n elements now; a failed allocation leaves no error behind.
 template <class T>
@@ -747,7 +748,7 @@ bool pinned_room(HArray<T>& a, int64_t n) {
 
 int values_to_host(const void* src, bool f64, int64_t count, double* dst, cudaStream_t s, HArray<int64_t>& ring,
                    const char* who) {
-    const int64_t el = f64 ? 8 : 4, piece = kRingPiece / el, n = (count + piece - 1) / piece;
+    const int64_t el = f64 ? 8 : 4, piece = (f64 ? 2 : 1) * kRingPiece / el, n = (count + piece - 1) / piece;
     const int64_t slots = std::min(n, kRingPieces);
     if ((f64 && n > 1) || !pinned_room(ring, n > 1 ? slots * kRingPiece / 8 : (count * el + 7) / 8)) {
         unsigned char* at = reinterpret_cast<unsigned char*>(dst) + (f64 ? 0 : count * 4);
@@ -1588,10 +1589,11 @@ struct psc_batch {
     DArray<double> loads_desc;  // chunk descriptors of all jobs, of the geometries in desc_built
     std::vector<uint64_t> desc_built;
     // loads of the last reporting step on the host (batch_fetch_loads): where each window's lie (-1: not there;
-    // empty: none read since the step), and how many windows the next transfer brings (0: no more of them)
+    // empty: none read since the step), and how many windows the next transfer brings (0: none, no room)
     HArray<double> loads_host;
     std::vector<int64_t> loads_at;
     size_t loads_take = 1;
+    int loads_last = -1;       // the window read last since the step
     bool loads_again = false;  // loads of an earlier step were read
     int jobs_n = 0, jobs_max_s = 1, jobs_max_p = 0;
     int64_t jobs_chunks = 0, jobs_particles = 0;
@@ -1683,34 +1685,35 @@ std::vector<uint64_t> batch_geometries(const psc_batch& b) {
     return v;
 }
 
-// The loads of windows `win` and on (cyclically) into loads_host, in place of what lay there, in one launch and
-// wait: one window for the first read after a step, then eight times as many each time until a transfer is for
-// all of them (as many as kLoadsHostBytes holds; the others are read singly).  So a caller that reads two
-// windows of hundreds brings over nine, and one that reads all 24 waits three times (24 windows of 1136
-// particles: all of them 219 to 229 us, two of them 50 to 57; with a doubling 250 and 45 us, with everything on the second
-// read 206 and 71, one at a time 800 and 66 us).
-constexpr int64_t kLoadsHostBytes = 64 << 20;
+// The loads of windows `win` and on (cyclically; downwards where the window read before lies above) into loads_host, in place of what lay there, in one launch and
+// wait: one window for the first read after a step, then eight times as many each time, as far as the room reaches
+// (a window that does not fit is read singly).  So a caller that reads two windows of hundreds brings over
+// nine, and one that reads all 24 waits a few times (24 windows of 1136 particles: all of them 250 us, two of them
+// 57; 200 of 300: 1020; everything on the second read 206 and 71 us, one at a time 800 and 66).
+constexpr int64_t kLoadsHostBytes = kRingPiece * kRingPieces;
 int batch_fetch_loads(psc_batch& b, size_t win, const char* who) {
     const size_t nwin = b.w.size(), take = b.loads_take;
-    b.loads_take = take >= nwin ? 0 : 8 * take;
+    b.loads_take = std::min(8 * take, nwin);
     b.loads_at.assign(nwin, -1);
     std::vector<int64_t> at(nwin, -1);
     std::vector<RowCopy> rows;
     int64_t total = 0, all = 0;
     for (const auto& w : b.w) all += 6 * (int64_t)w->P;
+    const bool down = b.loads_last > (int)win;
     for (size_t j = 0; j < nwin && rows.size() < 2 * take; ++j) {
-        const size_t k = (win + j) % nwin;
+        const size_t k = (down ? win + nwin - j : win + j) % nwin;
         const Window& w = *b.w[k];
         const int64_t n = 3 * (int64_t)w.P;
-        if (w.P == 0 || !w.loads_ready || (total + 2 * n) * 8 > kLoadsHostBytes) continue;
+        if (w.P == 0 || !w.loads_ready) continue;
+        if ((total + 2 * n) * 8 > kLoadsHostBytes) break;
         at[k] = total;
         rows.push_back({w.forces.p, total, n});
         rows.push_back({w.torques.p, total + n, n});
         total += 2 * n;
     }
-    // (room for all of them at once, up to the ring's size: each growth page-locks again)
-    const int64_t room = std::max(total, std::min(all, kRingPiece * kRingPieces / 8));
-    if (!pinned_room(b.loads_host, room)) {  // each window's on its own
+    if (rows.empty()) return PSC_OK;
+    // (room for all of them at once: each growth page-locks again)
+    if (!pinned_room(b.loads_host, std::min(all, kLoadsHostBytes / 8))) {  // each window's on its own
         b.loads_take = 0;
         return PSC_OK;
     }
@@ -2209,6 +2212,7 @@ int psc_batch_step(psc_batch* b, int nsteps, unsigned flags, psc_status* h_statu
         if (!desc_ready) b->desc_built.swap(geos);
         b->loads_at.clear();
         b->loads_take = 1;
+        b->loads_last = -1;
         for (int k = 0; k < nwin; ++k)
             if (b->frozen[(size_t)k] < 0) {
                 b->w[(size_t)k]->loads_enqueued();
@@ -2338,14 +2342,15 @@ int psc_batch_get_loads(psc_batch* b, int win, double* h_forces, double* h_torqu
     if (!w.loads_ready) return fail(PSC_E_INVALID, "psc_batch_get_loads: no PSC_RUN_DIAG step has run since the last step");
     DeviceScope ds(b->device);
     if (b->loads_at.empty() && !b->loads_again) {
-        // page-locking the room takes 1.5 to 3 ms, as long as reading some sixty windows one by one: not for a batch
-        // that is read after one step only
+        // page-locking the room may take 1.3 to 3 ms, as long as reading some sixty windows one by one: not for a
+        // batch that is read after one step only
         b->loads_again = true;
         b->loads_at.assign(b->w.size(), -1);
         b->loads_take = 0;
     }
     if (b->loads_at.empty() || (b->loads_at[(size_t)win] < 0 && b->loads_take > 0))
         PSC_TRY(batch_fetch_loads(*b, (size_t)win, "psc_batch_get_loads"));
+    b->loads_last = win;
     const int64_t at = b->loads_at[(size_t)win], n = 3 * (int64_t)w.P;
     if (at < 0) return window_loads_to_host(w, h_forces, h_torques, b->stream, b->tot, "psc_batch_get_loads");
     std::memcpy(h_forces, b->loads_host.p + at, (size_t)n * 8);

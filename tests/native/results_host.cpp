@@ -121,6 +121,7 @@ int main(int argc, char** argv) {
             if (!std::strcmp(argv[k], "step")) {  // what a reporting step leaves; counted from here
                 b.loads_at.clear();
                 b.loads_take = 1;
+                b.loads_last = -1;
                 g_copied = g_pinned = g_waits = 0;
             } else {
                 bad |= read(b, std::atoi(argv[k]));

@@ -43,17 +43,17 @@ def test_loads_arrive(run, no_pinned, P):
 
 @pytest.mark.parametrize("values", [1, 100 ** 3, 160 ** 3])
 def test_a_field_asks_for_less_than_a_mapping_of_page_locked_memory(run, values):
-    """A page-locked allocation of 2 MB and more is mapped by itself, which costs more than a field's transfer."""
+    """Page-locking takes longer than a field's transfer, per 2 MB in which smaller allocations share a place."""
     got = run("field", 0, values)
-    assert got["bad"] == 0 and got["pinned"] < 2 << 20
+    assert got["bad"] == 0 and got["pinned"] <= 512 << 10
 
 
 WINDOW = 2 * 3 * 50 * 8  # bytes of one window's loads
 
 
 def test_reading_two_windows_of_many_brings_a_few(run):
-    got = run("loads", 0, 400, 2000, 17, "step", 17, 200)  # 38 MB in all
-    assert got["bad"] == 0 and got["copied"] <= 9 * 40 * WINDOW and got["pinned"] < 2 << 20
+    got = run("loads", 0, 400, 1000, 17, "step", 17, 200)  # 19 MB in all
+    assert got["bad"] == 0 and got["copied"] <= 9 * 20 * WINDOW and got["pinned"] <= 512 << 10
 
 
 def test_the_reads_after_a_batchs_first_step_are_single(run):
@@ -62,10 +62,21 @@ def test_the_reads_after_a_batchs_first_step_are_single(run):
     assert got["bad"] == 0 and got["pinned"] <= 14 * WINDOW and got["copied"] == 24 * 14 * WINDOW
 
 
-def test_a_batch_asks_for_page_locked_memory_once(run):
-    """Up to the size of the ring; a free and a second allocation wait for the device."""
-    got = run("loads", 0, 24, 700, 0, "step", *range(24))
-    assert got["bad"] == 0 and got["pinned"] <= 24 * 14 * WINDOW
+@pytest.mark.parametrize("order", [1, -1])
+@pytest.mark.parametrize("P", [100, 700, 9000])  # 115 KB, 0.8 and 10 MB of loads
+def test_a_batch_asks_for_page_locked_memory_once(run, P, order):
+    """A free and a second allocation wait for the device.  Read in turn, up or down, loads beyond the room come over
+    once, in pieces of the room (the last of them may reach around)."""
+    got = run("loads", 0, 24, P, 0, "step", *range(24)[::order])
+    window, room = 48 * P, 512 << 10
+    assert got["bad"] == 0 and got["pinned"] <= min(24 * window, room)
+    assert got["copied"] <= 24 * window + max(window, min(room, 23 * window))
+    assert got["waits"] <= 2 + 24 // min(room // window, 24) + 1
+
+
+def test_windows_of_more_than_the_room(run):
+    got = run("loads", 0, 3, 12000, 0, "step", 0, 1, 2, 0)
+    assert got["bad"] == 0 and got["copied"] == 4 * 48 * 12000
 
 
 @pytest.mark.parametrize("order", ["up", "down", "mixed", "same"])
