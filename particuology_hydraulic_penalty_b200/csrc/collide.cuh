@@ -465,7 +465,9 @@ PSC_HD R csel(int c, R x) {
     return c == 0 ? R(0) : (c > 0 ? x : -x);
 }
 
-// Collide deviations g in place; irho = 1 / rho; B solid weight.  imb gets
+// Collide deviations g in place; irho = 1 / rho; B solid weight.  The plain form,
+// term by term: no kernel runs it, the host tests hold it and the regrouped form
+// below, which the kernels run, to the same oracle.  imb gets
 // sum_i c_i B Omega_s,i.  Returns nothing else: the caller owns the moments.
 template <typename R, bool MOVING, bool IMB>
 PSC_HD void collide_fast(R* g, const FastMoments<R>& mo, R irho, R B, R usx, R usy, R usz,
