@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(256) k_adjoint_step(const __grid_constant__ ps
 
 // Two consecutive z cells per thread in packed FP32 (nz even, pointers aligned): the accesses of
 // k_step_pair, half the arithmetic instructions.  Bound by HBM: 252 B per cell, 34 us on 96^3.  Twelve
-// warps per SM at 168 registers: 96^3 48.5 -> 39.8 us, 64^3 14.1 -> 9.6 us (sixteen warps at 128 registers
+// warps per SM at 168 registers: 96^3 48.5 -> 39.1 us, 64^3 14.1 -> 9.7 us (sixteen warps at 128 registers
 // spill: 49 us; eight at 255: 46 us; one cell per thread: 45 us).
 constexpr int ADJ_THREADS = 128, ADJ_CTAS = 3;
 __global__ void __launch_bounds__(ADJ_THREADS, ADJ_CTAS) k_adjoint_pair(const __grid_constant__ psc_adjoint_args a) {

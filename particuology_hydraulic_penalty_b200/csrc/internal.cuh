@@ -166,6 +166,5 @@ cudaError_t launch_guo(double fx, double fy, double fz, const double* ux, const 
 
 // exclusive scan of int32 counts -> int32 offsets, out has n + 1 entries
 size_t scan_tmp_bytes(int64_t n);
-cudaError_t scan_exclusive_i32(const int32_t* in, int32_t* out, int64_t n, void* tmp, cudaStream_t stream);
 
 }  // namespace psc

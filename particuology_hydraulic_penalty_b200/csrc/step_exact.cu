@@ -145,7 +145,7 @@ __device__ __noinline__ void exact_cell_general(const ExactShared& s, uint32_t c
 // (312 B/cell, 196 us at the measured copy rate) and the FP64 pipe (one warp instruction every other
 // cycle and SM quarter, about 575 per cell: 130 us).  Measured with branch-free divisions, one window
 // set-up per CTA and window, and range tests in integer instructions, in a chain of steps: 231 us
-// plain, 263 with IMB and sums (553 and 608 with a branch per division and a window look-up per tile);
+// plain, 271 with IMB and sums (553 and 608 with a branch per division and a window look-up per tile);
 // 96^3: 54 and 62 (126 and 137); 24^3: 3.9 and 5.1 (8.9 and 9.8).  Staging the next tile's populations in shared memory by
 // cp.async took another 1 to 4 %, at one more kernel per variant: not used.
 template <bool MOVING, bool RED>

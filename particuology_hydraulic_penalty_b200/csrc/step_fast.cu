@@ -14,7 +14,6 @@
 
 namespace psc {
 
-
 // Resident CTAs the register allocation aims for: four (64 registers) for
 // FP32/FP16/BF16 storage, three with moving particles (the solid-velocity
 // terms), two for FP64, whose arithmetic needs about twice the registers, and

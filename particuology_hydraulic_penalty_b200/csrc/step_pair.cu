@@ -8,8 +8,9 @@
 // stores; the ten z-shifted directions pull two scalars.  Measured on the
 // bare access pattern (19 planes read + 19 written, 33 M cells): 2-element
 // accesses at two CTAs per SM move 6.5 TB/s against 5.1-5.9 TB/s for scalar
-// ones.  The per-cell arithmetic is fast_cell(), the same function as the
-// one-cell kernel's, so both produce identical populations.
+// ones.  The per-cell arithmetic is the one-cell kernel's: fast_cell() for each
+// cell, or for 16-bit storage fast_cell_pair(), which takes both at once in
+// packed FP32 and rounds alike, so both kernels produce identical populations.
 #include <type_traits>
 
 #include "fast_cell.cuh"
@@ -52,9 +53,9 @@ __global__ void __launch_bounds__(STEP_THREADS, (PairOccupancy<STORE, MOVING, RE
     using R = typename TR::R;
     using O = typename TR::O;
     // Both cells in packed FP32 where the arithmetic weighs: 16-bit storage (FP16 160^3 90 -> 82 us plain and
-    // 107 -> 99 with IMB and sums, 78 and 95 in a chain of steps; 311 and 394 instructions per cell).  FP32
+    // 107 -> 99 with IMB and sums, 78 and 96 in a chain of steps; 311 and 394 instructions per cell).  FP32
     // storage is bound by HBM, and there the packed form was slower (114 against 108 us, although at 261
-    // instructions per cell instead of 378: its shorter bursts of arithmetic leave reads and writes less
+    // instructions per cell instead of 378, 351 now: its shorter bursts of arithmetic leave reads and writes less
     // spread).  FP64 has no packed form.
     constexpr bool PACKED = sizeof(T) == 2;
     using V = std::conditional_t<PACKED, F2, R>;
@@ -82,7 +83,7 @@ __global__ void __launch_bounds__(STEP_THREADS, (PairOccupancy<STORE, MOVING, RE
     bool have = false;
     bool skip = false;  // block-uniform: the window in sw cannot run here
     // this thread's first cell (ix, iy, iz) in the current tile: divided out when the CTA enters a
-    // window, then advanced tile by tile (consecutive tiles, tile_cells apart) by a carry-add
+    // window, then advanced to the CTA's next tile (walk.size tiles on) by a carry-add
     bool fresh = true;
     uint32_t ix = 0, iy = 0, iz = 0;
     for (uint32_t t = walk.first(); t < walk.end; t += walk.size) {
